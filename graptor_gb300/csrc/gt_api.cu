@@ -33,8 +33,10 @@ cudaError_t launch_radon(const float *img, float *sino, const float4 *ofs, int N
                          cudaStream_t st);
 cudaError_t launch_radon_ad(const float *sino, float *img, const float4 *ofs, int N, int nd, int nang, int S,
                             cudaStream_t st);
-cudaError_t launch_transpose(const float *in, float *out, int rows, int cols, cudaStream_t st);
-cudaError_t launch_output_f64(const float *in, double *out, int A, int B, int C, int Nz, int mode, cudaStream_t st);
+cudaError_t launch_transpose(const float *in, float *out, int rows, int cols, int ld_in, int ld_out,
+                             cudaStream_t st);
+cudaError_t launch_output_f64(const float *in, double *out, int A, int B, int C, int Nz, int Sd, int mode,
+                              cudaStream_t st);
 cudaError_t launch_feasible(float *f, const float *r1, int nbin1, int S, cudaStream_t st);
 cudaError_t launch_lambda_fixed(float *lam, const float *ku, const float *f, const double *mu, long long nbin, int S,
                                 int Nz, int disc, float empty_weight, float cap, cudaStream_t st);
@@ -60,10 +62,10 @@ cudaError_t fill_f32(float *x, size_t n, float v, cudaStream_t st);
 cudaError_t launch_ray_count(const float4 *ofs, int N, int nd, int nang, int *count, cudaStream_t st);
 cudaError_t launch_ray_fill(const float4 *ofs, int N, int nd, int nang, const long long *start, int2 *ent,
                             cudaStream_t st);
-cudaError_t launch_bp_table(const float4 *ofs, int N, int nd, int nang, int2 *tab, cudaStream_t st);
 cudaError_t launch_run_count(const float4 *ofs, int N, int nd, int nang, int *count, cudaStream_t st);
-size_t row_table_bytes(int N, int nang);
-cudaError_t launch_row_fill(const float4 *ofs, int N, int nd, int nang, int4 *tab, int *bad, cudaStream_t st);
+long long tap_entries(int N, int nd, int nang);
+cudaError_t launch_tap_fill(const float4 *ofs, int N, int nd, int nang, unsigned *hdr, float4 *frac, cudaStream_t st);
+int default_bp_shape(int S);
 cudaError_t launch_run_fill(const float4 *ofs, int N, int nd, int nang, const long long *start, int4 *ent,
                             cudaStream_t st);
 int num_proj_configs(int S, int which);
@@ -125,6 +127,13 @@ void angle_table(const double *angles, int N, int nd, int nang, std::vector<doub
   }
 }
 
+constexpr int kMuPad = 4;  // channel weights of the padding slices (channel index s / Nz >= C): 1
+
+// Slices per pixel in memory.  The vector kernels (projectors, primal update) move four
+// slices per load, so a count that is not a multiple of 4 is padded with zero slices,
+// which every kernel leaves zero.  One and two slices stay as they are.
+int padded_slices(int S) { return S <= 2 ? S : (S + 3) & ~3; }
+
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // cuTensorMapEncodeTiled from the driver (through the runtime's entry-point query,
@@ -166,6 +175,7 @@ bool encode_lambda_map(CUtensorMap *map, float *lam, int S, int nd, int nang, un
 
 struct gt_problem {
   gt::Dims d{};
+  int Sr = 0;                  // slices the caller sees: C*Nz (d.S is the count in memory)
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaStream_t side = nullptr;            // second stream: k_fwd runs beside k_dual
@@ -184,7 +194,7 @@ struct gt_problem {
   float *lam = nullptr, *f = nullptr, *ku = nullptr, *stage = nullptr, *kstar = nullptr;
   void *rays = nullptr;        // ray table (offsets + entries), built at creation
   void *runs = nullptr;        // 3-bin run table (offsets + entries), built at creation
-  void *tiles = nullptr;       // row-tile table of k_bp_row, built at creation
+  void *tiles = nullptr;       // row-tile table of k_bp_tap, built at creation
   size_t ray_bytes = 0;
   void *gap_ws = nullptr;      // gap workspace (v~ planes + FP64 block partials), allocated on first gt_gap
   float *snap = nullptr;       // copy of (u, p, v, w, lambda) for gt_movement, allocated on first gt_snapshot
@@ -283,6 +293,7 @@ int ensure_fused(gt_problem *p) {
     p->fused = nullptr;
     return cuda_err(e, "cudaMalloc (schedule 2 buffers)", __LINE__);
   }
+  CK(cudaMemsetAsync(p->fused, 0, sizeof(float) * n, p->stream));  // its padding slices stay zero
   return GT_OK;
 }
 
@@ -355,10 +366,10 @@ void set_scalars(gt_problem *p) {
 
 // channel weights of the data-term prox: KL mu, L2 mu/(sigma+mu) (3-D :1186-1189)
 int upload_mu_eff(gt_problem *p) {
-  std::vector<float> me(p->d.C);
+  std::vector<float> me(p->d.C + kMuPad, 1.f);
   for (int c = 0; c < p->d.C; ++c)
     me[c] = (float)(p->disc == GT_KL ? p->mu[c] : p->mu[c] / (p->sigma + p->mu[c]));
-  CK(cudaMemcpyAsync(p->mu_eff, me.data(), sizeof(float) * p->d.C, cudaMemcpyHostToDevice, p->stream));
+  CK(cudaMemcpyAsync(p->mu_eff, me.data(), sizeof(float) * me.size(), cudaMemcpyHostToDevice, p->stream));
   CK(cudaStreamSynchronize(p->stream));  // me is a host buffer
   return GT_OK;
 }
@@ -377,31 +388,31 @@ int autotune(gt_problem *p) {
   const bool tgv = p->reg == GT_TGV;
   // every dual shape is tuned: at 256^2 x 60 x 4 the order of the shapes timed
   // alone is their order inside the overlapped iteration
-  // back-projection shapes 14 and 15 (TMA-staged sinogram rows) are bit-identical
-  // but slower on every measured workload (256^2 x 60 x 4: 0.43 / 0.45 against
-  // 0.36 ms); they stay selectable by gt_set_tuning and are not tuned
   constexpr int kMaxCfg = 32;
   const int nc[3] = {std::min(kMaxCfg, gt::num_proj_configs(p->d.S, 0)),
                      std::min(kMaxCfg, gt::num_proj_configs(p->d.S, 1)),
                      std::min(kMaxCfg, gt::num_dual_configs(p->P))};
   // Shapes left out of the tuning (all stay selectable by gt_set_tuning), to bound
-  // its time on batches of many distinct problems: the TMA back projector (above);
-  // the multi-bin / multi-pixel run shapes (forward 5-8, back 9-12) once S >= 32,
-  // 2-4x slower than the best shape on every measured workload there; the
-  // chunk-outermost shapes (forward 9, back 13), which only pay when the image
-  // exceeds L2, below 64 MB of image; one slice per thread (forward 4, back 8)
-  // once S >= 128.
+  // its time on batches of many distinct problems: of the back projection all but the
+  // row-tile shapes (18, 19, 9) and the flat ones (10, 11), each in the range of slice
+  // counts where it can win (times at default_bp_shape; the one-pixel and TMA shapes
+  // never do); the multi-bin run shapes (forward 5-8) once S >= 32, 2-4x slower than
+  // the best shape on every measured workload there; the chunk-outermost shape
+  // (forward 9), which only pays when the image exceeds L2, below 64 MB of image; one
+  // slice per thread (forward 4) once S >= 128.
   const int S = p->d.S;
   const long long img_bytes = (long long)p->d.N * p->d.N * S * 4;
   auto skipped = [&](int which, int c) {
-    if (which == 1 && (c == 14 || c == 15)) return true;
-    if (S >= 32 && ((which == 0 && c >= 5 && c <= 8) || (which == 1 && c >= 9 && c <= 12))) return true;
-    if (img_bytes < (64ll << 20) && ((which == 0 && c == 9) || (which == 1 && c == 13))) return true;
-    if (S >= 128 && ((which == 0 && c == 4) || (which == 1 && c == 8))) return true;
+    if (which == 1)
+      return !((c == 18 && S >= 96) || (c == 19 && S >= 36) || (c == 9 && S >= 16 && S <= 128) ||
+               (c == 10 && S <= 128) || (c == 11 && S <= 16));
+    if (S >= 32 && which == 0 && c >= 5 && c <= 8) return true;
+    if (img_bytes < (64ll << 20) && which == 0 && c == 9) return true;
+    if (S >= 128 && which == 0 && c == 4) return true;
     return false;
   };
   p->P.fwd_cfg = 0;
-  p->P.bp_cfg = 0;
+  p->P.bp_cfg = gt::default_bp_shape(S);
   p->P.dual_cfg = 0;
   if ((nc[0] <= 1 && nc[1] <= 1 && nc[2] <= 1) || !p->autotune) return GT_OK;
   const TuneKey key{p->d.dim, p->d.N, p->d.S, p->d.nd, p->d.nang, p->disc, p->d.C, p->d.Nz, p->reg, p->cpl};
@@ -460,7 +471,7 @@ int autotune(gt_problem *p) {
   int best[3] = {0, 0, 0};
   static const char *names[3] = {"k_fwd", "k_bp", "k_dual"};
   for (int which = 0; which < 3; ++which)
-    for (int c = 1; c < nc[which]; ++c)
+    for (int c = 0; c < nc[which]; ++c)
       if (ms_cfg[which][c] < ms_cfg[which][best[which]]) best[which] = c;
   if (log && rc == GT_OK)
     for (int which = 0; which < 3; ++which)
@@ -560,7 +571,11 @@ int gt_set_schedule(gt_problem *p, int schedule) {
   return GT_OK;
 }
 
-int gt_problem_create(const gt_desc *desc, gt_problem **out) {
+}  // extern "C"
+
+// pad = false keeps exactly C*Nz slices (the inner problem of the two-resolution
+// solver, whose operator norm runs over whole fields)
+static int create_problem(const gt_desc *desc, bool pad, gt_problem **out) {
   if (!desc || !out) return set_err(GT_ERR_ARG, "null argument");
   *out = nullptr;
   const gt_desc &D = *desc;
@@ -576,15 +591,17 @@ int gt_problem_create(const gt_desc *desc, gt_problem **out) {
   if (!(D.stepsize > 0.f)) return set_err(GT_ERR_ARG, "stepsize must be positive");
   if (D.regularisation == GT_TGV && !(D.alpha0 > 0 && D.alpha1 > 0)) return set_err(GT_ERR_ARG, "alpha must be positive");
   if (D.regularisation == GT_TV && !(D.alpha1 > 0)) return set_err(GT_ERR_ARG, "alpha1 must be positive");
-  const long long S = (long long)D.Nz * D.C;
-  const long long vol = (long long)D.N * D.N * S, nbin = (long long)D.nd * D.nang * S;
-  if ((long long)D.N * D.N > (1LL << 30) || S > (1LL << 20) || (long long)D.nd * D.nang > (1LL << 30))
+  const long long Sr = (long long)D.Nz * D.C;
+  if ((long long)D.N * D.N > (1LL << 30) || Sr > (1LL << 20) || (long long)D.nd * D.nang > (1LL << 30))
     return set_err(GT_ERR_ARG, "problem too large for 32-bit pixel / bin indices");
+  const long long S = pad ? padded_slices((int)Sr) : Sr;
+  const long long vol = (long long)D.N * D.N * S, nbin = (long long)D.nd * D.nang * S;
 
   gt_problem *p = new (std::nothrow) gt_problem();
   if (!p) return set_err(GT_ERR_OOM, "host allocation failed");
   p->device = D.device;
   p->d.dim = D.dim; p->d.N = D.N; p->d.Nz = D.Nz; p->d.C = D.C; p->d.S = (int)S;
+  p->Sr = (int)Sr;
   p->d.nd = D.nd; p->d.nang = D.nang; p->d.vol = (size_t)vol; p->d.nbin = (size_t)nbin;
   p->disc = D.discrepancy; p->reg = D.regularisation; p->cpl = D.coupling;
   p->K = D.dim; p->KW = D.dim == 3 ? 6 : 3;
@@ -621,7 +638,7 @@ int gt_problem_create(const gt_desc *desc, gt_problem **out) {
   const size_t fv = sizeof(float) * (size_t)vol, fb = sizeof(float) * (size_t)nbin;
   size_t off[16], total = 0;
   size_t sizes[] = {
-      align256(sizeof(float4) * D.nang), align256(sizeof(dvec4) * D.nang), align256(sizeof(float) * D.C),
+      align256(sizeof(float4) * D.nang), align256(sizeof(dvec4) * D.nang), align256(sizeof(float) * (D.C + kMuPad)),
       align256(fv), align256(fv),                                   // u, ubar
       tgv ? align256(fv * p->K) : 0, tgv ? align256(fv * p->K) : 0, // p, pbar
       align256(fv * p->K),                                          // v
@@ -629,7 +646,7 @@ int gt_problem_create(const gt_desc *desc, gt_problem **out) {
       align256(fb), align256(fb), align256(fb),                     // lam, f, ku
       align256(std::max(fv, fb)),                                   // stage
       align256(fv),                                                 // kstar
-      align256(sizeof(double) * D.C),                               // mu (double)
+      align256(sizeof(double) * (D.C + kMuPad)),                    // mu (double)
       align256(sizeof(int) * 4)};                                   // error flags
   const int nsz = (int)(sizeof(sizes) / sizeof(sizes[0]));
   for (int k = 0; k < nsz; ++k) { off[k] = total; total += sizes[k]; }
@@ -680,8 +697,7 @@ int gt_problem_create(const gt_desc *desc, gt_problem **out) {
       return fail(cuda_err(e, "ray table count", __LINE__));
     for (int r = 0; r < nr; ++r) start[r + 1] = start[r] + cnt[r];
     const size_t off_b = align256(sizeof(long long) * (nr + 1));
-    const size_t off_bp = off_b + align256(sizeof(int2) * (size_t)start[nr]);
-    p->ray_bytes = off_bp + sizeof(int2) * (size_t)D.N * D.N * D.nang;
+    p->ray_bytes = off_b + sizeof(int2) * (size_t)start[nr];
     if ((e = cudaMalloc(&p->rays, p->ray_bytes)) != cudaSuccess) {
       cudaGetLastError();
       gt_problem_destroy(p);
@@ -692,13 +708,10 @@ int gt_problem_create(const gt_desc *desc, gt_problem **out) {
     if ((e = cudaMemcpyAsync(d_start, start.data(), sizeof(long long) * (nr + 1), cudaMemcpyHostToDevice,
                              p->stream)) != cudaSuccess ||
         (e = gt::launch_ray_fill(p->ofs, D.N, D.nd, D.nang, d_start, d_ent, p->stream)) != cudaSuccess ||
-        (e = gt::launch_bp_table(p->ofs, D.N, D.nd, D.nang, (int2 *)((char *)p->rays + off_bp), p->stream)) !=
-            cudaSuccess ||
         (e = cudaStreamSynchronize(p->stream)) != cudaSuccess)
       return fail(cuda_err(e, "ray table fill", __LINE__));
     p->P.ray_start = d_start;
     p->P.ray_ent = d_ent;
-    p->P.bp_tab = (const int2 *)((char *)p->rays + off_bp);
   }
 
   // 3-bin run table of the forward projector (k_fwd_rt); optional: without it
@@ -731,25 +744,18 @@ int gt_problem_create(const gt_desc *desc, gt_problem **out) {
     }
   }
 
-  // row-tile table of the register-blocked back projector (k_bp_row); optional:
-  // without it (no memory, nd < 2, a geometry the table cannot describe) those
-  // launch shapes fall back to the others
-  if (D.nd >= 2) {
-    const size_t tbytes = gt::row_table_bytes(D.N, D.nang);
-    if (cudaMalloc(&p->tiles, align256(tbytes) + 256) == cudaSuccess) {
-      int *d_bad = (int *)((char *)p->tiles + align256(tbytes));
-      int bad = 0;
-      if ((e = cudaMemsetAsync(d_bad, 0, sizeof(int), p->stream)) != cudaSuccess ||
-          (e = gt::launch_row_fill(p->ofs, D.N, D.nd, D.nang, (int4 *)p->tiles, d_bad, p->stream)) != cudaSuccess ||
-          (e = cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, p->stream)) != cudaSuccess ||
+  // row-tile table of the register-blocked back projector (k_bp_tap); optional: without
+  // it (no memory, a detector beyond its bins) those launch shapes fall back to others
+  if (const long long nt = gt::tap_entries(D.N, D.nd, D.nang)) {
+    const size_t off_f = align256(sizeof(unsigned) * nt);
+    if (cudaMalloc(&p->tiles, off_f + sizeof(float4) * nt) == cudaSuccess) {
+      unsigned *hdr = (unsigned *)p->tiles;
+      float4 *frac = (float4 *)((char *)p->tiles + off_f);
+      if ((e = gt::launch_tap_fill(p->ofs, D.N, D.nd, D.nang, hdr, frac, p->stream)) != cudaSuccess ||
           (e = cudaStreamSynchronize(p->stream)) != cudaSuccess)
         return fail(cuda_err(e, "row table fill", __LINE__));
-      if (!bad) {
-        p->P.row_ent = (const int4 *)p->tiles;
-      } else {  // some lower bins do not step by 0 / 1 along a row: not used
-        cudaFree(p->tiles);
-        p->tiles = nullptr;
-      }
+      p->P.tap_hdr = hdr;
+      p->P.tap_frac = frac;
     } else {
       cudaGetLastError();
       p->tiles = nullptr;
@@ -774,6 +780,10 @@ int gt_problem_create(const gt_desc *desc, gt_problem **out) {
   *out = p;
   return GT_OK;
 }
+
+extern "C" {
+
+int gt_problem_create(const gt_desc *desc, gt_problem **out) { return create_problem(desc, true, out); }
 
 void gt_problem_destroy(gt_problem *p) {
   if (!p) return;
@@ -801,8 +811,8 @@ int gt_set_data(gt_problem *p, const float *f_host, int make_feasible) {
   CK(cudaSetDevice(p->device));
   const gt::Dims &d = p->d;
   const int nb1 = d.nd * d.nang;
-  CK(cudaMemcpyAsync(p->stage, f_host, sizeof(float) * d.nbin, cudaMemcpyHostToDevice, p->stream));
-  CK(gt::launch_transpose(p->stage, p->f, d.S, nb1, p->stream));
+  CK(cudaMemcpyAsync(p->stage, f_host, sizeof(float) * (size_t)nb1 * p->Sr, cudaMemcpyHostToDevice, p->stream));
+  CK(gt::launch_transpose(p->stage, p->f, p->Sr, nb1, nb1, d.S, p->stream));  // padding slices stay zero
   if (make_feasible) {
     // Make_function_feasible (3-D :860-870): bins the all-ones slice does not reach
     // (R 1 <= 0) are zeroed in every slice.  ku is free scratch here.
@@ -834,7 +844,10 @@ int gt_set_data(gt_problem *p, const float *f_host, int make_feasible) {
     const int rc = upload_mu_eff(p);
     if (rc) return rc;
   }
-  CK(cudaMemcpyAsync(p->mu64, p->mu.data(), sizeof(double) * d.C, cudaMemcpyHostToDevice, p->stream));
+  std::vector<double> m64(p->mu);
+  m64.resize(d.C + kMuPad, 1.0);
+  CK(cudaMemcpyAsync(p->mu64, m64.data(), sizeof(double) * m64.size(), cudaMemcpyHostToDevice, p->stream));
+  CK(cudaStreamSynchronize(p->stream));  // m64 is a host buffer
   p->P.ne64 = p->ne;
   // pick the projector launch shapes (uses lambda / ku / kstar as scratch: they are reset below)
   {
@@ -902,10 +915,10 @@ int gt_get_state(gt_problem *p, int field, float *host) {
   int rc = field_info(p, field, &ptr, &comps, &X);
   if (rc) return rc;
   CK(cudaSetDevice(p->device));
-  const size_t S = p->d.S;
+  const size_t S = p->Sr;
   for (int k = 0; k < comps; ++k) {
     const size_t plane = (field == GT_LAMBDA || field == GT_KU || field == GT_DATA) ? p->d.nbin : p->d.vol;
-    CK(gt::launch_transpose(ptr + k * plane, p->stage, (int)X, (int)S, p->stream));
+    CK(gt::launch_transpose(ptr + k * plane, p->stage, (int)X, (int)S, p->d.S, (int)X, p->stream));
     CK(cudaMemcpyAsync(host + k * X * S, p->stage, sizeof(float) * X * S, cudaMemcpyDeviceToHost, p->stream));
   }
   CK(cudaStreamSynchronize(p->stream));
@@ -919,10 +932,10 @@ int gt_get_output_f64(gt_problem *p, int field, double *host) {
   CK(cudaSetDevice(p->device));
   const bool img = field == GT_U;
   const int A = img ? p->d.N : p->d.nang, B = img ? p->d.N : p->d.nd;
-  const size_t n = (size_t)A * B * p->d.S;
+  const size_t n = (size_t)A * B * p->Sr;
   double *tmp = nullptr;
   CK(cudaMallocAsync(&tmp, sizeof(double) * n, p->stream));
-  cudaError_t e = gt::launch_output_f64(img ? p->u : p->ku, tmp, A, B, p->d.C, p->d.Nz, img ? 0 : 1, p->stream);
+  cudaError_t e = gt::launch_output_f64(img ? p->u : p->ku, tmp, A, B, p->d.C, p->d.Nz, p->d.S, img ? 0 : 1, p->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(host, tmp, sizeof(double) * n, cudaMemcpyDeviceToHost, p->stream);
   const cudaError_t ef = cudaFreeAsync(tmp, p->stream);
   if (e == cudaSuccess) e = ef;
@@ -937,11 +950,11 @@ int gt_set_state(gt_problem *p, int field, const float *host) {
   int rc = field_info(p, field, &ptr, &comps, &X);
   if (rc) return rc;
   CK(cudaSetDevice(p->device));
-  const size_t S = p->d.S;
+  const size_t S = p->Sr;
   for (int k = 0; k < comps; ++k) {
     const size_t plane = (field == GT_LAMBDA || field == GT_KU || field == GT_DATA) ? p->d.nbin : p->d.vol;
     CK(cudaMemcpyAsync(p->stage, host + k * X * S, sizeof(float) * X * S, cudaMemcpyHostToDevice, p->stream));
-    CK(gt::launch_transpose(p->stage, ptr + k * plane, (int)S, (int)X, p->stream));
+    CK(gt::launch_transpose(p->stage, ptr + k * plane, (int)S, (int)X, (int)X, p->d.S, p->stream));
   }
   if (field == GT_U && p->ulo) CK(cudaMemsetAsync(p->ulo, 0, sizeof(float) * p->d.vol, p->stream));
   CK(cudaStreamSynchronize(p->stream));
@@ -954,10 +967,10 @@ int gt_get_state_device(gt_problem *p, int field, float *dev) {
   int rc = field_info(p, field, &ptr, &comps, &X);
   if (rc) return rc;
   CK(cudaSetDevice(p->device));
-  const size_t S = p->d.S;
+  const size_t S = p->Sr;
   for (int k = 0; k < comps; ++k) {
     const size_t plane = (field == GT_LAMBDA || field == GT_KU || field == GT_DATA) ? p->d.nbin : p->d.vol;
-    CK(gt::launch_transpose(ptr + k * plane, dev + k * X * S, (int)X, (int)S, p->stream));
+    CK(gt::launch_transpose(ptr + k * plane, dev + k * X * S, (int)X, (int)S, p->d.S, (int)X, p->stream));
   }
   return GT_OK;
 }
@@ -968,10 +981,10 @@ int gt_set_state_device(gt_problem *p, int field, const float *dev) {
   int rc = field_info(p, field, &ptr, &comps, &X);
   if (rc) return rc;
   CK(cudaSetDevice(p->device));
-  const size_t S = p->d.S;
+  const size_t S = p->Sr;
   for (int k = 0; k < comps; ++k) {
     const size_t plane = (field == GT_LAMBDA || field == GT_KU || field == GT_DATA) ? p->d.nbin : p->d.vol;
-    CK(gt::launch_transpose(dev + k * X * S, ptr + k * plane, (int)S, (int)X, p->stream));
+    CK(gt::launch_transpose(dev + k * X * S, ptr + k * plane, (int)S, (int)X, (int)X, p->d.S, p->stream));
   }
   if (field == GT_U && p->ulo) CK(cudaMemsetAsync(p->ulo, 0, sizeof(float) * p->d.vol, p->stream));
   return GT_OK;
@@ -1007,10 +1020,10 @@ void *gt_problem_stream(gt_problem *p) { return p ? (void *)p->stream : nullptr;
 
 int gt_set_tuning(gt_problem *p, int fwd_cfg, int bp_cfg) {
   if (!p) return set_err(GT_ERR_ARG, "null argument");
-  if (fwd_cfg < 0 || fwd_cfg >= gt::num_proj_configs(p->d.S, 0) || bp_cfg < 0 ||
-      bp_cfg >= gt::num_proj_configs(p->d.S, 1))
+  if (fwd_cfg < 0 || fwd_cfg >= gt::num_proj_configs(p->Sr, 0) || bp_cfg < 0 ||
+      bp_cfg >= gt::num_proj_configs(p->Sr, 1))
     return set_err(GT_ERR_ARG, "launch configuration out of range (%d forward, %d back-projection configurations)",
-                   gt::num_proj_configs(p->d.S, 0), gt::num_proj_configs(p->d.S, 1));
+                   gt::num_proj_configs(p->Sr, 0), gt::num_proj_configs(p->Sr, 1));
   CK(cudaSetDevice(p->device));
   CK(cudaStreamSynchronize(p->stream));
   p->P.fwd_cfg = fwd_cfg;
@@ -1734,7 +1747,7 @@ int gt_subs_create(const gt_subs_desc *D, gt_subs **out) {
   d.stepsize = D->stepsize; d.alpha0 = D->alpha0; d.alpha1 = D->alpha1; d.mu = D->mu;
   d.discrepancy = D->discrepancy; d.regularisation = D->regularisation; d.coupling = D->coupling;
   d.normest = 1.0; d.device = D->device; d.stream = D->stream; d.autotune = 0;
-  int rc = gt_problem_create(&d, &s->p);
+  int rc = create_problem(&d, false, &s->p);
   if (rc) { delete s; return rc; }
   s->p->lsqr = 36.0;
   gt_problem *p = s->p;
@@ -1842,10 +1855,10 @@ int gt_subs_set_data(gt_subs *s, const float *f0, const float *f1, int make_feas
   // host layout [S][bins] -> device [bins][S]
   if (s->C0) {
     CK(cudaMemcpyAsync(p->stage, f0, 4 * nb0, cudaMemcpyHostToDevice, p->stream));
-    CK(gt::launch_transpose(p->stage, s->f0, s->S0, s->nang0 * nd0, p->stream));
+    CK(gt::launch_transpose(p->stage, s->f0, s->S0, s->nang0 * nd0, s->nang0 * nd0, s->S0, p->stream));
   }
   CK(cudaMemcpyAsync(p->stage, f1, 4 * nblo, cudaMemcpyHostToDevice, p->stream));
-  CK(gt::launch_transpose(p->stage, s->f1, s->S1lo, s->nang1 * s->nd1, p->stream));
+  CK(gt::launch_transpose(p->stage, s->f1, s->S1lo, s->nang1 * s->nd1, s->nang1 * s->nd1, s->S1lo, p->stream));
   if (make_feasible) {
     // Make_function_feasible (3dsubsample :466-476): bins where the projection of the
     // all-ones slice is <= 0 are zeroed (the low-resolution data uses the mask of the
@@ -1969,7 +1982,7 @@ int gt_subs_get(gt_subs *s, int which, float *host) {
     default: return set_err(GT_ERR_ARG, "unknown field %d", which);
   }
   if (cols == 0) return GT_OK;
-  CK(gt::launch_transpose(src, p->stage, rows, cols, p->stream));
+  CK(gt::launch_transpose(src, p->stage, rows, cols, cols, rows, p->stream));
   CK(cudaMemcpyAsync(host, p->stage, 4 * (size_t)rows * cols, cudaMemcpyDeviceToHost, p->stream));
   CK(cudaStreamSynchronize(p->stream));
   return GT_OK;

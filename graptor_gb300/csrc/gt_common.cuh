@@ -25,7 +25,8 @@ enum { UNCORR = 0, FROB = 1, NUCL = 2 };
 
 struct Dims {
   int dim;     // 2 or 3
-  int N, Nz, C, S;
+  int N, Nz, C;
+  int S;       // slice values per pixel / bin in memory: C*Nz and padding (zero slices at the end)
   int nd, nang;
   size_t vol;  // N*N*S
   size_t nbin; // nd*nang*S
@@ -48,8 +49,8 @@ struct IterParams {
   const int2 *ray_ent;         // (pixel, weight bits) entries of all rays
   const long long *run_start;  // [nang*ceil(nd/3) + 1] offsets of the 3-bin run table (null: none)
   const int4 *run_ent;         // (pixel, weight bits of bins i0, i0+1, i0+2) entries of all runs
-  const int2 *bp_tab;          // [N*N][nang] (floor bin, fraction bits) of the back projection (or null)
-  const int4 *row_ent;           // [N][ceil(N/4)][nang][3] back-projection row-tile entries (or null)
+  const unsigned *tap_hdr;     // [N][ceil(N/4)][nang] row tiles of the back projection: first bin and step pattern (or null)
+  const float4 *tap_frac;      // [N][ceil(N/4)][nang] interpolation fractions of their 4 pixels
   const float *mu;       // [C] mu (KL) or mu/(sigma+mu) (L2)
   float *u, *ubar;       // [vol]
   float *p, *pbar, *v;   // [K][vol]

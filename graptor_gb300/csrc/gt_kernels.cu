@@ -1742,91 +1742,6 @@ __device__ __forceinline__ void radon_ad_pixel(const float *__restrict__ lam, si
   }
 }
 
-// Back-projection table: per (pixel, angle) the detector bin floor(t) and the
-// interpolation fraction p of radon_ad (3-D :832-839), computed once per problem
-// with the reference's arithmetic; il = INT_MIN marks t outside (-1, nd).
-__global__ void k_bp_table(const float4 *__restrict__ ofs, int N, int nd, int nang, int2 *__restrict__ tab) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)N * N * nang) return;
-  const int pix = (int)(t / nang), j = (int)(t - (long long)pix * nang);
-  const int y = pix / N, x = pix - y * N;
-  const float4 o = __ldg(ofs + j);
-  const float tt = __fadd_rn(__fadd_rn(__fmul_rn((float)x, o.x), __fmul_rn((float)y, o.y)), o.z);
-  int2 e = make_int2(INT_MIN, 0);
-  if (tt > -1.f && tt < (float)nd) {
-    const float fl = floorf(tt);
-    e = make_int2((int)fl, __float_as_int(fminf(__fsub_rn(tt, fl), 0x1.fffffep-1f)));
-  }
-  tab[t] = e;
-}
-
-template <int VW, bool EXACT>
-__device__ __forceinline__ void bp_tap(float (&acc)[VW], float w, const float (&v)[VW]) {
-#pragma unroll
-  for (int k = 0; k < VW; ++k) acc[k] = mac<EXACT>(acc[k], w, v[k]);
-}
-
-template <int VW, bool EXACT, int AU, class SL>
-__device__ __forceinline__ void radon_ad_table(const float *__restrict__ lam, size_t S, int nd, int nang,
-                                               const int2 *__restrict__ tab, const SL &sl,
-                                               float (&acc)[VW]) {
-#pragma unroll
-  for (int k = 0; k < VW; ++k) acc[k] = 0.f;
-  const size_t jstride = (size_t)nd * S;
-  int j = 0;
-  if (AU == 2) {
-    for (; j + 2 <= nang; j += 2) {  // two angles (four taps) in flight, accumulated in order
-      const int2 e0 = __ldg(tab + j), e1 = __ldg(tab + j + 1);
-      float a0[VW], b0[VW], a1[VW], b1[VW];
-      const float *l0 = lam + (size_t)j * jstride, *l1 = l0 + jstride;
-      const bool in0 = e0.x != INT_MIN, in1 = e1.x != INT_MIN;
-      const bool ta0 = in0 && e0.x >= 0, tb0 = in0 && e0.x <= nd - 2;
-      const bool ta1 = in1 && e1.x >= 0, tb1 = in1 && e1.x <= nd - 2;
-      if (ta0) sl.load(l0 + (size_t)e0.x * S, a0);
-      if (tb0) sl.load(l0 + (size_t)(e0.x + 1) * S, b0);
-      if (ta1) sl.load(l1 + (size_t)e1.x * S, a1);
-      if (tb1) sl.load(l1 + (size_t)(e1.x + 1) * S, b1);
-      const float p0 = __int_as_float(e0.y), p1 = __int_as_float(e1.y);
-      if (ta0) bp_tap<VW, EXACT>(acc, __fsub_rn(1.0f, p0), a0);
-      if (tb0) bp_tap<VW, EXACT>(acc, p0, b0);
-      if (ta1) bp_tap<VW, EXACT>(acc, __fsub_rn(1.0f, p1), a1);
-      if (tb1) bp_tap<VW, EXACT>(acc, p1, b1);
-    }
-  }
-  for (; AU > 2 && j + AU <= nang; j += AU) {  // AU angles (2 AU taps) in flight, accumulated in order
-    int2 e[AU];
-#pragma unroll
-    for (int u = 0; u < AU; ++u) e[u] = __ldg(tab + j + u);
-    float a[AU][VW], b[AU][VW];
-    bool ta[AU], tb[AU];
-#pragma unroll
-    for (int u = 0; u < AU; ++u) {
-      const bool in = e[u].x != INT_MIN;
-      ta[u] = in && e[u].x >= 0;
-      tb[u] = in && e[u].x <= nd - 2;
-      const float *l = lam + (size_t)(j + u) * jstride;
-      if (ta[u]) sl.load(l + (size_t)e[u].x * S, a[u]);
-      if (tb[u]) sl.load(l + (size_t)(e[u].x + 1) * S, b[u]);
-    }
-#pragma unroll
-    for (int u = 0; u < AU; ++u) {
-      const float p = __int_as_float(e[u].y);
-      if (ta[u]) bp_tap<VW, EXACT>(acc, __fsub_rn(1.0f, p), a[u]);
-      if (tb[u]) bp_tap<VW, EXACT>(acc, p, b[u]);
-    }
-  }
-  for (; j < nang; ++j) {
-    const int2 e0 = __ldg(tab + j);
-    if (e0.x != INT_MIN) {
-      const float *l0 = lam + (size_t)j * jstride;
-      const float p0 = __int_as_float(e0.y);
-      float a0[VW], b0[VW];
-      if (e0.x >= 0) { sl.load(l0 + (size_t)e0.x * S, a0); bp_tap<VW, EXACT>(acc, __fsub_rn(1.0f, p0), a0); }
-      if (e0.x <= nd - 2) { sl.load(l0 + (size_t)(e0.x + 1) * S, b0); bp_tap<VW, EXACT>(acc, p0, b0); }
-    }
-  }
-}
-
 // update_u (3-D :706-729, 2-D :340-357) + update_p (3-D :734-757, 2-D :359-376) +
 // extrapolation and swap (:1217-1221) for UW consecutive slices from s0.
 // PART selects the halves: PART_U the u / ubar half (needs K* lambda), PART_P the
@@ -1837,9 +1752,15 @@ template <int DIM, bool TGV, int UW, int PART = PART_ALL>
 __device__ __forceinline__ void primal_update(const IterParams &P, int x, int y, int s0, const float (&kstar)[UW]) {
   const Dims d = P.d;
   const size_t S = d.S, rowS = (size_t)d.N * S, vol = d.vol, i = ((size_t)y * d.N + x) * S + s0;
-  int z[UW];
+  // first / last slice of the channel; a padding slice (s >= C Nz) has no neighbours, so it stays zero
+  bool fz[UW], lz[UW];
 #pragma unroll
-  for (int k = 0; k < UW; ++k) z[k] = (DIM == 3) ? (s0 + k) % d.Nz : 0;
+  for (int k = 0; k < UW; ++k) {
+    const int z = (DIM == 3) ? (s0 + k) % d.Nz : 0;
+    const bool pad = s0 + k >= d.C * d.Nz;
+    fz[k] = pad || z == 0;
+    lz[k] = pad || z == d.Nz - 1;
+  }
   const float *__restrict__ v = P.v;
 
   if (PART != PART_P) {
@@ -1853,7 +1774,7 @@ __device__ __forceinline__ void primal_update(const IterParams &P, int x, int y,
   float c[UW], cprev = 0.f;
   if (DIM == 3) {
     ldw<UW>(v + 2 * vol + i, c);
-    if (z[0] > 0) cprev = v[2 * vol + i - 1];
+    if (!fz[0]) cprev = v[2 * vol + i - 1];
   }
   float lo[UW], lon[UW];  // the low parts of u (precise primal mode, P.ulo set)
   if (P.ulo) ldw<UW>(P.ulo + i, lo);
@@ -1867,8 +1788,8 @@ __device__ __forceinline__ void primal_update(const IterParams &P, int x, int y,
     float sum;
     if (DIM == 3) {
       float ck = c[k];
-      if (z[k] == d.Nz - 1) ck = 0.f;
-      if (z[k] > 0) ck -= (k > 0 ? c[k - 1] : cprev);
+      if (lz[k]) ck = 0.f;
+      if (!fz[k]) ck -= (k > 0 ? c[k - 1] : cprev);
       ck /= P.stepsize;
       sum = ak + bk + ck - P.norming * kstar[k];
     } else {
@@ -1915,7 +1836,7 @@ __device__ __forceinline__ void primal_update(const IterParams &P, int x, int y,
       float wc[UW], wcnext = 0.f;
       if (DIM == 3) {
         ldw<UW>(w + rz[k] * vol + i, wc);
-        if (z[UW - 1] < d.Nz - 1) wcnext = w[rz[k] * vol + i + UW];
+        if (!lz[UW - 1]) wcnext = w[rz[k] * vol + i + UW];
       }
 #pragma unroll
       for (int e = 0; e < UW; ++e) {
@@ -1927,7 +1848,7 @@ __device__ __forceinline__ void primal_update(const IterParams &P, int x, int y,
         float r;
         if (DIM == 3) {
           r = p_step3(po[e], vk[e], wa[e], wan[e], wb[e], wbn[e], wc[e], e < UW - 1 ? wc[e + 1] : wcnext, x == 0,
-                      x < d.N - 1, y == 0, y < d.N - 1, z[e] == 0, z[e] < d.Nz - 1, P.tau, P.stepsize);
+                      x < d.N - 1, y == 0, y < d.N - 1, fz[e], !lz[e], P.tau, P.stepsize);
         } else {
           r = po[e] + P.tau * (vk[e] + A + B);
         }
@@ -1940,103 +1861,24 @@ __device__ __forceinline__ void primal_update(const IterParams &P, int x, int y,
   }
 }
 
-// Back projection of R consecutive pixels of one row at once.  Along a row the
-// detector coordinate moves by X = cos(angle) per pixel (|X| <= 1), so the R
-// pixels' taps span about R|X| + 2 bins: the pixels are visited in the order in
-// which their bins increase and the two current taps slide along, each bin loaded
-// once per angle.  Every pixel adds its taps in the reference's order (angles
-// ascending, lower tap then upper tap) with the reference's interpolation weights.
-template <int VW, int R, bool REV>
-__device__ __forceinline__ void bp_run_angle(const float *__restrict__ lj, size_t S, int nd, float fnd, const float4 o,
-                                             int x0, float yf, int N, const Slices<VW> &sl, float (&acc)[R][VW]) {
-  int cur = -3;  // bins held: A = cur, B = cur + 1
-  float A[VW], Bv[VW];
-#pragma unroll
-  for (int k = 0; k < VW; ++k) { A[k] = 0.f; Bv[k] = 0.f; }
-#pragma unroll
-  for (int rr = 0; rr < R; ++rr) {
-    const int r = REV ? R - 1 - rr : rr;
-    if (x0 + r >= N) continue;
-    const float xf = (float)(x0 + r);
-    const float tt = __fadd_rn(__fadd_rn(__fmul_rn(xf, o.x), __fmul_rn(yf, o.y)), o.z);
-    if (!(tt > -1.f && tt < fnd)) continue;
-    const float fl = floorf(tt);
-    const float p = fminf(__fsub_rn(tt, fl), 0x1.fffffep-1f);
-    const float q = __fsub_rn(1.0f, p);
-    const int il = (int)fl;
-    if (il != cur) {
-      if (il == cur + 1) {
-#pragma unroll
-        for (int k = 0; k < VW; ++k) A[k] = Bv[k];
-      } else if (il >= 0) {
-        sl.load(lj + (size_t)il * S, A);
-      }
-      if (il <= nd - 2) sl.load(lj + (size_t)(il + 1) * S, Bv);
-      cur = il;
-    }
-    if (il >= 0) {
-#pragma unroll
-      for (int k = 0; k < VW; ++k) acc[r][k] = __fmaf_rn(q, A[k], acc[r][k]);
-    }
-    if (il <= nd - 2) {
-#pragma unroll
-      for (int k = 0; k < VW; ++k) acc[r][k] = __fmaf_rn(p, Bv[k], acc[r][k]);
-    }
-  }
-}
-
-template <int VW, int R>
-__global__ void __launch_bounds__(256) k_bp_run(const IterParams P) {
-  const Dims d = P.d;
-  const int nrun = (d.N + R - 1) / R;
-  long long unit;
-  Slices<VW> sl;
-  if (!map_thread<VW>((long long)d.N * nrun, d.S, unit, sl)) return;
-  const int y = (int)(unit / nrun), x0 = (int)(unit - (long long)y * nrun) * R;
-  float acc[R][VW];
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int k = 0; k < VW; ++k) acc[r][k] = 0.f;
-  const float fnd = (float)d.nd, yf = (float)y;
-  for (int j = 0; j < d.nang; ++j) {
-    const float4 o = __ldg(P.ofs + j);
-    const float *lj = P.lam + (size_t)j * d.nd * d.S;
-    if (o.x < 0.f) bp_run_angle<VW, R, true>(lj, d.S, d.nd, fnd, o, x0, yf, d.N, sl, acc);
-    else bp_run_angle<VW, R, false>(lj, d.S, d.nd, fnd, o, x0, yf, d.N, sl, acc);
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-    if (x0 + r < d.N) sl.store(P.kstar + ((size_t)y * d.N + x0 + r) * d.S, acc[r]);
-}
-
 // k_bp: back projection K* lambda of every (pixel, slice) into P.kstar; it only
 // needs lambda, so it runs beside k_dual.
-template <int VW, int AU, bool TAB, bool WL = false, int UA = 2>
+template <int VW, int AU, int UA = 2>
 __device__ __forceinline__ void bp_body(const IterParams &P, long long bid) {
   const Dims d = P.d;
   long long unit;
-  typename std::conditional<WL, SlicesWL, Slices<VW>>::type sl;
-  if constexpr (WL) {
-    static_assert(VW == 1 && !TAB, "one slice per lane, geometry on the fly");
-    if (!map_thread_wl((long long)d.N * d.N, d.S, unit, sl)) return;
-  } else {
-    if (!map_thread<VW>(bid, (long long)d.N * d.N, d.S, unit, sl)) return;
-  }
+  Slices<VW> sl;
+  if (!map_thread<VW>(bid, (long long)d.N * d.N, d.S, unit, sl)) return;
   const int pix = (int)unit;
   float acc[VW];
-  if (TAB && P.bp_tab) {
-    radon_ad_table<VW, false, AU>(P.lam, d.S, d.nd, d.nang, P.bp_tab + (size_t)pix * d.nang, sl, acc);
-  } else {
-    const int y = pix / d.N, x = pix - y * d.N;
-    radon_ad_pixel<VW, false, AU, decltype(sl), UA>(P.lam, d.S, d.nd, d.nang, P.ofs, (float)x, (float)y, sl, acc);
-  }
+  const int y = pix / d.N, x = pix - y * d.N;
+  radon_ad_pixel<VW, false, AU, Slices<VW>, UA>(P.lam, d.S, d.nd, d.nang, P.ofs, (float)x, (float)y, sl, acc);
   sl.store(P.kstar + (size_t)pix * d.S, acc);
 }
 
-template <int VW, int AU, bool TAB, bool WL = false, int UA = 2>
+template <int VW, int AU, int UA = 2>
 __global__ void __launch_bounds__(256) k_bp(const IterParams P) {
-  bp_body<VW, AU, TAB, WL, UA>(P, blockIdx.x);
+  bp_body<VW, AU, UA>(P, blockIdx.x);
 }
 
 // k_bp_tma: back projection with the sinogram rows a pixel tile needs staged in
@@ -2250,20 +2092,22 @@ __global__ void k_radon_ad(const float *__restrict__ sino, float *__restrict__ i
 }
 
 // out[c][r] = in[r][c]: host layout [S][X] <-> device layout [X][S], 32x32 tiles,
-// one block per tile (1-D grid, so neither extent is limited to 65535 tiles)
-__global__ void k_transpose(const float *__restrict__ in, float *__restrict__ out, int rows, int cols) {
+// one block per tile (1-D grid, so neither extent is limited to 65535 tiles);
+// ld_in / ld_out: row lengths of in and out (>= cols / rows)
+__global__ void k_transpose(const float *__restrict__ in, float *__restrict__ out, int rows, int cols, int ld_in,
+                            int ld_out) {
   __shared__ float tile[32][33];
   const int tiles_c = (cols + 31) / 32;
   const int tr = blockIdx.x / tiles_c, tc = blockIdx.x - tr * tiles_c;
   const int bx = tc * 32, by = tr * 32;
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
     const int r = by + k, c = bx + threadIdx.x;
-    if (r < rows && c < cols) tile[k][threadIdx.x] = in[(size_t)r * cols + c];
+    if (r < rows && c < cols) tile[k][threadIdx.x] = in[(size_t)r * ld_in + c];
   }
   __syncthreads();
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
     const int r = bx + k, c = by + threadIdx.x;
-    if (r < cols && c < rows) out[(size_t)r * rows + c] = tile[threadIdx.x][k];
+    if (r < cols && c < rows) out[(size_t)r * ld_out + c] = tile[threadIdx.x][k];
   }
 }
 
@@ -2762,8 +2606,8 @@ __global__ void __launch_bounds__(256) k_gap_box(const IterParams P, const float
   const Dims d = P.d;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   double box = 0.0;
-  if (t < (long long)d.vol) {
-    const int pix = (int)(t / d.S), s = (int)(t - (long long)pix * d.S);
+  const int pix = (int)(t / d.S), s = (int)(t - (long long)pix * d.S);
+  if (t < (long long)d.vol && s < d.C * d.Nz) {  // not the padding slices (v~ is not set there)
     const int y = pix / d.N, x = pix - y * d.N, z = s % d.Nz;
     const size_t vol = d.vol, S = d.S, rowS = (size_t)d.N * S, i = (size_t)t;
     double a = vt[i], b = vt[vol + i];
@@ -3153,19 +2997,18 @@ static inline int vec_width(int S) { return (S % 4 == 0) ? 8 : (S % 2 == 0 ? 2 :
 // (slices per lane, ray-table entries in flight) = (8, 4), (8, 8), (4, 4), (4, 8),
 // configs 5..8 = (slices per lane, bins per run) of k_fwd_run = (8, 2), (8, 4),
 // (4, 4), (4, 8);
-// k_bp configs 0..7 = (slices per lane, angles per step, geometry) = (8, 2, table),
-// (8, 4, table), (4, 2, table), (4, 4, table), (8, 1, on the fly), (4, 1, on the fly),
-// (8, 2, on the fly), (4, 2, on the fly); configs 9..12 = (slices per lane,
-// pixels per run) of k_bp_run = (8, 4), (4, 8), (8, 8), (4, 4).  k_fwd config 9 and
-// k_bp config 13: one slice per lane with the 32-slice chunk outermost (SlicesWL),
-// for images and sinograms larger than L2.  k_fwd configs 10, 11: the 3-bin run
+// k_bp configs 0..8 = (slices per lane, angles per step) of the one-pixel kernel = (8, 2),
+// (8, 4), (4, 2), (4, 4), (8, 1), (4, 1), (8, 2), (4, 2), (1, 1); 16 and 17 are 4 with its
+// angle loop unrolled 4x or not at all; 14 and 15 the TMA-staged kernel; 18, 19 and 9
+// the row-tile kernel k_bp_tap with 8, 4 and 2 slices per lane, 10 (and 13), 11, 12 the
+// flat kernel k_bp_flat with 4, 2 and 1 slices per thread (gt_proj.cu).  k_fwd config 9:
+// one slice per lane with the 32-slice chunk outermost (SlicesWL), for images larger
+// than L2.  k_fwd configs 10, 11: the 3-bin run
 // table (k_fwd_rt) with (slices per lane, entries in flight) = (8, 4), (4, 8);
 // configs 12, 13: (8, 8) and (8, 4) with registers capped for 5 / 6 resident blocks.
-// k_bp configs 18, 19: the register-blocked row-tile kernel (gt_proj.cu) with 4 or
-// 2 slices per lane.
 // Otherwise one fixed shape with 2 or 1 slices per thread.
-// One more candidate each: one slice per thread (k_fwd config 4, k_bp config 8),
-// which keeps all lanes busy when S is small.
+// One more candidate of k_fwd: one slice per thread (config 4), which keeps all lanes
+// busy when S is small.
 int num_proj_configs(int S, int which) {
   if (S % 4 != 0) return 1;
   return which == 0 ? 20 : 20;  // configs 4 / 8 (one slice per thread) stay candidates for every S
@@ -3208,7 +3051,8 @@ static void fwd_run(const IterParams &P, int disc, cudaStream_t st) {
   else k_fwd_run<L2, VW, R><<<g, 256, 0, st>>>(P);
 }
 
-cudaError_t launch_bp_row(const IterParams &P, int shape, cudaStream_t st);
+cudaError_t launch_bp_tap(const IterParams &P, int vw, cudaStream_t st);
+cudaError_t launch_bp_flat(const IterParams &P, int vw, cudaStream_t st);
 
 cudaError_t launch_fwd(const IterParams &P, int disc, cudaStream_t st) {
   const int S = P.d.S;
@@ -3249,63 +3093,52 @@ cudaError_t launch_fwd(const IterParams &P, int disc, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-template <int VW, int AU, bool TAB = true>
+template <int VW, int AU, int UA = 2>
 static void bp_vw(const IterParams &P, cudaStream_t st) {
-  k_bp<VW, AU, TAB><<<blocks_for(threads_for<VW>((long long)P.d.N * P.d.N, P.d.S), 256), 256, 0, st>>>(P);
+  k_bp<VW, AU, UA><<<blocks_for(threads_for<VW>((long long)P.d.N * P.d.N, P.d.S), 256), 256, 0, st>>>(P);
 }
 
-template <int UA>
-static void bp_ua(const IterParams &P, cudaStream_t st) {
-  k_bp<8, 1, false, false, UA><<<blocks_for(threads_for<8>((long long)P.d.N * P.d.N, P.d.S), 256), 256, 0, st>>>(P);
-}
-
-static void bp_wl(const IterParams &P, cudaStream_t st) {
-  k_bp<1, 1, false, true><<<blocks_for(threads_for_wl((long long)P.d.N * P.d.N, P.d.S), 256), 256, 0, st>>>(P);
-}
-
-template <int VW, int R>
-static void bp_run(const IterParams &P, cudaStream_t st) {
-  const long long units = (long long)P.d.N * ((P.d.N + R - 1) / R);
-  k_bp_run<VW, R><<<blocks_for(threads_for<VW>(units, P.d.S), 256), 256, 0, st>>>(P);
+// default back-projection shape (no autotuning).  256^2 and smaller, us of k_bp_tap with
+// 8 / 4 / 2 slices per lane and k_bp_flat with 4 slices per thread: 16 slices (177^2, 45
+// angles) 73 / 45 / 41 / 18; 32 (64^2, 71) 39 / 33 / 31 / 14; 40 (101^2, 45) 33 / 25 / 25 / 17;
+// 64 (128^2, 71) 74 / 41 / 36 / 45; 92 (128^2, 71) 74 / 43 / 62 / 62; 240 (256^2, 71)
+// 213 / 242 / 362 / 558; 384 (512^2, 141) 2912 / 2628 / 4050 / 6856 (there 8 per lane leave
+// a quarter of the lanes idle).
+int default_bp_shape(int S) {
+  if (S <= 48) return 10;
+  if (S <= 64) return 9;
+  const int w8 = (S + 255) / 256 * 256, w4 = (S + 127) / 128 * 128;
+  return S >= 192 && w8 <= w4 + w4 / 8 ? 18 : 19;
 }
 
 cudaError_t launch_bp(const IterParams &P, cudaStream_t st) {
   const int S = P.d.S;
-  if (S % 4 == 0 && (P.bp_cfg == 18 || P.bp_cfg == 19)) {
-    // register-blocked row-tile kernel (gt_proj.cu); without its table the one-angle shape
-    if (P.row_ent) return launch_bp_row(P, P.bp_cfg - 18, st);
-    bp_vw<8, 1, false>(P, st);
-    return cudaGetLastError();
-  }
-  if (S % 4 == 0) {
-    switch (P.bp_cfg) {
-      case 1: bp_vw<8, 4>(P, st); break;
-      case 2: bp_vw<4, 2>(P, st); break;
-      case 3: bp_vw<4, 4>(P, st); break;
-      case 4: bp_vw<8, 1, false>(P, st); break;
-      case 5: bp_vw<4, 1, false>(P, st); break;
-      case 6: bp_vw<8, 2, false>(P, st); break;
-      case 7: bp_vw<4, 2, false>(P, st); break;
-      case 8: bp_vw<1, 1, false>(P, st); break;
-      case 9: bp_run<8, 4>(P, st); break;
-      case 10: bp_run<4, 8>(P, st); break;
-      case 11: bp_run<8, 8>(P, st); break;
-      case 12: bp_run<4, 4>(P, st); break;
-      case 13: bp_wl(P, st); break;
-      case 14:  // no descriptor: the one-angle shape (identical sums)
-        if (P.bp_tmap) bp_tma<4>(P, st); else bp_vw<8, 1, false>(P, st);
-        break;
-      case 15:
-        if (P.bp_tmap_wide) bp_tma<8>(P, st); else bp_vw<8, 1, false>(P, st);
-        break;
-      case 16: bp_ua<4>(P, st); break;  // the one-angle shape (4) with its angle loop unrolled 4x
-      case 17: bp_ua<1>(P, st); break;  // ... not unrolled (fewer instructions in flight, faster)
-      default: bp_vw<8, 2>(P, st); break;
-    }
-  } else if (S % 2 == 0) {
-    bp_vw<2, 2>(P, st);
-  } else {
-    bp_vw<1, 2>(P, st);
+  if (S % 4 != 0) return launch_bp_flat(P, S % 2 == 0 ? 2 : 1, st);
+  switch (P.bp_cfg) {
+    case 0: bp_vw<8, 2>(P, st); break;
+    case 1: bp_vw<8, 4>(P, st); break;
+    case 2: bp_vw<4, 2>(P, st); break;
+    case 3: bp_vw<4, 4>(P, st); break;
+    case 5: bp_vw<4, 1>(P, st); break;
+    case 6: bp_vw<8, 2>(P, st); break;
+    case 7: bp_vw<4, 2>(P, st); break;
+    case 8: bp_vw<1, 1>(P, st); break;
+    case 10: case 13: return launch_bp_flat(P, 4, st);
+    case 11: return launch_bp_flat(P, 2, st);
+    case 12: return launch_bp_flat(P, 1, st);
+    case 14:  // no descriptor: the one-angle shape (identical sums)
+      if (P.bp_tmap) bp_tma<4>(P, st); else bp_vw<8, 1>(P, st);
+      break;
+    case 15:
+      if (P.bp_tmap_wide) bp_tma<8>(P, st); else bp_vw<8, 1>(P, st);
+      break;
+    case 16: bp_vw<8, 1, 4>(P, st); break;  // the one-angle shape (4) with its angle loop unrolled 4x
+    case 17: bp_vw<8, 1, 1>(P, st); break;  // ... not unrolled
+    case 9: case 18: case 19:  // without the row-tile table the one-angle shape
+      if (P.tap_hdr) return launch_bp_tap(P, P.bp_cfg == 18 ? 8 : P.bp_cfg == 19 ? 4 : 2, st);
+      bp_vw<8, 1>(P, st);
+      break;
+    default: bp_vw<8, 1>(P, st); break;  // 4
   }
   return cudaGetLastError();
 }
@@ -3356,9 +3189,9 @@ __global__ void __launch_bounds__(256) k_bp_batch(const BatchTab T) {
   const IterParams P = T.P[k];
   const long long bid = (long long)blockIdx.x - __ldg(T.start + k);
   const int sh = __ldg(T.shape + k);
-  if (sh == 2) bp_body<8, 1, false, false, 1>(P, bid);
-  else if (sh == 1) bp_body<4, 1, false, false, 1>(P, bid);
-  else bp_body<1, 1, false>(P, bid);
+  if (sh == 2) bp_body<8, 1, 1>(P, bid);
+  else if (sh == 1) bp_body<4, 1, 1>(P, bid);
+  else bp_body<1, 1>(P, bid);
 }
 
 template <int DIM, bool TGV>
@@ -3557,19 +3390,14 @@ cudaError_t launch_gap_pass2(const IterParams &P, const float *vt, double theta,
   return cudaGetLastError();
 }
 
-cudaError_t launch_bp_table(const float4 *ofs, int N, int nd, int nang, int2 *tab, cudaStream_t st) {
-  k_bp_table<<<blocks_for((long long)N * N * nang, 256), 256, 0, st>>>(ofs, N, nd, nang, tab);
-  return cudaGetLastError();
-}
-
-// A state field in the device layout in[(a B + b) S + c Nz + z] to float64 in the
+// A state field in the device layout in[(a B + b) Sd + c Nz + z] to float64 in the
 // reference's output layout: mode 0 (the image, a = y, b = x) out[c][b][a][z]
 // (Solution [C][x][y][z]); mode 1 (the sinogram, a = angle, b = bin)
 // out[c][a][z][b] (Sinogram [C][nang][Nz][nd]).  Mode 0 runs over (a, b, s) with
 // s fastest, mode 1 over (a, s, b) with b fastest, so the float64 writes are
 // contiguous (runs of Nz, resp. B).
 __global__ void k_output_f64(const float *__restrict__ in, double *__restrict__ out, int A, int B, int C, int Nz,
-                             int mode) {
+                             int Sd, int mode) {
   const long long S = (long long)C * Nz;
   const long long n = (long long)A * B * S;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
@@ -3586,22 +3414,24 @@ __global__ void k_output_f64(const float *__restrict__ in, double *__restrict__ 
       a = as / S;
     }
     const long long c = s / Nz, z = s - c * Nz;
-    const float v = __ldg(in + (a * B + b) * S + s);
+    const float v = __ldg(in + (a * B + b) * Sd + s);
     const long long o = mode == 0 ? ((c * B + b) * A + a) * Nz + z : ((c * A + a) * Nz + z) * B + b;
     out[o] = (double)v;
   }
 }
 
-cudaError_t launch_output_f64(const float *in, double *out, int A, int B, int C, int Nz, int mode, cudaStream_t st) {
+cudaError_t launch_output_f64(const float *in, double *out, int A, int B, int C, int Nz, int Sd, int mode,
+                              cudaStream_t st) {
   const long long n = (long long)A * B * C * Nz;
   const unsigned g = (unsigned)std::min<long long>((n + 255) / 256, 152LL * 16);
-  k_output_f64<<<g, 256, 0, st>>>(in, out, A, B, C, Nz, mode);
+  k_output_f64<<<g, 256, 0, st>>>(in, out, A, B, C, Nz, Sd, mode);
   return cudaGetLastError();
 }
 
-cudaError_t launch_transpose(const float *in, float *out, int rows, int cols, cudaStream_t st) {
+cudaError_t launch_transpose(const float *in, float *out, int rows, int cols, int ld_in, int ld_out,
+                             cudaStream_t st) {
   const long long tiles = (long long)((rows + 31) / 32) * ((cols + 31) / 32);
-  k_transpose<<<(unsigned)tiles, dim3(32, 8), 0, st>>>(in, out, rows, cols);
+  k_transpose<<<(unsigned)tiles, dim3(32, 8), 0, st>>>(in, out, rows, cols, ld_in, ld_out);
   return cudaGetLastError();
 }
 

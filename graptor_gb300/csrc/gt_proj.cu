@@ -1,157 +1,107 @@
-// Register-blocked back projector of the solver iteration (sm_103a).
+// Register-blocked back projector of the solver iteration (sm_103a): back projection
+// `radon_ad`, radon_tgv_primal_dual_3d.py:818-844.
 //
-// The back-projection kernels of gt_kernels.cu give each warp one pixel and S
-// slice values per lane group; both interpolation taps of every (pixel, angle)
-// pair are loaded from L1 for that pixel alone, one load per two multiply-adds.
-// Here (k_bp_row, back projection `radon_ad`, radon_tgv_primal_dual_3d.py:818-844)
-// a warp owns 4 adjacent pixels of a row: per angle their taps lie on at most 5
-// consecutive detector bins, loaded once and shared, so the L1 traffic halves.
+// What bounds it: every (pixel, angle) pair reads two detector taps of S slice values, and
+// the loads' way back to the registers (128 bytes a clock and SM, broadcasts included)
+// is the limit, then instruction issue.  So a loaded tap is shared between pixels, the
+// geometry is kept as small as it can be, and the multiply-adds are done two at a time
+// (fma.rn.f32x2, each half rounding as a scalar one).
 //
-// The geometry is fixed for a solve, so it is computed once per problem into a
-// table with the reference's arithmetic.  Which accumulator a product goes to must
-// be known at compile time (registers cannot be indexed at run time): the lower
-// bins of 4 adjacent pixels of a row step by 0 or 1 (the detector coordinate
-// moves by |cos| <= 1 per pixel), one of 8 step patterns per direction, and the
-// kernel branches once per angle on the pattern.  Every pixel adds its two taps
-// in the reference's order with the reference's weights (fused multiply-add, as
-// the solver's other projector shapes); where a tap falls outside the detector
-// the entry pairs the pixel with a zero weight on a bin inside it, and a zero
-// product leaves a sum unchanged, so the iterates are identical to those of the
-// other back-projection shapes.
+// k_bp_tap: a warp owns 4 adjacent pixels of a row and 32 VW slices.  Along a row the
+// detector coordinate moves by |cos| <= 1 per pixel, so the pixels' lower bins step by 0 or
+// 1 -- one of 8 patterns per direction -- and their taps lie on 2 to 5 consecutive bins,
+// each loaded once.  Which accumulator a product goes to must be known at compile time
+// (registers cannot be indexed at run time), so the kernel branches once per angle on
+// the pattern and loads exactly the bins it needs.  A table of 20 bytes per (row tile,
+// angle) holds the first bin with the pattern and the 4 interpolation fractions; the lower
+// weight 1 - p is recomputed.  A first form with both weights and a three-word header
+// (48 bytes, three 16-byte broadcasts against five taps at 4 slices per lane) took
+// 328 us on 256^2 x 60 x 4, 71 angles and 3635 us on 512^2 x 96 x 4, 141 angles; this one
+// takes 213 us (8 slices per lane; 59 % of the write-back path busy, half of the issue
+// slots) and 2628 us (4 per lane).
+//
+// k_bp_flat: a thread owns one pixel and VW slices, threads of a warp run on over pixels.
+// With few slices per pixel a warp per tile leaves lanes idle; here a warp holds
+// several pixels and the geometry is computed on the fly, UA angles at a time so that
+// 2 UA loads are in flight.  64^2, 71 angles, 32 slices: 14.4 us against 26.7 us with
+// one slice per thread; 177^2, 45 angles, 16 slices: 18.5 against 37 us.
+//
+// Every pixel adds its taps in the reference's order (angles ascending, lower tap then
+// upper tap) with the reference's weights, so all shapes give identical iterates.
 #include <cuda_runtime.h>
-
-#include <climits>
 
 #include "gt_common.cuh"
 #include "gt_geom.cuh"
+#include "gt_vec.cuh"
 
 namespace gt {
 
 namespace {
 
-constexpr int ROW_P = 4;            // pixels per back-projection row tile
-constexpr int ROW_NB = ROW_P + 1;   // most consecutive bins their taps span
-constexpr int ROW_WORDS = 3;        // int4 per (row tile, angle) entry
+constexpr int ROW_P = 4;  // pixels per row tile
 
 inline unsigned blocks(long long threads, int bs) { return (unsigned)((threads + bs - 1) / bs); }
 
 // ---------------------------------------------------------------------------
 // row-tile table
 // ---------------------------------------------------------------------------
-// Entry of the row tile (x0 .. x0 + 3, y) and angle o, ROW_WORDS int4:
-// (b0, nb, pattern, 0), the lower-tap weights of its 4 pixels, the upper-tap
-// weights.  Per pixel radon_ad's detector coordinate t = x X + y Y + off, lower
-// bin floor(t) and fraction p (:832-839); taps (floor(t), 1 - p), (floor(t) + 1, p).
-// The reference drops the lower tap at bin -1 and the upper tap at bin nd; the
-// entry pairs the remaining tap with a zero-weight tap on the detector instead
-// ((0, p; 1, 0) and (nd - 2, 0; nd - 1, 1 - p)), so every tap lies in [0, nd - 1].
-// A pixel outside (-1, nd) or outside the image adds nothing: it takes the lower
-// bin of its nearest pixel that does (t is monotone along the row, so such pixels
-// are at the ends) with zero weights.  The lower bins lo_0..lo_3 then step by 0
-// or 1 in one direction: pattern = dir * 8 + steps (bit r: step between pixels r
-// and r + 1, dir 0: lo_r non-decreasing from lo_0 = b0, dir 1: non-increasing to
-// lo_3 = b0).  Returns nb (taps b0 .. b0 + nb - 1), or -1 when the steps are not
-// of that form (the tile kernel is then not used).
-__device__ int row_entry(const float4 o, int x0, int y, int N, int nd, int4 *out) {
+// Header of (row tile (x0 .. x0 + 3, y), angle o): the first bin of the tile's taps in
+// the low 26 bits and pattern = dir * 8 + steps above them (bit r: the lower bin steps
+// between pixels r and r + 1; dir 0: ascending from the first bin, dir 1: descending to it).
+// TAP_EDGE: a tap is off the detector or the bins do not step like that; the kernel then
+// takes each pixel by itself.  TAP_NONE: no pixel is inside (-1, nd).
+constexpr unsigned TAP_EDGE = 1u << 31, TAP_NONE = 0xffffffffu;
+
+// Per pixel radon_ad's detector coordinate t = x X + y Y + off, lower bin floor(t) and
+// fraction p (:832-839), with the reference's arithmetic.
+__device__ unsigned tap_entry(const float4 o, int x0, int y, int N, int nd, float4 *pout) {
   int lo[ROW_P];
-  float wl[ROW_P], wh[ROW_P];
-  bool in[ROW_P];
-  int first = -1, last = -1;
+  float p[ROW_P];
+  int in = 0;
+  bool edge = false;
 #pragma unroll
   for (int r = 0; r < ROW_P; ++r) {
-    const int x = x0 + r;
-    in[r] = false;
-    lo[r] = 0;
-    wl[r] = wh[r] = 0.f;
-    if (x >= N || y >= N) continue;
+    const int x = min(x0 + r, N - 1);  // pixels past the row end repeat its last one (their sums are not stored)
     const float tt = __fadd_rn(__fadd_rn(__fmul_rn((float)x, o.x), __fmul_rn((float)y, o.y)), o.z);
+    lo[r] = 0;
+    p[r] = 0.f;
     if (!(tt > -1.f && tt < (float)nd)) continue;
+    ++in;
     const float fl = floorf(tt);
-    const float p = fminf(__fsub_rn(tt, fl), 0x1.fffffep-1f);
-    const float q = __fsub_rn(1.0f, p);
-    int il = (int)fl;
-    float a = q, b = p;
-    if (il < 0) { il = 0; a = p; b = 0.f; }                  // only the upper tap, at bin 0
-    else if (il > nd - 2) { il = nd - 2; a = 0.f; b = q; }   // only the lower tap, at bin nd - 1
-    in[r] = true;
-    lo[r] = il;
-    wl[r] = a;
-    wh[r] = b;
-    if (first < 0) first = r;
-    last = r;
+    p[r] = fminf(__fsub_rn(tt, fl), 0x1.fffffep-1f);
+    lo[r] = (int)fl;
+    if (lo[r] < 0 || lo[r] > nd - 2) edge = true;
   }
-  int nb = 0, b0 = 0, pattern = 0;
-  if (first >= 0) {
-    for (int r = first - 1; r >= 0; --r) lo[r] = lo[r + 1];
-    for (int r = last + 1; r < ROW_P; ++r) lo[r] = lo[r - 1];
-    for (int r = first + 1; r <= last; ++r)
-      if (!in[r]) return -1;  // not expected: t is monotone along the row
-    bool up = true, down = true;
+  *pout = make_float4(p[0], p[1], p[2], p[3]);
+  if (in == 0) return TAP_NONE;
+  if (in < ROW_P) edge = true;
+  bool up = true, down = true;
+  unsigned pattern = 0;
 #pragma unroll
-    for (int r = 0; r + 1 < ROW_P; ++r) {
-      const int dlt = lo[r + 1] - lo[r];
-      up = up && (dlt == 0 || dlt == 1);
-      down = down && (dlt == 0 || dlt == -1);
-    }
-    if (!up && !down) return -1;
-    const int dir = up ? 0 : 1;
-#pragma unroll
-    for (int r = 0; r + 1 < ROW_P; ++r) pattern |= (lo[r + 1] != lo[r]) << r;
-    pattern |= dir << 3;
-    b0 = up ? lo[0] : lo[ROW_P - 1];
-    nb = (up ? lo[ROW_P - 1] : lo[0]) + 2 - b0;
+  for (int r = 0; r + 1 < ROW_P; ++r) {
+    const int dlt = lo[r + 1] - lo[r];
+    up = up && (dlt == 0 || dlt == 1);
+    down = down && (dlt == 0 || dlt == -1);
+    pattern |= (unsigned)(dlt != 0) << r;
   }
-  out[0] = make_int4(b0, nb, pattern, 0);
-  out[1] = make_int4(__float_as_int(wl[0]), __float_as_int(wl[1]), __float_as_int(wl[2]), __float_as_int(wl[3]));
-  out[2] = make_int4(__float_as_int(wh[0]), __float_as_int(wh[1]), __float_as_int(wh[2]), __float_as_int(wh[3]));
-  return nb;
+  if (edge || (!up && !down)) return TAP_EDGE;
+  if (!up) pattern |= 8u;
+  return (unsigned)(up ? lo[0] : lo[ROW_P - 1]) | (pattern << 26);
 }
 
-// one thread per (row tile, angle); *bad is set when an entry cannot be formed
-__global__ void k_row_fill(const float4 *__restrict__ ofs, int N, int nd, int nang, int4 *__restrict__ tab,
-                           int *__restrict__ bad) {
+// one thread per (row tile, angle)
+__global__ void k_tap_fill(const float4 *__restrict__ ofs, int N, int nd, int nang, unsigned *__restrict__ hdr,
+                           float4 *__restrict__ frac) {
   const int ntx = (N + ROW_P - 1) / ROW_P;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)ntx * N * nang) return;
   const long long tile = t / nang;
   const int j = (int)(t - tile * nang);
   const int y = (int)(tile / ntx), tx = (int)(tile - (long long)y * ntx);
-  if (row_entry(__ldg(ofs + j), tx * ROW_P, y, N, nd, tab + t * ROW_WORDS) < 0) atomicExch(bad, 1);
+  hdr[t] = tap_entry(__ldg(ofs + j), tx * ROW_P, y, N, nd, frac + t);
 }
 
-// ---------------------------------------------------------------------------
-// slice block of a lane: VW consecutive slices from s0 (VW = 4: one float4,
-// VW = 2: one float2)
-// ---------------------------------------------------------------------------
-template <int VW>
-__device__ __forceinline__ void st_slices(float *p, const float (&r)[VW]) {
-  if (VW == 4) *reinterpret_cast<float4 *>(p) = make_float4(r[0], r[1 % VW], r[2 % VW], r[3 % VW]);
-  else *reinterpret_cast<float2 *>(p) = make_float2(r[0], r[1 % VW]);
-}
-
-template <int VW>
-__device__ __forceinline__ void fma2(float (&acc)[VW], float w, const float (&v)[VW]) {
-#pragma unroll
-  for (int s = 0; s < VW; ++s) acc[s] = __fmaf_rn(w, v[s], acc[s]);
-}
-
-// unpredicated load of VW slices (the caller clamps the address into the field)
-template <int VW>
-__device__ __forceinline__ void ld_any(const float *p, float (&r)[VW]) {
-  if (VW == 4) {
-    const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
-    r[0] = a.x; r[1 % VW] = a.y; r[2 % VW] = a.z; r[3 % VW] = a.w;
-  } else {
-    const float2 a = __ldg(reinterpret_cast<const float2 *>(p));
-    r[0] = a.x; r[1 % VW] = a.y;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// k_bp_row: a block's 8 warps own 2 x 4 row tiles of one slice block (an 8 x 4
-// pixel region), so the taps they load for an angle overlap in L1.
-// ---------------------------------------------------------------------------
-// pixel r's lower tap for pattern PAT (see row_entry)
+// pixel r's lower tap for pattern PAT, as an index into the tile's bins
 template <int PAT, int R>
 struct RowTap {
   static constexpr int step(int r) { return (PAT >> r) & 1; }
@@ -161,67 +111,153 @@ struct RowTap {
 };
 
 template <int PAT, int VW>
-__device__ __forceinline__ void row_apply(float (&acc)[ROW_P][VW], const float (&T)[ROW_NB][VW],
-                                          const float (&wl)[ROW_P], const float (&wh)[ROW_P]) {
-  fma2<VW>(acc[0], wl[0], T[RowTap<PAT, 0>::k]);
-  fma2<VW>(acc[0], wh[0], T[RowTap<PAT, 0>::k + 1]);
-  fma2<VW>(acc[1], wl[1], T[RowTap<PAT, 1>::k]);
-  fma2<VW>(acc[1], wh[1], T[RowTap<PAT, 1>::k + 1]);
-  fma2<VW>(acc[2], wl[2], T[RowTap<PAT, 2>::k]);
-  fma2<VW>(acc[2], wh[2], T[RowTap<PAT, 2>::k + 1]);
-  fma2<VW>(acc[3], wl[3], T[RowTap<PAT, 3>::k]);
-  fma2<VW>(acc[3], wh[3], T[RowTap<PAT, 3>::k + 1]);
+__device__ __forceinline__ void tap_apply(VecAcc<VW> (&acc)[ROW_P], const float *__restrict__ lj, size_t S, int off2,
+                                          const float4 f) {
+  constexpr int NB = 2 + (PAT & 1) + ((PAT >> 1) & 1) + ((PAT >> 2) & 1);
+  Vec<VW> T[NB];
+#pragma unroll
+  for (int m = 0; m < NB; ++m) T[m].load(lj + (size_t)m * S, off2);
+  acc[0].fma(__fsub_rn(1.0f, f.x), T[RowTap<PAT, 0>::k]);
+  acc[0].fma(f.x, T[RowTap<PAT, 0>::k + 1]);
+  acc[1].fma(__fsub_rn(1.0f, f.y), T[RowTap<PAT, 1>::k]);
+  acc[1].fma(f.y, T[RowTap<PAT, 1>::k + 1]);
+  acc[2].fma(__fsub_rn(1.0f, f.z), T[RowTap<PAT, 2>::k]);
+  acc[2].fma(f.z, T[RowTap<PAT, 2>::k + 1]);
+  acc[3].fma(__fsub_rn(1.0f, f.w), T[RowTap<PAT, 3>::k]);
+  acc[3].fma(f.w, T[RowTap<PAT, 3>::k + 1]);
 }
 
+// one pixel of an edge tile: each tap only where it is on the detector
 template <int VW>
-__global__ void __launch_bounds__(256) k_bp_row(const IterParams P) {
-  static_assert(ROW_P == 4, "row_apply handles 4 pixels");
+__device__ __forceinline__ void tap_edge(VecAcc<VW> &acc, const float *__restrict__ lj, size_t S, int off2, int nd,
+                                         const float4 o, float xf, float yf) {
+  const float tt = __fadd_rn(__fadd_rn(__fmul_rn(xf, o.x), __fmul_rn(yf, o.y)), o.z);
+  if (!(tt > -1.f && tt < (float)nd)) return;
+  const float fl = floorf(tt);
+  const float p = fminf(__fsub_rn(tt, fl), 0x1.fffffep-1f);
+  const int il = (int)fl;
+  Vec<VW> v;
+  if (il >= 0) {
+    v.load(lj + (size_t)il * S, off2);
+    acc.fma(__fsub_rn(1.0f, p), v);
+  }
+  if (il <= nd - 2) {
+    v.load(lj + (size_t)(il + 1) * S, off2);
+    acc.fma(p, v);
+  }
+}
+
+// a block's 8 warps own 2 x 4 row tiles of one slice chunk (an 8 x 4 pixel region, whose taps
+// overlap in L1); MINB resident blocks cap the registers
+template <int VW, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_bp_tap(const IterParams P) {
   const Dims d = P.d;
   const int ntx = (d.N + ROW_P - 1) / ROW_P;
-  const int warp = threadIdx.x >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tx = blockIdx.x * 2 + (warp & 1), y = blockIdx.y * 4 + (warp >> 1);
   if (tx >= ntx || y >= d.N) return;
-  const int s0 = blockIdx.z * 32 * VW + (int)(threadIdx.x & 31) * VW;
-  const size_t S = d.S;
-  const size_t jstride = (size_t)d.nd * S;
-  const int4 *__restrict__ ent = P.row_ent + ((size_t)y * ntx + tx) * d.nang * ROW_WORDS;
+  constexpr int LW = VW == 8 ? 4 : VW;
+  const int s0 = blockIdx.z * 32 * VW + lane * LW;
+  const bool va = s0 < d.S, vb = VW == 8 && s0 + 128 < d.S;
+  const size_t S = d.S, jstride = (size_t)d.nd * S;
+  const size_t tile = ((size_t)y * ntx + tx) * d.nang;
+  const unsigned *__restrict__ hdr = P.tap_hdr + tile;
+  const float4 *__restrict__ frac = P.tap_frac + tile;
   // lanes past S read the last slices (their sums are not stored)
-  const float *__restrict__ lam = P.lam + min(s0, d.S - VW);
-
-  float acc[ROW_P][VW];
+  const float *__restrict__ lam = P.lam + min(s0, d.S - LW);
+  const int off2 = vb ? 128 : 0;
+  VecAcc<VW> acc[ROW_P];
 #pragma unroll
-  for (int r = 0; r < ROW_P; ++r)
+  for (int r = 0; r < ROW_P; ++r) acc[r].zero();
+  unsigned hn = __ldg(hdr);
+  for (int j = 0; j < d.nang; ++j, lam += jstride) {
+    const unsigned h = hn;
+    if (j + 1 < d.nang) hn = __ldg(hdr + j + 1);
+    if (h == TAP_NONE) continue;
+    const float4 f = __ldg(frac + j);
+    if (h & TAP_EDGE) {
+      const float4 o = __ldg(P.ofs + j);
 #pragma unroll
-    for (int s = 0; s < VW; ++s) acc[r][s] = 0.f;
-
-  for (int j = 0; j < d.nang; ++j, ent += ROW_WORDS) {
-    const int4 h = __ldg(ent);
-    const int nb = h.y;
-    if (nb == 0) continue;
-    const int4 la = __ldg(ent + 1), ha = __ldg(ent + 2);
-    const float wl[ROW_P] = {__int_as_float(la.x), __int_as_float(la.y), __int_as_float(la.z), __int_as_float(la.w)};
-    const float wh[ROW_P] = {__int_as_float(ha.x), __int_as_float(ha.y), __int_as_float(ha.z), __int_as_float(ha.w)};
-    const float *lj = lam + (size_t)j * jstride + (size_t)h.x * S;
-    // taps past the tile's last bin re-read that bin (never used by the pattern)
-    float T[ROW_NB][VW];
-#pragma unroll
-    for (int m = 0; m < ROW_NB; ++m) ld_any<VW>(lj + (size_t)min(m, nb - 1) * S, T[m]);
-    switch (h.z) {
-#define GT_ROW_CASE(c) \
-  case c: row_apply<c, VW>(acc, T, wl, wh); break;
-      GT_ROW_CASE(0) GT_ROW_CASE(1) GT_ROW_CASE(2) GT_ROW_CASE(3) GT_ROW_CASE(4) GT_ROW_CASE(5)
-      GT_ROW_CASE(6) GT_ROW_CASE(7) GT_ROW_CASE(8) GT_ROW_CASE(9) GT_ROW_CASE(10) GT_ROW_CASE(11)
-      GT_ROW_CASE(12) GT_ROW_CASE(13) GT_ROW_CASE(14) GT_ROW_CASE(15)
-#undef GT_ROW_CASE
+      for (int r = 0; r < ROW_P; ++r)
+        tap_edge<VW>(acc[r], lam, S, off2, d.nd, o, (float)min(tx * ROW_P + r, d.N - 1), (float)y);
+      continue;
+    }
+    const float *__restrict__ lj = lam + (size_t)(h & 0x3ffffffu) * S;
+    switch (h >> 26) {
+#define GT_TAP_CASE(c) \
+  case c: tap_apply<c, VW>(acc, lj, S, off2, f); break;
+      GT_TAP_CASE(0) GT_TAP_CASE(1) GT_TAP_CASE(2) GT_TAP_CASE(3) GT_TAP_CASE(4) GT_TAP_CASE(5)
+      GT_TAP_CASE(6) GT_TAP_CASE(7) GT_TAP_CASE(8) GT_TAP_CASE(9) GT_TAP_CASE(10) GT_TAP_CASE(11)
+      GT_TAP_CASE(12) GT_TAP_CASE(13) GT_TAP_CASE(14) GT_TAP_CASE(15)
+#undef GT_TAP_CASE
       default: break;
     }
   }
-  if (s0 >= d.S) return;
+  if (!va) return;
 #pragma unroll
   for (int r = 0; r < ROW_P; ++r) {
     const int x = tx * ROW_P + r;
-    if (x < d.N) st_slices<VW>(P.kstar + ((size_t)y * d.N + x) * S + s0, acc[r]);
+    float a[VW];
+    acc[r].get(a);
+    if (x < d.N) Vec<VW>::store(P.kstar + ((size_t)y * d.N + x) * S + s0, a, vb);
   }
+}
+
+template <int VW, int MINB>
+void bp_tap(const IterParams &P, cudaStream_t st) {
+  const int ntx = (P.d.N + ROW_P - 1) / ROW_P;
+  const dim3 grid((ntx + 1) / 2, (P.d.N + 3) / 4, (P.d.S + 32 * VW - 1) / (32 * VW));
+  k_bp_tap<VW, MINB><<<grid, 256, 0, st>>>(P);
+}
+
+// thread = (pixel, VW slices), UA angles at a time: their taps are loaded together, then
+// accumulated in angle order (taps off the detector read a bin inside it and are not added)
+template <int VW, int UA, int NT>
+__global__ void __launch_bounds__(NT) k_bp_flat(const IterParams P) {
+  const Dims d = P.d;
+  const int ng = d.S / VW;
+  const long long t = (long long)blockIdx.x * NT + threadIdx.x;
+  if (t >= (long long)ng * d.N * d.N) return;
+  const int pix = (int)(t / ng), s0 = (int)(t - (long long)pix * ng) * VW;
+  const int y = pix / d.N, x = pix - y * d.N;
+  const float xf = (float)x, yf = (float)y, fnd = (float)d.nd;
+  const size_t S = d.S, jstride = (size_t)d.nd * S;
+  const float *__restrict__ lam = P.lam + s0;
+  VecAcc<VW> acc;
+  acc.zero();
+  for (int j0 = 0; j0 < d.nang; j0 += UA) {
+    Vec<VW> a[UA], b[UA];
+    float p[UA];
+    bool ta[UA], tb[UA];
+#pragma unroll
+    for (int u = 0; u < UA; ++u) {
+      const int j = min(j0 + u, d.nang - 1);
+      const float4 o = __ldg(P.ofs + j);
+      const float tt = __fadd_rn(__fadd_rn(__fmul_rn(xf, o.x), __fmul_rn(yf, o.y)), o.z);
+      const bool in = tt > -1.f && tt < fnd && j0 + u < d.nang;
+      const float fl = floorf(tt);
+      p[u] = fminf(__fsub_rn(tt, fl), 0x1.fffffep-1f);
+      const int il = (int)fl;
+      ta[u] = in && il >= 0;
+      tb[u] = in && il <= d.nd - 2;
+      const float *__restrict__ lj = lam + (size_t)j * jstride;
+      a[u].load(lj + (size_t)(ta[u] ? il : 0) * S, 0);
+      b[u].load(lj + (size_t)(tb[u] ? il + 1 : 0) * S, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < UA; ++u) {
+      if (ta[u]) acc.fma(__fsub_rn(1.0f, p[u]), a[u]);
+      if (tb[u]) acc.fma(p[u], b[u]);
+    }
+  }
+  float r[VW];
+  acc.get(r);
+  Vec<VW>::store(P.kstar + (size_t)pix * S + s0, r, false);
+}
+
+template <int VW, int UA, int NT>
+void bp_flat(const IterParams &P, cudaStream_t st) {
+  k_bp_flat<VW, UA, NT><<<blocks((long long)(P.d.S / VW) * P.d.N * P.d.N, NT), NT, 0, st>>>(P);
 }
 
 }  // namespace
@@ -229,23 +265,30 @@ __global__ void __launch_bounds__(256) k_bp_row(const IterParams P) {
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-size_t row_table_bytes(int N, int nang) {
-  return sizeof(int4) * ROW_WORDS * (size_t)((N + ROW_P - 1) / ROW_P) * N * nang;
+// (row tile, angle) pairs of the table; 0 where it does not apply (bins beyond the header's bits)
+long long tap_entries(int N, int nd, int nang) {
+  return nd < (1 << 26) ? (long long)((N + ROW_P - 1) / ROW_P) * N * nang : 0;
 }
 
-cudaError_t launch_row_fill(const float4 *ofs, int N, int nd, int nang, int4 *tab, int *bad, cudaStream_t st) {
-  const long long n = (long long)((N + ROW_P - 1) / ROW_P) * N * nang;
-  k_row_fill<<<blocks(n, 128), 128, 0, st>>>(ofs, N, nd, nang, tab, bad);
+cudaError_t launch_tap_fill(const float4 *ofs, int N, int nd, int nang, unsigned *hdr, float4 *frac, cudaStream_t st) {
+  const long long n = tap_entries(N, nd, nang);
+  k_tap_fill<<<blocks(n, 128), 128, 0, st>>>(ofs, N, nd, nang, hdr, frac);
   return cudaGetLastError();
 }
 
-// shape 0: 4 slices per lane; 1: 2 slices per lane
-cudaError_t launch_bp_row(const IterParams &P, int shape, cudaStream_t st) {
-  const int ntx = (P.d.N + ROW_P - 1) / ROW_P;
-  const int vw = shape == 1 ? 2 : 4;
-  const dim3 grid((ntx + 1) / 2, (P.d.N + 3) / 4, (P.d.S + 32 * vw - 1) / (32 * vw));
-  if (vw == 4) k_bp_row<4><<<grid, 256, 0, st>>>(P);
-  else k_bp_row<2><<<grid, 256, 0, st>>>(P);
+// k_bp_tap with vw slices per lane (8, 4: S a multiple of 4; 2: even S)
+cudaError_t launch_bp_tap(const IterParams &P, int vw, cudaStream_t st) {
+  if (vw == 8) bp_tap<8, 3>(P, st);
+  else if (vw == 4) bp_tap<4, 4>(P, st);
+  else bp_tap<2, 5>(P, st);
+  return cudaGetLastError();
+}
+
+// k_bp_flat with vw slices per thread (4, 2 or 1, a divisor of S)
+cudaError_t launch_bp_flat(const IterParams &P, int vw, cudaStream_t st) {
+  if (vw == 4) bp_flat<4, 8, 64>(P, st);
+  else if (vw == 2) bp_flat<2, 8, 128>(P, st);
+  else bp_flat<1, 8, 128>(P, st);
   return cudaGetLastError();
 }
 
