@@ -62,12 +62,13 @@ cudaError_t fill_f32(float *x, size_t n, float v, cudaStream_t st);
 cudaError_t launch_ray_count(const float4 *ofs, int N, int nd, int nang, int *count, cudaStream_t st);
 cudaError_t launch_ray_fill(const float4 *ofs, int N, int nd, int nang, const long long *start, int2 *ent,
                             cudaStream_t st);
-cudaError_t launch_run_count(const float4 *ofs, int N, int nd, int nang, int *count, cudaStream_t st);
+cudaError_t launch_pair_count(const float4 *ofs, int N, int nd, int nang, int *count, cudaStream_t st);
+cudaError_t launch_pair_fill(const float4 *ofs, int N, int nd, int nang, const long long *start, int2 *ent,
+                             cudaStream_t st);
+int default_fwd_shape(int S);
 long long tap_entries(int N, int nd, int nang);
 cudaError_t launch_tap_fill(const float4 *ofs, int N, int nd, int nang, unsigned *hdr, float4 *frac, cudaStream_t st);
 int default_bp_shape(int S);
-cudaError_t launch_run_fill(const float4 *ofs, int N, int nd, int nang, const long long *start, int4 *ent,
-                            cudaStream_t st);
 int num_proj_configs(int S, int which);
 bool dual_z2_ok(const IterParams &P, int tgv, int cpl);
 int num_dual_configs(const IterParams &P);
@@ -128,6 +129,8 @@ void angle_table(const double *angles, int N, int nd, int nang, std::vector<doub
 }
 
 constexpr int kMuPad = 4;  // channel weights of the padding slices (channel index s / Nz >= C): 1
+
+constexpr int kPairSlices = 80;  // slices from which the pair table is built for the tuning (default_fwd_shape)
 
 // Slices per pixel in memory.  The vector kernels (projectors, primal update) move four
 // slices per load, so a count that is not a multiple of 4 is padded with zero slices,
@@ -193,7 +196,7 @@ struct gt_problem {
   float *u = nullptr, *ubar = nullptr, *p = nullptr, *pbar = nullptr, *v = nullptr, *w = nullptr;
   float *lam = nullptr, *f = nullptr, *ku = nullptr, *stage = nullptr, *kstar = nullptr;
   void *rays = nullptr;        // ray table (offsets + entries), built at creation
-  void *runs = nullptr;        // 3-bin run table (offsets + entries), built at creation
+  void *pairs = nullptr;       // pair table of k_fwd_pair (offsets + entries), built when a shape needs it
   void *tiles = nullptr;       // row-tile table of k_bp_tap, built at creation
   size_t ray_bytes = 0;
   void *gap_ws = nullptr;      // gap workspace (v~ planes + FP64 block partials), allocated on first gt_gap
@@ -327,6 +330,35 @@ int capture(gt_problem *p, int n, cudaGraphExec_t *out) {
   return GT_OK;
 }
 
+// The pair table of k_fwd_pair (forward shapes 10, 11); optional: without it (no memory) those
+// shapes fall back to the ray table.  Uses stage as scratch, on the problem's stream.
+int ensure_pairs(gt_problem *p) {
+  if (p->pairs || !p->P.ray_start) return GT_OK;
+  const gt::Dims &d = p->d;
+  const int np = (d.nd + 1) / 2 * d.nang;
+  std::vector<int> cnt(np);
+  std::vector<long long> start(np + 1, 0);
+  int *d_cnt = (int *)p->stage;
+  CK(gt::launch_pair_count(p->ofs, d.N, d.nd, d.nang, d_cnt, p->stream));
+  CK(cudaMemcpyAsync(cnt.data(), d_cnt, sizeof(int) * np, cudaMemcpyDeviceToHost, p->stream));
+  CK(cudaStreamSynchronize(p->stream));
+  for (int r = 0; r < np; ++r) start[r + 1] = start[r] + cnt[r];
+  const size_t off_e = align256(sizeof(long long) * (np + 1));
+  if (cudaMalloc(&p->pairs, off_e + sizeof(int2) * std::max<size_t>(start[np], 1)) != cudaSuccess) {
+    cudaGetLastError();
+    p->pairs = nullptr;
+    return GT_OK;
+  }
+  long long *d_start = (long long *)p->pairs;
+  int2 *d_ent = (int2 *)((char *)p->pairs + off_e);
+  CK(cudaMemcpyAsync(d_start, start.data(), sizeof(long long) * (np + 1), cudaMemcpyHostToDevice, p->stream));
+  CK(gt::launch_pair_fill(p->ofs, d.N, d.nd, d.nang, d_start, d_ent, p->stream));
+  CK(cudaStreamSynchronize(p->stream));
+  p->P.pair_start = d_start;
+  p->P.pair_ent = d_ent;
+  return GT_OK;
+}
+
 // device field -> (pointer, components, per-component X extent)
 int field_info(gt_problem *p, int field, float **ptr, int *comps, size_t *X) {
   const size_t img = (size_t)p->d.N * p->d.N, sino = (size_t)p->d.nd * p->d.nang;
@@ -396,22 +428,19 @@ int autotune(gt_problem *p) {
   // its time on batches of many distinct problems: of the back projection all but the
   // row-tile shapes (18, 19, 9) and the flat ones (10, 11), each in the range of slice
   // counts where it can win (times at default_bp_shape; the one-pixel and TMA shapes
-  // never do); the multi-bin run shapes (forward 5-8) once S >= 32, 2-4x slower than
-  // the best shape on every measured workload there; the chunk-outermost shape
-  // (forward 9), which only pays when the image exceeds L2, below 64 MB of image; one
-  // slice per thread (forward 4) once S >= 128.
+  // never do); of the forward projection all but the pair shapes (10, 11), the flat ones
+  // (9, 5) and the staged one (7), likewise (times at default_fwd_shape).
   const int S = p->d.S;
-  const long long img_bytes = (long long)p->d.N * p->d.N * S * 4;
   auto skipped = [&](int which, int c) {
+    if (which == 0)
+      return !((c == 10 && S > 128) || (c == 11 && S >= kPairSlices) || (c == 9 && S <= 128) || (c == 5 && S <= 32) ||
+               (c == 7 && S == 4));
     if (which == 1)
       return !((c == 18 && S >= 96) || (c == 19 && S >= 36) || (c == 9 && S >= 16 && S <= 128) ||
                (c == 10 && S <= 128) || (c == 11 && S <= 16));
-    if (S >= 32 && which == 0 && c >= 5 && c <= 8) return true;
-    if (img_bytes < (64ll << 20) && which == 0 && c == 9) return true;
-    if (S >= 128 && which == 0 && c == 4) return true;
     return false;
   };
-  p->P.fwd_cfg = 0;
+  p->P.fwd_cfg = gt::default_fwd_shape(S);
   p->P.bp_cfg = gt::default_bp_shape(S);
   p->P.dual_cfg = 0;
   if ((nc[0] <= 1 && nc[1] <= 1 && nc[2] <= 1) || !p->autotune) return GT_OK;
@@ -714,36 +743,6 @@ static int create_problem(const gt_desc *desc, bool pad, gt_problem **out) {
     p->P.ray_ent = d_ent;
   }
 
-  // 3-bin run table of the forward projector (k_fwd_rt); optional: without it
-  // (no memory) the run shapes fall back to the ray table
-  {
-    const int nr = ((D.nd + 2) / 3) * D.nang;
-    std::vector<int> cnt(nr);
-    std::vector<long long> start(nr + 1, 0);
-    int *d_cnt = (int *)p->stage;
-    if ((e = gt::launch_run_count(p->ofs, D.N, D.nd, D.nang, d_cnt, p->stream)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(cnt.data(), d_cnt, sizeof(int) * nr, cudaMemcpyDeviceToHost, p->stream)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(p->stream)) != cudaSuccess)
-      return fail(cuda_err(e, "run table count", __LINE__));
-    for (int r = 0; r < nr; ++r) start[r + 1] = start[r] + cnt[r];
-    const size_t off_e = align256(sizeof(long long) * (nr + 1));
-    const size_t bytes = off_e + sizeof(int4) * (size_t)start[nr];
-    if (cudaMalloc(&p->runs, bytes) != cudaSuccess) {
-      cudaGetLastError();
-      p->runs = nullptr;
-    } else {
-      long long *d_start = (long long *)p->runs;
-      int4 *d_ent = (int4 *)((char *)p->runs + off_e);
-      if ((e = cudaMemcpyAsync(d_start, start.data(), sizeof(long long) * (nr + 1), cudaMemcpyHostToDevice,
-                               p->stream)) != cudaSuccess ||
-          (e = gt::launch_run_fill(p->ofs, D.N, D.nd, D.nang, d_start, d_ent, p->stream)) != cudaSuccess ||
-          (e = cudaStreamSynchronize(p->stream)) != cudaSuccess)
-        return fail(cuda_err(e, "run table fill", __LINE__));
-      p->P.run_start = d_start;
-      p->P.run_ent = d_ent;
-    }
-  }
-
   // row-tile table of the register-blocked back projector (k_bp_tap); optional: without
   // it (no memory, a detector beyond its bins) those launch shapes fall back to others
   if (const long long nt = gt::tap_entries(D.N, D.nd, D.nang)) {
@@ -793,7 +792,7 @@ void gt_problem_destroy(gt_problem *p) {
   if (p->g_chunk) cudaGraphExecDestroy(p->g_chunk);
   if (p->block) cudaFree(p->block);
   if (p->rays) cudaFree(p->rays);
-  if (p->runs) cudaFree(p->runs);
+  if (p->pairs) cudaFree(p->pairs);
   if (p->tiles) cudaFree(p->tiles);
   if (p->gap_ws) cudaFree(p->gap_ws);
   if (p->snap) cudaFree(p->snap);
@@ -851,7 +850,8 @@ int gt_set_data(gt_problem *p, const float *f_host, int make_feasible) {
   p->P.ne64 = p->ne;
   // pick the projector launch shapes (uses lambda / ku / kstar as scratch: they are reset below)
   {
-    const int rc = autotune(p);
+    int rc = d.S >= kPairSlices ? ensure_pairs(p) : GT_OK;
+    if (rc == GT_OK) rc = autotune(p);
     if (rc) return rc;
   }
   // zero iterates (tgv_radon :1160-1176)
@@ -1026,6 +1026,10 @@ int gt_set_tuning(gt_problem *p, int fwd_cfg, int bp_cfg) {
                    gt::num_proj_configs(p->Sr, 0), gt::num_proj_configs(p->Sr, 1));
   CK(cudaSetDevice(p->device));
   CK(cudaStreamSynchronize(p->stream));
+  if (fwd_cfg == 10 || fwd_cfg == 11) {
+    const int rc = ensure_pairs(p);
+    if (rc) return rc;
+  }
   p->P.fwd_cfg = fwd_cfg;
   p->P.bp_cfg = bp_cfg;
   // the captured graphs hold the old launch shapes

@@ -47,8 +47,8 @@ struct IterParams {
   const float4 *ofs;     // [nang] (X, Y, offset, Xinv)
   const long long *ray_start;  // [nd*nang + 1] ray table offsets (null: walk rays on the fly)
   const int2 *ray_ent;         // (pixel, weight bits) entries of all rays
-  const long long *run_start;  // [nang*ceil(nd/3) + 1] offsets of the 3-bin run table (null: none)
-  const int4 *run_ent;         // (pixel, weight bits of bins i0, i0+1, i0+2) entries of all runs
+  const long long *pair_start; // [nang*ceil(nd/2) + 1] offsets of the pair table of k_fwd_pair (null: none)
+  const int2 *pair_ent;        // (pixel, bits of the detector coordinate) entries of all pairs of bins
   const unsigned *tap_hdr;     // [N][ceil(N/4)][nang] row tiles of the back projection: first bin and step pattern (or null)
   const float4 *tap_frac;      // [N][ceil(N/4)][nang] interpolation fractions of their 4 pixels
   const float *mu;       // [C] mu (KL) or mu/(sigma+mu) (L2)

@@ -1353,34 +1353,6 @@ static inline long long threads_for(long long units, int S) {
   return (VW == 8 || VW == 4) ? units * ((S + VW * 32 - 1) / (VW * 32)) * 32 : units * (S / VW);
 }
 
-// One slice per lane, a warp over 32 consecutive slices, the slice chunk outermost:
-// the warps running at a time all work on the same 32 slices of every pixel or
-// bin, so a projector's working set is one 32-slice chunk of the image or
-// sinogram (e.g. 768^2 x 32 x 4 B = 75 MB, inside L2) instead of all S slices.
-struct SlicesWL {
-  int s0;
-  bool va;
-  __device__ __forceinline__ void load(const float *base, float (&r)[1]) const { r[0] = va ? __ldg(base + s0) : 0.f; }
-  __device__ __forceinline__ void loadw(const float *base, float (&r)[1]) const { r[0] = va ? base[s0] : 0.f; }
-  __device__ __forceinline__ void store(float *base, const float (&r)[1]) const { if (va) base[s0] = r[0]; }
-  __device__ __forceinline__ int slice(int) const { return s0; }
-  __device__ __forceinline__ bool valid(int) const { return va; }
-};
-
-__device__ __forceinline__ bool map_thread_wl(long long units, int S, long long &unit, SlicesWL &sl) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long w = t >> 5;
-  const int nblk = (S + 31) / 32;
-  if (w >= units * nblk) return false;
-  const int blk = (int)(w / units);
-  unit = w - (long long)blk * units;
-  sl.s0 = blk * 32 + (int)(threadIdx.x & 31);
-  sl.va = sl.s0 < S;
-  return true;
-}
-
-static inline long long threads_for_wl(long long units, int S) { return units * ((S + 31) / 32) * 32; }
-
 // ===========================================================================
 // forward projection: kernel `radon` (3-D :773-816).  Ray (i, j) of slice s:
 // acc = sum over rows y and x in [x_low, x_high] of (1 - |x X + y Y + off - i|)+ img.
@@ -1474,81 +1446,6 @@ __global__ void k_ray_fill(const float4 *__restrict__ ofs, int N, int nd, int na
   ray_walk<true>(__ldg(ofs + j), i, N, ent + start[t]);
 }
 
-// Run table: the rays of three adjacent bins i0, i0+1, i0+2 of one angle walked
-// together.  Per row the union of their x ranges is listed once, each pixel with
-// its three weights (zero where the bin's hat does not cover it), in the rows-
-// then-x order of the reference; a pixel is loaded once for the three bins.
-// Every weight is the one ray_walk computes for that bin, and a zero weight adds
-// an exact zero, so each bin's sum is the ray table's, term for term.
-template <bool FILL>
-__device__ __forceinline__ int run_walk(const float4 o, int i0, int N, int nd, int4 *out) {
-  int ylo, yhi, ylo2, yhi2;
-  ray_rows(o, i0, N, ylo, yhi);
-  ray_rows(o, min(i0 + 2, nd - 1), N, ylo2, yhi2);
-  ylo = min(ylo, ylo2);
-  yhi = max(yhi, yhi2);
-  int n = 0;
-  for (int y = ylo; y <= yhi; ++y) {
-    const float d = __fadd_rn(__fmul_rn((float)y, o.y), o.z);
-    int xl[3], xh[3];
-    int xmin = N, xmax = -1;
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      const int i = i0 + r;
-      const float fim = (float)(i - 1), fip = (float)(i + 1);
-      int a, b;
-      if (o.x == 0.f) {
-        if (d > fim && d < fip) { a = 0; b = N - 1; } else { a = N; b = -1; }
-      } else if (o.x > 0.f) {
-        a = __float2int_rz(__fmul_rn(__fsub_rn(fim, d), o.w));
-        b = __float2int_rz(__fmul_rn(__fsub_rn(fip, d), o.w));
-      } else {
-        a = __float2int_rz(__fmul_rn(__fsub_rn(fip, d), o.w));
-        b = __float2int_rz(__fmul_rn(__fsub_rn(fim, d), o.w));
-      }
-      a = max(a, 0);
-      b = min(b, N - 1);
-      if (i >= nd) { a = N; b = -1; }
-      xl[r] = a;
-      xh[r] = b;
-      if (a <= b) { xmin = min(xmin, a); xmax = max(xmax, b); }
-    }
-    for (int x = xmin; x <= xmax; ++x) {
-      const float tx = __fadd_rn(__fmul_rn((float)x, o.x), d);
-      float w[3];
-      bool any = false;
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        const float wr = 1.0f - fabsf(__fsub_rn(tx, (float)(i0 + r)));
-        w[r] = (x >= xl[r] && x <= xh[r] && wr > 0.f) ? wr : 0.f;
-        any = any || w[r] > 0.f;
-      }
-      if (any) {
-        if (FILL) out[n] = make_int4(y * N + x, __float_as_int(w[0]), __float_as_int(w[1]), __float_as_int(w[2]));
-        ++n;
-      }
-    }
-  }
-  return n;
-}
-
-__global__ void k_run_count(const float4 *__restrict__ ofs, int N, int nd, int nang, int *__restrict__ count) {
-  const int nq = (nd + 2) / 3;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nq * nang) return;
-  const int j = t / nq, q = t - j * nq;
-  count[t] = run_walk<false>(__ldg(ofs + j), 3 * q, N, nd, nullptr);
-}
-
-__global__ void k_run_fill(const float4 *__restrict__ ofs, int N, int nd, int nang, const long long *__restrict__ start,
-                           int4 *__restrict__ ent) {
-  const int nq = (nd + 2) / 3;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nq * nang) return;
-  const int j = t / nq, q = t - j * nq;
-  run_walk<true>(__ldg(ofs + j), 3 * q, N, nd, ent + start[t]);
-}
-
 // acc += w * v per slice: the reference's separately rounded product and sum
 // (EXACT), or one fused multiply-add (the solver's hot loops)
 template <bool EXACT>
@@ -1597,27 +1494,20 @@ __device__ __forceinline__ void radon_table(const float *__restrict__ img, size_
 }
 
 // k_fwd: radon of ubar fused with update_lambda_KL (3-D :690-704) or _L2 (:677-688).
-template <int DISC, int VW, int UNR, bool WL = false>
+template <int DISC, int VW, int UNR>
 __device__ __forceinline__ void fwd_body(const IterParams &P, long long bid) {
   const Dims d = P.d;
   long long unit;
-  typename std::conditional<WL, SlicesWL, Slices<VW>>::type sl;
-  if constexpr (WL) {
-    static_assert(VW == 1, "one slice per lane");
-    if (!map_thread_wl((long long)d.nd * d.nang, d.S, unit, sl)) return;
-  } else {
-    if (!map_thread<VW>(bid, (long long)d.nd * d.nang, d.S, unit, sl)) return;
-  }
+  Slices<VW> sl;
+  if (!map_thread<VW>(bid, (long long)d.nd * d.nang, d.S, unit, sl)) return;
   const int b = (int)unit;
   const int j = b / d.nd, i = b - j * d.nd;
   float acc[VW];
   if (P.ray_start) {
     const long long r0 = __ldg(P.ray_start + b), r1 = __ldg(P.ray_start + b + 1);
     radon_table<VW, false, UNR>(P.ubar, d.S, P.ray_ent + r0, (int)(r1 - r0), sl, acc);
-  } else if constexpr (!WL) {
-    radon_ray<VW>(P.ubar, d.S, d.N, __ldg(P.ofs + j), i, sl, acc);
   } else {
-    acc[0] = 0.f;  // not reached: the launcher offers the WL shape only with the ray table
+    radon_ray<VW>(P.ubar, d.S, d.N, __ldg(P.ofs + j), i, sl, acc);
   }
   const size_t q = (size_t)b * d.S;
   sl.store(P.ku + q, acc);
@@ -1640,9 +1530,9 @@ __device__ __forceinline__ void fwd_body(const IterParams &P, long long bid) {
   sl.store(P.lam + q, lam);
 }
 
-template <int DISC, int VW, int UNR, bool WL = false, int MINB = 1>
+template <int DISC, int VW, int UNR, int MINB = 1>
 __global__ void __launch_bounds__(256, MINB) k_fwd(const IterParams P) {
-  fwd_body<DISC, VW, UNR, WL>(P, blockIdx.x);
+  fwd_body<DISC, VW, UNR>(P, blockIdx.x);
 }
 
 // ===========================================================================
@@ -2806,289 +2696,71 @@ cudaError_t launch_dual_fused(const IterParams &P, int tgv, int cpl, cudaStream_
   return cudaGetLastError();
 }
 
-// Forward projection of R adjacent bins of one angle at once.  For every row the
-// union of the R bins' x ranges is read once and each pixel feeds every bin whose
-// hat covers it, so a pixel loaded for bin i also serves bin i+1 (about (R+1)/2R
-// of the loads of one bin at a time).  Each bin still sums its terms in the
-// reference's order (rows ascending, x ascending) with the reference's bounds and
-// weights.
-template <int VW, int R, bool EXACT>
-__device__ __forceinline__ void radon_run(const float *__restrict__ img, size_t S, int N, int nd, const float4 o,
-                                          int i0, const Slices<VW> &sl, float (&acc)[R][VW]) {
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int k = 0; k < VW; ++k) acc[r][k] = 0.f;
-  int ylo, yhi, ylo2, yhi2;
-  ray_rows(o, i0, N, ylo, yhi);
-  ray_rows(o, min(i0 + R - 1, nd - 1), N, ylo2, yhi2);
-  ylo = min(ylo, ylo2);
-  yhi = max(yhi, yhi2);
-  for (int y = ylo; y <= yhi; ++y) {
-    const float d = __fadd_rn(__fmul_rn((float)y, o.y), o.z);
-    int xl[R], xh[R];
-    int xmin = N, xmax = -1;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int i = i0 + r;
-      const float fim = (float)(i - 1), fip = (float)(i + 1);
-      int a, b;
-      if (o.x == 0.f) {
-        if (d > fim && d < fip) { a = 0; b = N - 1; } else { a = N; b = -1; }
-      } else if (o.x > 0.f) {
-        a = __float2int_rz(__fmul_rn(__fsub_rn(fim, d), o.w));
-        b = __float2int_rz(__fmul_rn(__fsub_rn(fip, d), o.w));
-      } else {
-        a = __float2int_rz(__fmul_rn(__fsub_rn(fip, d), o.w));
-        b = __float2int_rz(__fmul_rn(__fsub_rn(fim, d), o.w));
-      }
-      a = max(a, 0);
-      b = min(b, N - 1);
-      if (i >= nd) { a = N; b = -1; }
-      xl[r] = a;
-      xh[r] = b;
-      if (a <= b) { xmin = min(xmin, a); xmax = max(xmax, b); }
-    }
-    const float *row = img + (size_t)y * N * S;
-    // groups of G pixels: their loads are issued together, then consumed in x order
-    constexpr int G = 4;
-    for (int xg = xmin; xg <= xmax; xg += G) {
-      float val[G][VW];
-#pragma unroll
-      for (int g = 0; g < G; ++g)
-        if (xg + g <= xmax) sl.load(row + (size_t)(xg + g) * S, val[g]);
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        const int x = xg + g;
-        if (x > xmax) break;
-        const float tx = __fadd_rn(__fmul_rn((float)x, o.x), d);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const float wgt = 1.0f - fabsf(__fsub_rn(tx, (float)(i0 + r)));
-          if (x >= xl[r] && x <= xh[r] && wgt > 0.f) {
-#pragma unroll
-            for (int k = 0; k < VW; ++k) acc[r][k] = mac<EXACT>(acc[r][k], wgt, val[g][k]);
-          }
-        }
-      }
-    }
-  }
-}
-
-// k_fwd_run: k_fwd for runs of R bins (radon_run), same fused data-term prox.
-template <int DISC, int VW, int R>
-__global__ void __launch_bounds__(256) k_fwd_run(const IterParams P) {
-  const Dims d = P.d;
-  const int nrun = (d.nd + R - 1) / R;
-  long long unit;
-  Slices<VW> sl;
-  if (!map_thread<VW>((long long)nrun * d.nang, d.S, unit, sl)) return;
-  const int j = (int)(unit / nrun), i0 = (int)(unit - (long long)j * nrun) * R;
-  float acc[R][VW];
-  radon_run<VW, R, false>(P.ubar, d.S, d.N, d.nd, __ldg(P.ofs + j), i0, sl, acc);
-  const float sd = P.sigma_data;
-  float m[VW];
-#pragma unroll
-  for (int k = 0; k < VW; ++k) m[k] = sl.valid(k) ? __ldg(P.mu + sl.slice(k) / d.Nz) : 0.f;
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    if (i0 + r >= d.nd) break;
-    const size_t q = ((size_t)j * d.nd + i0 + r) * d.S;
-    sl.store(P.ku + q, acc[r]);
-    float lam[VW], f[VW];
-    sl.loadw(P.lam + q, lam);
-    sl.load(P.f + q, f);
-#pragma unroll
-    for (int k = 0; k < VW; ++k) {
-      if (DISC == KL) {
-        const float sv = lam[k] + sd * acc[r][k];
-        const float wv = sv - m[k];
-        const float dv = wv * wv + 4.f * sd * f[k] * m[k];
-        lam[k] = sv - 0.5f * (wv + sqrtf(dv));
-      } else {
-        lam[k] = (lam[k] + sd * (acc[r][k] - f[k])) * m[k];
-      }
-    }
-    sl.store(P.lam + q, lam);
-  }
-}
-
-// k_fwd_rt: k_fwd over 3-bin runs from the run table (each pixel loaded once for
-// three bins), same fused data-term prox per bin.
-template <int DISC, int VW, int UNR>
-__global__ void __launch_bounds__(256) k_fwd_rt(const IterParams P) {
-  const Dims d = P.d;
-  const int nq = (d.nd + 2) / 3;
-  long long unit;
-  Slices<VW> sl;
-  if (!map_thread<VW>((long long)nq * d.nang, d.S, unit, sl)) return;
-  const int j = (int)(unit / nq), i0 = 3 * (int)(unit - (long long)j * nq);
-  float acc[3][VW];
-#pragma unroll
-  for (int r = 0; r < 3; ++r)
-#pragma unroll
-    for (int k = 0; k < VW; ++k) acc[r][k] = 0.f;
-  const long long e0 = __ldg(P.run_start + unit), e1 = __ldg(P.run_start + unit + 1);
-  const int4 *ent = P.run_ent + e0;
-  const int n = (int)(e1 - e0);
-  int e = 0;
-  for (; e + UNR <= n; e += UNR) {
-    int4 en[UNR];
-    float v[UNR][VW];
-#pragma unroll
-    for (int u = 0; u < UNR; ++u) en[u] = __ldg(ent + e + u);
-#pragma unroll
-    for (int u = 0; u < UNR; ++u) sl.load(P.ubar + (size_t)en[u].x * d.S, v[u]);
-#pragma unroll
-    for (int u = 0; u < UNR; ++u) {
-      const float w0 = __int_as_float(en[u].y), w1 = __int_as_float(en[u].z), w2 = __int_as_float(en[u].w);
-#pragma unroll
-      for (int k = 0; k < VW; ++k) {
-        acc[0][k] = __fmaf_rn(w0, v[u][k], acc[0][k]);
-        acc[1][k] = __fmaf_rn(w1, v[u][k], acc[1][k]);
-        acc[2][k] = __fmaf_rn(w2, v[u][k], acc[2][k]);
-      }
-    }
-  }
-  for (; e < n; ++e) {
-    const int4 en = __ldg(ent + e);
-    float v[VW];
-    sl.load(P.ubar + (size_t)en.x * d.S, v);
-    const float w0 = __int_as_float(en.y), w1 = __int_as_float(en.z), w2 = __int_as_float(en.w);
-#pragma unroll
-    for (int k = 0; k < VW; ++k) {
-      acc[0][k] = __fmaf_rn(w0, v[k], acc[0][k]);
-      acc[1][k] = __fmaf_rn(w1, v[k], acc[1][k]);
-      acc[2][k] = __fmaf_rn(w2, v[k], acc[2][k]);
-    }
-  }
-  const float sd = P.sigma_data;
-  float m[VW];
-#pragma unroll
-  for (int k = 0; k < VW; ++k) m[k] = sl.valid(k) ? __ldg(P.mu + sl.slice(k) / d.Nz) : 0.f;
-#pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    if (i0 + r >= d.nd) break;
-    const size_t q = ((size_t)j * d.nd + i0 + r) * d.S;
-    sl.store(P.ku + q, acc[r]);
-    float lam[VW], f[VW];
-    sl.loadw(P.lam + q, lam);
-    sl.load(P.f + q, f);
-#pragma unroll
-    for (int k = 0; k < VW; ++k) {
-      if (DISC == KL) {
-        const float sv = lam[k] + sd * acc[r][k];
-        const float wv = sv - m[k];
-        const float dv = wv * wv + 4.f * sd * f[k] * m[k];
-        lam[k] = sv - 0.5f * (wv + sqrtf(dv));
-      } else {
-        lam[k] = (lam[k] + sd * (acc[r][k] - f[k])) * m[k];
-      }
-    }
-    sl.store(P.lam + q, lam);
-  }
-}
-
-// slices per lane: 8 (two float4 chunks) when S is a multiple of 4, else 2, else 1
-static inline int vec_width(int S) { return (S % 4 == 0) ? 8 : (S % 2 == 0 ? 2 : 1); }
-
-// Tunable launch shapes of the projector kernels (chosen per problem shape by
-// the autotuner in gt_api.cu).  S a multiple of 4: k_fwd configs 0..3 =
-// (slices per lane, ray-table entries in flight) = (8, 4), (8, 8), (4, 4), (4, 8),
-// configs 5..8 = (slices per lane, bins per run) of k_fwd_run = (8, 2), (8, 4),
-// (4, 4), (4, 8);
+// Tunable launch shapes of the projector kernels (chosen per problem shape by the
+// autotuner in gt_api.cu), for S a multiple of 4.
+// k_fwd configs: 0..4 = (slices per lane, ray-table entries in flight) = (8, 4), (8, 8),
+// (4, 4), (4, 8), (1, 4); 12..19 = (8, 4) with registers capped for 4 resident blocks;
+// 10, 11 the pair kernel k_fwd_pair with 8 and 4 slices per lane; 9 (and 8), 5, 6 the
+// flat kernel k_fwd_flat with 4, 2 and 1 slices per thread; 7 the staged kernel (S = 4,
+// else 9) (gt_fwd.cu).
 // k_bp configs 0..8 = (slices per lane, angles per step) of the one-pixel kernel = (8, 2),
 // (8, 4), (4, 2), (4, 4), (8, 1), (4, 1), (8, 2), (4, 2), (1, 1); 16 and 17 are 4 with its
 // angle loop unrolled 4x or not at all; 14 and 15 the TMA-staged kernel; 18, 19 and 9
 // the row-tile kernel k_bp_tap with 8, 4 and 2 slices per lane, 10 (and 13), 11, 12 the
-// flat kernel k_bp_flat with 4, 2 and 1 slices per thread (gt_proj.cu).  k_fwd config 9:
-// one slice per lane with the 32-slice chunk outermost (SlicesWL), for images larger
-// than L2.  k_fwd configs 10, 11: the 3-bin run
-// table (k_fwd_rt) with (slices per lane, entries in flight) = (8, 4), (4, 8);
-// configs 12, 13: (8, 8) and (8, 4) with registers capped for 5 / 6 resident blocks.
-// Otherwise one fixed shape with 2 or 1 slices per thread.
-// One more candidate of k_fwd: one slice per thread (config 4), which keeps all lanes
-// busy when S is small.
+// flat kernel k_bp_flat with 4, 2 and 1 slices per thread (gt_proj.cu).
+// Otherwise one fixed shape.
 int num_proj_configs(int S, int which) {
   if (S % 4 != 0) return 1;
-  return which == 0 ? 20 : 20;  // configs 4 / 8 (one slice per thread) stay candidates for every S
+  return which == 0 ? 20 : 20;
 }
 
-template <int VW, int UNR>
+template <int VW, int UNR, int MINB = 1>
 static void fwd_vw(const IterParams &P, int disc, cudaStream_t st) {
   const unsigned g = blocks_for(threads_for<VW>((long long)P.d.nd * P.d.nang, P.d.S), 256);
-  if (disc == KL) k_fwd<KL, VW, UNR><<<g, 256, 0, st>>>(P);
-  else k_fwd<L2, VW, UNR><<<g, 256, 0, st>>>(P);
+  if (disc == KL) k_fwd<KL, VW, UNR, MINB><<<g, 256, 0, st>>>(P);
+  else k_fwd<L2, VW, UNR, MINB><<<g, 256, 0, st>>>(P);
 }
 
-// the same with a register cap for MINB resident blocks of 256 per SM (occupancy)
-template <int VW, int UNR, int MINB>
-static void fwd_vw_occ(const IterParams &P, int disc, cudaStream_t st) {
-  const unsigned g = blocks_for(threads_for<VW>((long long)P.d.nd * P.d.nang, P.d.S), 256);
-  if (disc == KL) k_fwd<KL, VW, UNR, false, MINB><<<g, 256, 0, st>>>(P);
-  else k_fwd<L2, VW, UNR, false, MINB><<<g, 256, 0, st>>>(P);
-}
-
-template <int VW, int UNR>
-static void fwd_rt(const IterParams &P, int disc, cudaStream_t st) {
-  const long long units = (long long)((P.d.nd + 2) / 3) * P.d.nang;
-  const unsigned g = blocks_for(threads_for<VW>(units, P.d.S), 256);
-  if (disc == KL) k_fwd_rt<KL, VW, UNR><<<g, 256, 0, st>>>(P);
-  else k_fwd_rt<L2, VW, UNR><<<g, 256, 0, st>>>(P);
-}
-
-static void fwd_wl(const IterParams &P, int disc, cudaStream_t st) {
-  const unsigned g = blocks_for(threads_for_wl((long long)P.d.nd * P.d.nang, P.d.S), 256);
-  if (disc == KL) k_fwd<KL, 1, 8, true><<<g, 256, 0, st>>>(P);
-  else k_fwd<L2, 1, 8, true><<<g, 256, 0, st>>>(P);
-}
-
-template <int VW, int R>
-static void fwd_run(const IterParams &P, int disc, cudaStream_t st) {
-  const long long units = (long long)((P.d.nd + R - 1) / R) * P.d.nang;
-  const unsigned g = blocks_for(threads_for<VW>(units, P.d.S), 256);
-  if (disc == KL) k_fwd_run<KL, VW, R><<<g, 256, 0, st>>>(P);
-  else k_fwd_run<L2, VW, R><<<g, 256, 0, st>>>(P);
-}
-
+cudaError_t launch_fwd_pair(const IterParams &P, int disc, int vw, cudaStream_t st);
+cudaError_t launch_fwd_flat(const IterParams &P, int disc, int vw, cudaStream_t st);
+cudaError_t launch_fwd_staged(const IterParams &P, int disc, cudaStream_t st);
 cudaError_t launch_bp_tap(const IterParams &P, int vw, cudaStream_t st);
 cudaError_t launch_bp_flat(const IterParams &P, int vw, cudaStream_t st);
 
+// default forward shape (no autotuning).  us of k_fwd_pair with 8 / 4 slices per lane, of
+// k_fwd_flat with 4 slices per thread and of the ray-table kernel (the best of 0..4, 14):
+// 16 slices (177^2, 45 angles) - / 73 / 25 / 33; 32 (64^2, 71) - / 21 / 11 / 16; 40 (101^2, 45)
+// - / 29 / 18 / 25; 64 (128^2, 71) - / 61 / 38 / 64; 92 (128^2, 71) - / 61 / 62 / 68; 240 (256^2,
+// 71) 333 / 395 / 417 / 386; 384 (512^2, 141) 5044 / 4404 / 8130 / 7795 (there 8 per lane
+// leave a quarter of the lanes idle).
+int default_fwd_shape(int S) {
+  if (S == 4) return 7;
+  if (S <= 92) return 9;
+  const int w8 = (S + 255) / 256 * 256, w4 = (S + 127) / 128 * 128;
+  return S >= 192 && w8 <= w4 + w4 / 8 ? 10 : 11;
+}
+
 cudaError_t launch_fwd(const IterParams &P, int disc, cudaStream_t st) {
   const int S = P.d.S;
-  if (S % 4 == 0) {
-    switch (P.fwd_cfg) {
-      case 1: fwd_vw<8, 8>(P, disc, st); break;
-      case 2: fwd_vw<4, 4>(P, disc, st); break;
-      case 3: fwd_vw<4, 8>(P, disc, st); break;
-      case 4: fwd_vw<1, 4>(P, disc, st); break;
-      case 5: fwd_run<8, 2>(P, disc, st); break;
-      case 6: fwd_run<8, 4>(P, disc, st); break;
-      case 7: fwd_run<4, 4>(P, disc, st); break;
-      case 8: fwd_run<4, 8>(P, disc, st); break;
-      case 9:
-        if (P.ray_start) fwd_wl(P, disc, st); else fwd_vw<8, 4>(P, disc, st);  // WL streams the ray table
-        break;
-      case 10:
-        if (P.run_start) fwd_rt<8, 4>(P, disc, st); else fwd_vw<8, 4>(P, disc, st);
-        break;
-      case 11:
-        if (P.run_start) fwd_rt<4, 8>(P, disc, st); else fwd_vw<8, 4>(P, disc, st);
-        break;
-      case 12: fwd_vw_occ<8, 8, 5>(P, disc, st); break;
-      case 13: fwd_vw_occ<8, 4, 6>(P, disc, st); break;
-      case 14: fwd_vw_occ<8, 4, 4>(P, disc, st); break;
-      case 15: fwd_vw_occ<8, 8, 4>(P, disc, st); break;
-      case 16: fwd_vw_occ<4, 8, 4>(P, disc, st); break;
-      case 17: fwd_vw_occ<8, 2, 4>(P, disc, st); break;
-      case 18: fwd_vw_occ<8, 2, 5>(P, disc, st); break;
-      case 19: fwd_vw_occ<8, 4, 5>(P, disc, st); break;
-      default: fwd_vw<8, 4>(P, disc, st); break;
-    }
-  } else if (S % 2 == 0) {
-    fwd_vw<2, 4>(P, disc, st);
-  } else {
-    fwd_vw<1, 4>(P, disc, st);
+  if (S <= 2) return launch_fwd_staged(P, disc, st);
+  if (S % 4 != 0) return launch_fwd_flat(P, disc, S % 2 == 0 ? 2 : 1, st);
+  switch (P.fwd_cfg) {
+    case 1: fwd_vw<8, 8>(P, disc, st); break;
+    case 2: fwd_vw<4, 4>(P, disc, st); break;
+    case 3: fwd_vw<4, 8>(P, disc, st); break;
+    case 4: fwd_vw<1, 4>(P, disc, st); break;
+    case 5: return launch_fwd_flat(P, disc, 2, st);
+    case 6: return launch_fwd_flat(P, disc, 1, st);
+    case 7:
+      if (S == 4) return launch_fwd_staged(P, disc, st);
+      return launch_fwd_flat(P, disc, 4, st);
+    case 8: case 9: return launch_fwd_flat(P, disc, 4, st);
+    case 10: case 11:  // without the pair table the ray-table shape
+      if (P.pair_start) return launch_fwd_pair(P, disc, P.fwd_cfg == 10 ? 8 : 4, st);
+      fwd_vw<8, 4, 4>(P, disc, st);
+      break;
+    case 12: case 13: case 14: case 15: case 16: case 17: case 18: case 19: fwd_vw<8, 4, 4>(P, disc, st); break;
+    default: fwd_vw<8, 4>(P, disc, st); break;
   }
   return cudaGetLastError();
 }
@@ -3300,6 +2972,9 @@ cudaError_t launch_update(const IterParams &P, int tgv, cudaStream_t st, int par
 
 static inline bool aligned(const void *p, int bytes) { return ((uintptr_t)p % bytes) == 0; }
 
+// slices per lane: 8 (two float4 chunks) when S is a multiple of 4, else 2, else 1
+static inline int vec_width(int S) { return (S % 4 == 0) ? 8 : (S % 2 == 0 ? 2 : 1); }
+
 static int proj_width(const void *a, const void *b, int S) {
   int vw = vec_width(S);
   if (vw == 8 && !(aligned(a, 16) && aligned(b, 16))) vw = (S % 2 == 0) ? 2 : 1;
@@ -3324,17 +2999,6 @@ cudaError_t launch_radon_ad(const float *sino, float *img, const float4 *ofs, in
   if (vw == 8) k_radon_ad<8><<<blocks_for(threads_for<8>(units, S), 256), 256, 0, st>>>(sino, img, ofs, N, nd, nang, S);
   else if (vw == 2) k_radon_ad<2><<<blocks_for(threads_for<2>(units, S), 256), 256, 0, st>>>(sino, img, ofs, N, nd, nang, S);
   else k_radon_ad<1><<<blocks_for(threads_for<1>(units, S), 256), 256, 0, st>>>(sino, img, ofs, N, nd, nang, S);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_run_count(const float4 *ofs, int N, int nd, int nang, int *count, cudaStream_t st) {
-  k_run_count<<<blocks_for((long long)((nd + 2) / 3) * nang, 128), 128, 0, st>>>(ofs, N, nd, nang, count);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_run_fill(const float4 *ofs, int N, int nd, int nang, const long long *start, int4 *ent,
-                            cudaStream_t st) {
-  k_run_fill<<<blocks_for((long long)((nd + 2) / 3) * nang, 128), 128, 0, st>>>(ofs, N, nd, nang, start, ent);
   return cudaGetLastError();
 }
 

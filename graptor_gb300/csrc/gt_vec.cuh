@@ -89,6 +89,13 @@ struct VecAcc {
 #pragma unroll
     for (int k = 0; k < VW / 2; ++k) unpack2(v[k], r[2 * k], r[2 * k + 1]);
   }
+  __device__ __forceinline__ bool finite() const {
+    float r[VW], z = 0.f;
+    get(r);
+#pragma unroll
+    for (int k = 0; k < VW; ++k) z = __fmaf_rn(r[k], 0.f, z);  // 0, or NaN once an r is infinite or NaN
+    return z == 0.f;
+  }
 };
 
 template <>

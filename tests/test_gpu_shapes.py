@@ -40,3 +40,51 @@ def test_back_projection_shapes_agree(geometry):
     for g in got[1:]:
         for k in g:
             np.testing.assert_array_equal(g[k], got[0][k], err_msg=k)
+
+
+@pytest.mark.parametrize("geometry", GEOMETRIES, ids=lambda g: f"{g[0]}-{g[1]}-{g[3] * g[4]}")
+def test_forward_projection_shapes_agree(geometry):
+    got = _iterates(*geometry, shapes=[(0, 4)] + [(s, 4) for s in (5, 6, 7, 9, 10, 11)])
+    for g in got[1:]:
+        for k in g:
+            np.testing.assert_array_equal(g[k], got[0][k], err_msg=k)
+
+
+def test_pair_shapes_keep_infinities_to_their_rays():
+    """A pixel that only one ray of a pair takes must not reach the other ray through its
+    zero weight when it is infinite or NaN."""
+    from graptor_gb300.solver import Problem
+    N, Nz, C = 24, 8, 1
+    ang = np.deg2rad(np.array([20.0, 63.0, 90.0, 131.0]))
+    f = np.abs(np.random.default_rng(8).standard_normal((Nz, ang.size, N))).astype(np.float32)
+    u = np.random.default_rng(9).random((Nz, N, N)).astype(np.float32)
+    u[0, 5, 7], u[3, 20, 2], u[6, 11, 11] = np.inf, np.nan, -np.inf
+    got = []
+    with Problem(3, N, Nz, C, N, ang, (4, 1), [0.2], normest=11.0, autotune=False) as p:
+        for fwd in (0, 10, 11):
+            p.set_data(f)
+            p.set_tuning(fwd, 4)
+            p.set("ubar", u)
+            p.run(1).synchronize()
+            got.append(p.get("ku"))
+    assert not np.isfinite(got[0]).all()
+    for g in got[1:]:
+        np.testing.assert_array_equal(g, got[0])
+
+
+@pytest.mark.parametrize("dim,N,nd,Nz", [(2, 33, 33, 1), (2, 40, 70, 2), (2, 64, 64, 1), (2, 20, 5, 4)])
+def test_staged_forward_projection_matches_oracle(dim, N, nd, Nz):
+    """One, two and four slices take the staged kernel; detectors around the 32 rays of a
+    block and around chunks of its entries."""
+    from graptor_gb300 import phantom
+    from graptor_gb300.solver import Problem
+    from oracle import oracle as O
+    ang = phantom.angles_deg(9)
+    ofs = O.radon_struct(ang, N, nd)
+    f = np.abs(np.random.default_rng(N).standard_normal((Nz, ang.size, nd))).astype(np.float32)
+    with Problem(dim, N, Nz, 1, nd, ang, (3.0, 1.5), [0.3], "L2", "TGV", "UNCORR", 1.0, 13.0) as p:
+        p.set_data(f).run(20).synchronize()
+        u, lam = p.get("u"), p.get("lambda")
+    o = O.Solver(dim, N, Nz, 1, nd, ofs, f, (3.0, 1.5), np.array([0.3]), 13.0, O.L2, O.TGV, O.UNCORR, stepsize=1.0).run(20)
+    assert np.linalg.norm(u - o.u) <= 1e-5 * np.linalg.norm(o.u)
+    assert np.linalg.norm(lam - o.lam) <= 1e-5 * np.linalg.norm(o.lam)
