@@ -20,7 +20,7 @@ struct __align__(32) dvec4 {
 
 namespace gt {
 
-enum { KL = 0, L2 = 1 };
+enum { KL = 0, L2 = 1, DATA_NONE = 2 };  // DATA_NONE: the forward projection alone
 enum { UNCORR = 0, FROB = 1, NUCL = 2 };
 
 struct Dims {

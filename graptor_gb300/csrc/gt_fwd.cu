@@ -178,6 +178,7 @@ __device__ __forceinline__ void data_step(const IterParams &P, const VecAcc<VW> 
   float a[VW], lam[VW], f[VW];
   acc.get(a);
   Vec<VW>::store(P.ku + q, a, vb);
+  if constexpr (DISC == DATA_NONE) return;
   Vec<VW>::loadw(P.lam + q, lam, vb);
   Vec<VW>::loadw(P.f + q, f, vb);
 #pragma unroll
@@ -250,7 +251,8 @@ void fwd_pair(const IterParams &P, int disc, cudaStream_t st) {
   const int np = (P.d.nd + 1) / 2, nb = (np + BG - 1) / BG, na = (P.d.nang + AG - 1) / AG;
   const dim3 g((unsigned)nb * na, (P.d.S + 32 * VW - 1) / (32 * VW));
   if (disc == KL) k_fwd_pair<KL, VW, UNR, AG, BG, MINB><<<g, AG * BG * 32, 0, st>>>(P);
-  else k_fwd_pair<L2, VW, UNR, AG, BG, MINB><<<g, AG * BG * 32, 0, st>>>(P);
+  else if (disc == L2) k_fwd_pair<L2, VW, UNR, AG, BG, MINB><<<g, AG * BG * 32, 0, st>>>(P);
+  else k_fwd_pair<DATA_NONE, VW, UNR, AG, BG, MINB><<<g, AG * BG * 32, 0, st>>>(P);
 }
 
 // ---------------------------------------------------------------------------
@@ -275,7 +277,8 @@ template <int VW, int UNR, int NT>
 void fwd_flat(const IterParams &P, int disc, cudaStream_t st) {
   const unsigned g = blocks((long long)(P.d.S / VW) * P.d.nd * P.d.nang, NT);
   if (disc == KL) k_fwd_flat<KL, VW, UNR, NT><<<g, NT, 0, st>>>(P);
-  else k_fwd_flat<L2, VW, UNR, NT><<<g, NT, 0, st>>>(P);
+  else if (disc == L2) k_fwd_flat<L2, VW, UNR, NT><<<g, NT, 0, st>>>(P);
+  else k_fwd_flat<DATA_NONE, VW, UNR, NT><<<g, NT, 0, st>>>(P);
 }
 
 // ---------------------------------------------------------------------------
@@ -347,7 +350,8 @@ template <int VW, int CH>
 void fwd_staged(const IterParams &P, int disc, cudaStream_t st) {
   const unsigned g = (unsigned)P.d.nang * ((P.d.nd + 31) / 32);
   if (disc == KL) k_fwd_staged<KL, VW, CH><<<g, 256, 0, st>>>(P);
-  else k_fwd_staged<L2, VW, CH><<<g, 256, 0, st>>>(P);
+  else if (disc == L2) k_fwd_staged<L2, VW, CH><<<g, 256, 0, st>>>(P);
+  else k_fwd_staged<DATA_NONE, VW, CH><<<g, 256, 0, st>>>(P);
 }
 
 }  // namespace

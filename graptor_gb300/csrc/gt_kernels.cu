@@ -1511,6 +1511,7 @@ __device__ __forceinline__ void fwd_body(const IterParams &P, long long bid) {
   }
   const size_t q = (size_t)b * d.S;
   sl.store(P.ku + q, acc);
+  if constexpr (DISC == DATA_NONE) return;
   float lam[VW], f[VW];
   sl.loadw(P.lam + q, lam);
   sl.load(P.f + q, f);
@@ -2065,32 +2066,53 @@ cudaError_t launch_add2(float *a, float *b, const float *d, long long n, cudaStr
 // ---------------------------------------------------------------------------
 // two-resolution subsampling (radon_tgv_primal_dual_3dsubsample.py)
 // ---------------------------------------------------------------------------
-// slices [s0, s0 + Sg) of a [X][S] field <-> a contiguous [X][Sg] field
-__global__ void k_gather_slices(const float *__restrict__ src, int S, int s0, float *__restrict__ dst, int Sg,
-                                long long X) {
+// The slices of a [X][ld] field in two groups, [0, S0) and [S0, S0 + S1), each a field of its
+// own [X][ld0], [X][ld1] (ld0, ld1: the groups' padded slice counts), and back.  One launch
+// for both groups: HBM / L2 traffic of 8 bytes per value.
+__global__ void k_split_slices(const float *__restrict__ src, int ld, int S0, int S1, float *__restrict__ d0, int ld0,
+                               float *__restrict__ d1, int ld1, long long X) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= X * Sg) return;
-  const long long x = t / Sg;
-  dst[t] = src[x * S + s0 + (t - x * Sg)];
+  const int S = S0 + S1;
+  if (t >= X * S) return;
+  const long long x = t / S;
+  const int s = (int)(t - x * S);
+  const float v = src[x * ld + s];
+  if (s < S0) d0[x * ld0 + s] = v;
+  else d1[x * ld1 + s - S0] = v;
 }
 
-__global__ void k_scatter_slices(const float *__restrict__ src, int Sg, float *__restrict__ dst, int S, int s0,
-                                 long long X) {
+__global__ void k_merge_slices(float *__restrict__ dst, int ld, int S0, int S1, const float *__restrict__ s0, int ld0,
+                               const float *__restrict__ s1, int ld1, long long X) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= X * Sg) return;
-  const long long x = t / Sg;
-  dst[x * S + s0 + (t - x * Sg)] = src[t];
+  const int S = S0 + S1;
+  if (t >= X * S) return;
+  const long long x = t / S;
+  const int s = (int)(t - x * S);
+  dst[x * ld + s] = s < S0 ? s0[x * ld0 + s] : s1[x * ld1 + s - S0];
+}
+
+// update_lambda_KL / _L2 (3-D :677-704) of one value
+__device__ __forceinline__ float lambda_step(float lam, float ku, float f, float m, float sigma, int disc) {
+  if (disc == KL) {
+    const float sv = lam + sigma * ku;
+    const float wv = sv - m;
+    const float dv = wv * wv + 4 * sigma * f * m;
+    return sv - 0.5f * (wv + sqrtf(dv));
+  }
+  return (lam + sigma * (ku - f)) * m;
 }
 
 // Sparsemultiplication (3dsubsample :403-428): for every angle j and channel c,
 // out(x_o, z_o) = sum over the row (x_o + nx_o z_o) of the interpolation matrix of
 // val * in(x_i, z_i), the column index being x_i + nx_i z_i; separately rounded
-// products summed in entry order.  Layouts [(j nx + x)][c nz + z].
+// products summed in entry order.  Layouts [(j nx + x)][c nz + z], rows of ld_i / ld_o values.
+// With lam, the data dual of the outputs is updated in the same pass (channel c's weight mu[c]).
 __global__ void k_csr_planes(const float *__restrict__ in, float *__restrict__ out, const int *__restrict__ start,
                              const int *__restrict__ idx, const float *__restrict__ val, int nang, int C, int nx_o,
-                             int nz_o, int nx_i, int nz_i) {
+                             int nz_o, int nx_i, int nz_i, int ld_i, int ld_o, float *__restrict__ lam,
+                             const float *__restrict__ f, const float *__restrict__ mu, float sigma, int disc) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int So = C * nz_o, Si = C * nz_i;
+  const int So = C * nz_o;
   if (t >= (long long)nang * nx_o * So) return;
   const int s = (int)(t % So);
   const long long jx = t / So;
@@ -2101,25 +2123,11 @@ __global__ void k_csr_planes(const float *__restrict__ in, float *__restrict__ o
   for (int e = start[row]; e < start[row + 1]; ++e) {
     const int k1 = idx[e];
     const int zi = k1 / nx_i, xi = k1 - zi * nx_i;
-    sum = __fadd_rn(sum, __fmul_rn(val[e], in[((size_t)j * nx_i + xi) * Si + c * nz_i + zi]));
+    sum = __fadd_rn(sum, __fmul_rn(val[e], in[((size_t)j * nx_i + xi) * ld_i + c * nz_i + zi]));
   }
-  out[t] = sum;
-}
-
-// update_lambda_KL / _L2 (3-D :677-704) on a sinogram [bins][S], channel s / Nz
-__global__ void k_lambda_update(float *__restrict__ lam, const float *__restrict__ ku, const float *__restrict__ f,
-                                const float *__restrict__ mu, float sigma, long long n, int S, int Nz, int disc) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const float m = mu[(int)(t % S) / Nz];
-  if (disc == 0) {
-    const float sv = lam[t] + sigma * ku[t];
-    const float wv = sv - m;
-    const float dv = wv * wv + 4 * sigma * f[t] * m;
-    lam[t] = sv - 0.5f * (wv + sqrtf(dv));
-  } else {
-    lam[t] = (lam[t] + sigma * (ku[t] - f[t])) * m;
-  }
+  const size_t o = (size_t)jx * ld_o + s;
+  out[o] = sum;
+  if (lam) lam[o] = lambda_step(lam[o], sum, f[o], mu[c], sigma, disc);
 }
 
 // sum of squares in FP64, block partials
@@ -2162,23 +2170,21 @@ __global__ void k_scale_f32(float *__restrict__ x, long long n, float s) {
   if (t < n) x[t] *= s;
 }
 
-cudaError_t launch_gather_slices(const float *src, int S, int s0, float *dst, int Sg, long long X, cudaStream_t st) {
-  k_gather_slices<<<(unsigned)((X * Sg + 255) / 256), 256, 0, st>>>(src, S, s0, dst, Sg, X);
+cudaError_t launch_split_slices(const float *src, int ld, int S0, int S1, float *d0, int ld0, float *d1, int ld1,
+                                long long X, cudaStream_t st) {
+  k_split_slices<<<(unsigned)((X * (S0 + S1) + 255) / 256), 256, 0, st>>>(src, ld, S0, S1, d0, ld0, d1, ld1, X);
   return cudaGetLastError();
 }
-cudaError_t launch_scatter_slices(const float *src, int Sg, float *dst, int S, int s0, long long X, cudaStream_t st) {
-  k_scatter_slices<<<(unsigned)((X * Sg + 255) / 256), 256, 0, st>>>(src, Sg, dst, S, s0, X);
+cudaError_t launch_merge_slices(float *dst, int ld, int S0, int S1, const float *s0, int ld0, const float *s1, int ld1,
+                                long long X, cudaStream_t st) {
+  k_merge_slices<<<(unsigned)((X * (S0 + S1) + 255) / 256), 256, 0, st>>>(dst, ld, S0, S1, s0, ld0, s1, ld1, X);
   return cudaGetLastError();
 }
 cudaError_t launch_csr_planes(const float *in, float *out, const int *start, const int *idx, const float *val,
-                              int nang, int C, int nx_o, int nz_o, int nx_i, int nz_i, cudaStream_t st) {
-  k_csr_planes<<<(unsigned)(((long long)nang * nx_o * C * nz_o + 255) / 256), 256, 0, st>>>(in, out, start, idx, val, nang, C,
-                                                                                  nx_o, nz_o, nx_i, nz_i);
-  return cudaGetLastError();
-}
-cudaError_t launch_lambda_update(float *lam, const float *ku, const float *f, const float *mu, float sigma,
-                                 long long n, int S, int Nz, int disc, cudaStream_t st) {
-  k_lambda_update<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(lam, ku, f, mu, sigma, n, S, Nz, disc);
+                              int nang, int C, int nx_o, int nz_o, int nx_i, int nz_i, int ld_i, int ld_o, float *lam,
+                              const float *f, const float *mu, float sigma, int disc, cudaStream_t st) {
+  k_csr_planes<<<(unsigned)(((long long)nang * nx_o * C * nz_o + 255) / 256), 256, 0, st>>>(
+      in, out, start, idx, val, nang, C, nx_o, nz_o, nx_i, nz_i, ld_i, ld_o, lam, f, mu, sigma, disc);
   return cudaGetLastError();
 }
 cudaError_t launch_sqdiff(const float *a, const float *b, long long n, double *part, int nb, cudaStream_t st) {
@@ -2538,6 +2544,11 @@ bool dual_z2_ok(const IterParams &P, int tgv, int cpl) {
 int num_dual_configs(const IterParams &P) { return P.d.C <= 4 ? 10 : 1; }
 bool dual_cl_ok(const IterParams &P, int cpl) { return cpl != NUCL && P.d.C <= 4; }
 bool dual_cl2_ok(const IterParams &P, int cpl) { return dual_cl_ok(P, cpl) && P.d.dim == 3 && P.d.Nz % 2 == 0; }
+// dual shape without autotuning: the shapes of one channel per thread where they apply
+// (256^2 x 60 x 4: 9 takes 0.23, 8 0.29, 3 0.34 and 0 0.43 ms)
+int default_dual_shape(const IterParams &P, int cpl) {
+  return dual_cl2_ok(P, cpl) ? 9 : dual_cl_ok(P, cpl) ? 8 : P.d.C <= 4 ? 3 : 0;
+}
 // shape 7 or 9 where it is not available falls back to 6 or 8 (one slice per thread)
 
 template <int CPL>
@@ -2718,7 +2729,8 @@ template <int VW, int UNR, int MINB = 1>
 static void fwd_vw(const IterParams &P, int disc, cudaStream_t st) {
   const unsigned g = blocks_for(threads_for<VW>((long long)P.d.nd * P.d.nang, P.d.S), 256);
   if (disc == KL) k_fwd<KL, VW, UNR, MINB><<<g, 256, 0, st>>>(P);
-  else k_fwd<L2, VW, UNR, MINB><<<g, 256, 0, st>>>(P);
+  else if (disc == L2) k_fwd<L2, VW, UNR, MINB><<<g, 256, 0, st>>>(P);
+  else k_fwd<DATA_NONE, VW, UNR, MINB><<<g, 256, 0, st>>>(P);
 }
 
 cudaError_t launch_fwd_pair(const IterParams &P, int disc, int vw, cudaStream_t st);
