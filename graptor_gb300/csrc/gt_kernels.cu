@@ -2216,18 +2216,37 @@ __global__ void k_fill(T *__restrict__ x, size_t n, T v) {
 // ===========================================================================
 // FP64 operator-norm power iteration (radon_normest, 3-D :1018-1030), one slice
 // ===========================================================================
+// Geometry in fixed point, FIX = 44 fraction bits: FP64 arithmetic runs at a sixty-fourth of the
+// FP32 rate here, and computed in FP64 the detector coordinate, its floor, fraction and
+// weights were nearly all of the projectors' time (128^2, 71 angles: 0.45 ms per round).
+// The coordinate t = x X + y Y + off is a sum of 64-bit integers (|t| < 2^18, rounding of
+// X, Y and off 3e-14 each, as that of an FP64 t of a few hundred), its bin a shift and its
+// fraction a mantissa; only the sums stay FP64 operations.  Wider geometries take FIX = 30
+// (|t| < 2^32; an FP64 t beyond 2^18 has no more than 35 fraction bits itself).
+template <int FIX>
+__device__ __forceinline__ long long to_fix(double v) { return __double2ll_rn(v * (double)(1ll << FIX)); }
+
+// f 2^-FIX for 0 <= f <= 2^FIX, exactly
+template <int FIX>
+__device__ __forceinline__ double from_fix(long long f) {
+  return __longlong_as_double((f << (52 - FIX)) + 0x3ff0000000000000ll) - 1.0;
+}
+
 // FP64 forward projection of one slice, a warp per ray: lane l sums rows l, l+32,
 // ..., then a fixed butterfly adds the 32 partial sums (deterministic).  Weights
-// and bounds as the float projector, in double (the x range is widened by one
-// pixel and the weight test decides).
+// and bounds as the float projector (the x range is widened by one pixel and the
+// weight test decides).
+template <int FIX>
 __global__ void k_radon64_warp(const double *__restrict__ img, double *__restrict__ sino,
                                const dvec4 *__restrict__ ofs, int N, int nd, int nang) {
+  constexpr long long FIX_ONE = 1ll << FIX;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long ray = t >> 5;
   const int lane = threadIdx.x & 31;
   if (ray >= (long long)nd * nang) return;  // whole warps leave together
   const int j = (int)(ray / nd), i = (int)(ray - (long long)j * nd);
   const dvec4 o = ofs[j];
+  const long long X = to_fix<FIX>(o.x), Y = to_fix<FIX>(o.y), off = to_fix<FIX>(o.z) - (long long)i * FIX_ONE;
   double acc = 0.0;
   for (int y = lane; y < N; y += 32) {
     const double dd = y * o.y + o.z;
@@ -2240,33 +2259,53 @@ __global__ void k_radon64_warp(const double *__restrict__ img, double *__restric
       xl = (int)((i + 1 - dd) * o.w); xh = (int)((i - 1 - dd) * o.w);
     }
     xl = max(xl - 1, 0); xh = min(xh + 1, N - 1);
-    for (int x = xl; x <= xh; ++x) {
-      const double wgt = 1.0 - fabs(x * o.x + dd - i);
-      if (wgt > 0.0) acc += wgt * img[(size_t)y * N + x];
+    long long c = xl * X + y * Y + off;  // t - i
+    const double *__restrict__ row = img + (size_t)y * N;
+    for (int x = xl; x <= xh; ++x, c += X) {
+      const long long wgt = FIX_ONE - (c < 0 ? -c : c);
+      if (wgt > 0) acc = __fma_rn(from_fix<FIX>(wgt), row[x], acc);
     }
   }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+  for (int off2 = 16; off2 > 0; off2 >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off2);
   if (lane == 0) sino[ray] = acc;
 }
 
-__global__ void k_radon_ad64(const double *__restrict__ sino, double *__restrict__ img, const dvec4 *__restrict__ ofs,
-                             int N, int nd, int nang) {
+// back projection: a thread per pixel; the block converts ANG angles at a time
+template <int FIX>
+__global__ void __launch_bounds__(128) k_radon_ad64(const double *__restrict__ sino, double *__restrict__ img,
+                                                    const dvec4 *__restrict__ ofs, int N, int nd, int nang) {
+  constexpr long long FIX_ONE = 1ll << FIX;
+  constexpr int ANG = 128;
+  __shared__ long long sx[ANG], sy[ANG], so[ANG];
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= N * N) return;
   const int y = t / N, x = t - y * N;
+  const long long end = (long long)nd * FIX_ONE;
   double acc = 0.0;
-  for (int j = 0; j < nang; ++j) {
-    const dvec4 o = ofs[j];
-    const double tt = x * o.x + y * o.y + o.z;
-    if (tt > -1.0 && tt < nd) {
-      const double fl = floor(tt), p = tt - fl;
-      const int il = (int)fl;
-      if (il >= 0) acc += (1.0 - p) * sino[(size_t)j * nd + il];
-      if (il <= nd - 2) acc += p * sino[(size_t)j * nd + il + 1];
+  for (int j0 = 0; j0 < nang; j0 += ANG) {
+    __syncthreads();
+    for (int k = threadIdx.x; k < min(ANG, nang - j0); k += blockDim.x) {
+      const dvec4 o = ofs[j0 + k];
+      sx[k] = to_fix<FIX>(o.x);
+      sy[k] = to_fix<FIX>(o.y);
+      so[k] = to_fix<FIX>(o.z);
+    }
+    __syncthreads();
+    if (t >= N * N) continue;
+    const int m = min(ANG, nang - j0);
+#pragma unroll 4
+    for (int k = 0; k < m; ++k) {
+      const long long c = x * sx[k] + y * sy[k] + so[k];
+      if (c > -FIX_ONE && c < end) {
+        const int il = (int)(c >> FIX);
+        const double p = from_fix<FIX>(c & (FIX_ONE - 1));
+        const double *__restrict__ row = sino + (size_t)(j0 + k) * nd;
+        if (il >= 0) acc = __fma_rn(1.0 - p, row[il], acc);
+        if (il <= nd - 2) acc = __fma_rn(p, row[il + 1], acc);
+      }
     }
   }
-  img[t] = acc;
+  if (t < N * N) img[t] = acc;
 }
 
 // deterministic two-level sum: block partials then one block
@@ -3149,8 +3188,14 @@ cudaError_t normest64(const dvec4 *ofs, int N, int nd, int nang, int rounds, dou
       prev = s;
     }
     k_scale64<<<64, 256, 0, st>>>(d_img, n, d_part + nb);
-    k_radon64_warp<<<blocks_for(32LL * nd * nang, 256), 256, 0, st>>>(d_img, d_sino, ofs, N, nd, nang);
-    k_radon_ad64<<<blocks_for((long long)n, 128), 128, 0, st>>>(d_sino, d_img, ofs, N, nd, nang);
+    const unsigned gf = blocks_for(32LL * nd * nang, 256), gb = blocks_for((long long)n, 128);
+    if ((long long)nd + 2LL * N < (1 << 18)) {
+      k_radon64_warp<44><<<gf, 256, 0, st>>>(d_img, d_sino, ofs, N, nd, nang);
+      k_radon_ad64<44><<<gb, 128, 0, st>>>(d_sino, d_img, ofs, N, nd, nang);
+    } else {
+      k_radon64_warp<30><<<gf, 256, 0, st>>>(d_img, d_sino, ofs, N, nd, nang);
+      k_radon_ad64<30><<<gb, 128, 0, st>>>(d_sino, d_img, ofs, N, nd, nang);
+    }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   k_sum64_partial<<<nb, 256, 0, st>>>(d_img, n, d_part);

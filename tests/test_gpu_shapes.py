@@ -88,3 +88,24 @@ def test_staged_forward_projection_matches_oracle(dim, N, nd, Nz):
     o = O.Solver(dim, N, Nz, 1, nd, ofs, f, (3.0, 1.5), np.array([0.3]), 13.0, O.L2, O.TGV, O.UNCORR, stepsize=1.0).run(20)
     assert np.linalg.norm(u - o.u) <= 1e-5 * np.linalg.norm(o.u)
     assert np.linalg.norm(lam - o.lam) <= 1e-5 * np.linalg.norm(o.lam)
+
+
+@pytest.mark.parametrize("N,nd,deg", [(1, 1, (10,)), (19, 19, (0, 45, 90, 135)), (40, 23, (-70, -20, 3, 70, 89.99)),
+                                      (64, 90, tuple(range(20, 161, 10))), (33, 33, tuple(range(0, 180)))])
+def test_operator_norm_matches_fp64_power_iteration(N, nd, deg):
+    """The fixed-point projectors of the norm estimate (rounding about 1e-13 in the weights)
+    against the power iteration with the exact FP64 matrix; it stops when two
+    consecutive sums agree to 1e-8.  More than 128 angles: a second chunk of the table."""
+    from graptor_gb300.solver import Problem
+    from oracle import fp64 as F
+    ang = np.deg2rad(np.asarray(deg, np.float64))
+    R = F.radon_matrix(ang, N, nd)
+    x = np.ones(N * N)
+    for _ in range(30):
+        s = x.sum()
+        x = R.T @ (R @ (x / s))
+    with Problem(2, N, 1, 1, nd, ang, (4, 1), [0.2], "L2", "TGV", "UNCORR", autotune=False) as p:
+        p.set_data(np.ones((1, ang.size, nd), np.float32))
+        ne = p.scalars["normest"]
+    want = np.sqrt(x.sum())
+    assert abs(ne - want) <= 1e-6 * want, (ne, want)
