@@ -10,25 +10,17 @@
 //                       inputs with 16k in and out channels run on the tensor cores
 //                       (k_conv3d_tc: tcgen05 MMA, accumulator in tensor memory)
 //   gt_nn_flip_weights  w[co][ci][t] -> w'[ci][co][K3-1-t]   (data-gradient weights)
-//   gt_nn_conv3d_wgrad  weight gradient as a split-K GEMM  dW = dY * im2col(X)^T
-//   gt_nn_bias_grad, gt_nn_relu_bwd, gt_nn_pool2 / _bwd, gt_nn_up2 / _bwd,
+//   gt_nn_conv3d_wgrad, gt_nn_bias_grad  parameter gradients (gt_nn_grad.cu)
+//   gt_nn_relu_bwd, gt_nn_pool2 / _bwd, gt_nn_up2 / _bwd,
 //   gt_nn_mse, gt_nn_adam, gt_nn_cast
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include "graptor_gb300.h"
+#include "gt_nn.cuh"
 #include "gt_tc.cuh"
 
 namespace {
-
-template <class T> __device__ __forceinline__ float ld(const T *p) { return (float)*p; }
-template <> __device__ __forceinline__ float ld<__nv_bfloat16>(const __nv_bfloat16 *p) { return __bfloat162float(*p); }
-template <class T> __device__ __forceinline__ void st(T *p, float v) { *p = (T)v; }
-template <> __device__ __forceinline__ void st<__nv_bfloat16>(__nv_bfloat16 *p, float v) { *p = __float2bfloat16_rn(v); }
-
-struct Shape {
-  int B, D, H, W;
-};
 
 // ---------------------------------------------------------------------------
 // forward convolution: a thread computes CO_T output channels for VX voxels
@@ -499,98 +491,6 @@ __global__ void k_flip(const __nv_bfloat16 *__restrict__ w, __nv_bfloat16 *__res
   wf[((size_t)ci * Co + co) * K3 + (K3 - 1 - tp)] = w[t];
 }
 
-// ---------------------------------------------------------------------------
-// weight gradient: dW[co][ci*K3 + t] = sum_{b, voxel} dY[b][co][v] X[b][ci][v + off(t)]
-// GEMM M = Co, N = Ci*K3, K = voxels; a block computes a 16 x 64 tile over one
-// K-chunk and writes it to part[chunk]; k_wgrad_reduce sums the chunks in order.
-// ---------------------------------------------------------------------------
-constexpr int WG_M = 16, WG_N = 64, WG_K = 32;
-
-template <class TX, int KS>
-__global__ void __launch_bounds__(256) k_wgrad(const float *__restrict__ dy, int Co, int Cdy, int dy_off,
-                                               const TX *__restrict__ x, int Ci, int Cx, int x_off, Shape s,
-                                               long long kchunk, float *__restrict__ part) {
-  constexpr int K3 = KS * KS * KS, R = KS / 2;
-  __shared__ float sa[WG_M][WG_K + 1];
-  __shared__ float sb[WG_K][WG_N + 1];
-  const int m0 = blockIdx.y * WG_M, n0 = blockIdx.x * WG_N, N = Ci * K3;
-  const long long nvox = (long long)s.B * s.D * s.H * s.W;
-  const long long k0 = (long long)blockIdx.z * kchunk, k1 = min(nvox, k0 + kchunk);
-  const size_t plane = (size_t)s.H * s.W, vol = plane * s.D;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // 16 x 16 threads, 4 columns each
-  float acc[4] = {0, 0, 0, 0};
-  for (long long kb = k0; kb < k1; kb += WG_K) {
-    __syncthreads();
-    for (int q = threadIdx.x; q < WG_M * WG_K; q += blockDim.x) {
-      const int m = q / WG_K, kk = q - m * WG_K;
-      const long long v = kb + kk;
-      float val = 0.f;
-      if (m0 + m < Co && v < k1) {
-        const long long bb = v / vol, rv = v - bb * vol;
-        val = dy[((size_t)bb * Cdy + dy_off + m0 + m) * vol + rv];
-      }
-      sa[m][kk] = val;
-    }
-    for (int q = threadIdx.x; q < WG_K * WG_N; q += blockDim.x) {
-      const int kk = q / WG_N, n = q - kk * WG_N;
-      const long long v = kb + kk;
-      float val = 0.f;
-      if (n0 + n < N && v < k1) {
-        const int ci = (n0 + n) / K3, tp = (n0 + n) - ci * K3;
-        const int kd = tp / (KS * KS), kh = (tp / KS) % KS, kw = tp % KS;
-        long long r = v;
-        const int ww = (int)(r % s.W); r /= s.W;
-        const int hh = (int)(r % s.H); r /= s.H;
-        const int dd = (int)(r % s.D); const int bb = (int)(r / s.D);
-        const int zd = dd + kd - R, zh = hh + kh - R, zw = ww + kw - R;
-        if (zd >= 0 && zd < s.D && zh >= 0 && zh < s.H && zw >= 0 && zw < s.W)
-          val = ld<TX>(x + ((size_t)bb * Cx + x_off + ci) * vol + (size_t)zd * plane + (size_t)zh * s.W + zw);
-      }
-      sb[kk][n] = val;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < WG_K; ++kk) {
-      const float a = sa[ty][kk];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[j] = fmaf(a, sb[kk][tx + 16 * j], acc[j]);
-    }
-  }
-  const int m = m0 + ty;
-  if (m >= Co) return;
-  for (int j = 0; j < 4; ++j) {
-    const int n = n0 + tx + 16 * j;
-    if (n < N) part[((size_t)blockIdx.z * Co + m) * N + n] = acc[j];
-  }
-}
-
-__global__ void k_wgrad_reduce(const float *__restrict__ part, int nchunk, long long n, float *__restrict__ g,
-                               int accumulate) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  float a = 0.f;
-  for (int c = 0; c < nchunk; ++c) a += part[(size_t)c * n + t];
-  g[t] = accumulate ? g[t] + a : a;
-}
-
-// db[co] (+)= sum over batch and voxels of dY (channel-offset view; one block per
-// channel, fixed summation order)
-__global__ void k_bias_grad(const float *__restrict__ dy, int Co, int Cdy, int dy_off, long long vol, int B,
-                            float *__restrict__ db, int accumulate) {
-  __shared__ float sh[256];
-  const int co = blockIdx.x;
-  float a = 0.f;
-  for (int b = 0; b < B; ++b)
-    for (long long v = threadIdx.x; v < vol; v += blockDim.x) a += dy[((size_t)b * Cdy + dy_off + co) * vol + v];
-  sh[threadIdx.x] = a;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) db[co] = accumulate ? db[co] + sh[0] : sh[0];
-}
-
 // dY *= (Y > 0) for a ReLU output Y; dY and Y are the same channel-offset view
 // (channels [co_off, co_off+C) of Cy-channel tensors)
 template <class TY>
@@ -728,8 +628,6 @@ __global__ void k_cast_b2f(const __nv_bfloat16 *__restrict__ a, float *__restric
   if (t < n) b[t] = __bfloat162float(a[t]);
 }
 
-inline unsigned nblk(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
-
 template <class TI, class TO, int KS, int CO_T>
 cudaError_t conv_t(const void *x, int Ci, int Cx, int x_off, const void *w, const float *bias, void *y, int Co, int Cy,
                    int co_off, Shape s, int relu, int accumulate, cudaStream_t st) {
@@ -750,17 +648,6 @@ cudaError_t conv_k(int ks, const void *x, int Ci, int Cx, int x_off, const void 
 }
 
 }  // namespace
-
-namespace gt {
-int set_error(int code, const char *msg);
-int cuda_error(cudaError_t e, const char *what, int line);
-}  // namespace gt
-
-#define NN_CK(expr, what)                                              \
-  do {                                                                 \
-    cudaError_t e_ = (expr);                                           \
-    if (e_ != cudaSuccess) return gt::cuda_error(e_, what, __LINE__);   \
-  } while (0)
 
 extern "C" {
 
@@ -856,43 +743,6 @@ int gt_nn_flip_weights(const void *w_bf16, void *wf_bf16, int Co, int Ci, int ks
   k_flip<<<nblk((long long)Co * Ci * K3, 256), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16 *)w_bf16, (__nv_bfloat16 *)wf_bf16, Co, Ci, K3);
   NN_CK(cudaGetLastError(), "gt_nn_flip_weights");
-  return GT_OK;
-}
-
-// part must hold nchunk * Co * Ci * K3 floats; nchunk = ceil(voxels / kchunk)
-int gt_nn_conv3d_wgrad(const float *dy, int Co, int Cdy, int dy_off, const void *x, int x_dtype, int Ci, int Cx,
-                       int x_off, int B, int D, int H, int W, int ksize, long long kchunk, float *part, float *g,
-                       int accumulate, void *stream) {
-  if (!dy || !x || !part || !g || kchunk < 1 || dy_off < 0 || dy_off + Co > Cdy || x_off < 0 || x_off + Ci > Cx)
-    return gt::set_error(GT_ERR_ARG, "gt_nn_conv3d_wgrad: bad argument");
-  const int K3 = ksize * ksize * ksize, N = Ci * K3;
-  const long long nvox = (long long)B * D * H * W;
-  const long long nchunk = (nvox + kchunk - 1) / kchunk;
-  if (nchunk > 65535) return gt::set_error(GT_ERR_ARG, "gt_nn_conv3d_wgrad: kchunk too small (more than 65535 chunks)");
-  const Shape s{B, D, H, W};
-  cudaStream_t st = (cudaStream_t)stream;
-  dim3 grid(nblk(N, WG_N), nblk(Co, WG_M), (unsigned)nchunk);
-  if (ksize == 3 && x_dtype == 1)
-    k_wgrad<__nv_bfloat16, 3><<<grid, 256, 0, st>>>(dy, Co, Cdy, dy_off, (const __nv_bfloat16 *)x, Ci, Cx, x_off, s, kchunk, part);
-  else if (ksize == 1 && x_dtype == 1)
-    k_wgrad<__nv_bfloat16, 1><<<grid, 256, 0, st>>>(dy, Co, Cdy, dy_off, (const __nv_bfloat16 *)x, Ci, Cx, x_off, s, kchunk, part);
-  else if (ksize == 3 && x_dtype == 0)
-    k_wgrad<float, 3><<<grid, 256, 0, st>>>(dy, Co, Cdy, dy_off, (const float *)x, Ci, Cx, x_off, s, kchunk, part);
-  else if (ksize == 1 && x_dtype == 0)
-    k_wgrad<float, 1><<<grid, 256, 0, st>>>(dy, Co, Cdy, dy_off, (const float *)x, Ci, Cx, x_off, s, kchunk, part);
-  else
-    return gt::set_error(GT_ERR_ARG, "gt_nn_conv3d_wgrad: ksize 1 or 3, dtype 0 or 1");
-  const long long n = (long long)Co * N;
-  k_wgrad_reduce<<<nblk(n, 256), 256, 0, st>>>(part, (int)nchunk, n, g, accumulate);
-  NN_CK(cudaGetLastError(), "gt_nn_conv3d_wgrad");
-  return GT_OK;
-}
-
-int gt_nn_bias_grad(const float *dy, int Co, int Cdy, int dy_off, int B, long long vol, float *db, int accumulate,
-                    void *stream) {
-  if (!dy || !db || Co < 1 || dy_off < 0 || dy_off + Co > Cdy) return gt::set_error(GT_ERR_ARG, "gt_nn_bias_grad: bad argument");
-  k_bias_grad<<<Co, 256, 0, (cudaStream_t)stream>>>(dy, Co, Cdy, dy_off, vol, B, db, accumulate);
-  NN_CK(cudaGetLastError(), "gt_nn_bias_grad");
   return GT_OK;
 }
 

@@ -151,10 +151,11 @@ class UNet3D:
         self._bufs = {key: b}  # one shape at a time
         return b
 
-    def _kchunk(self, nvox, n_cols, co):
-        tiles = ((n_cols + 63) // 64) * ((co + 15) // 16)
-        chunks = max(1, min(512, math.ceil(2 * 152 * 4 / tiles)))
-        return max(1024, math.ceil(nvox / chunks))
+    def _kchunk(self, nvox, ci, co, k):
+        """Voxels per partial sum of the weight gradient: two blocks per SM over the channel
+        tiles (16 x 16 channels, 8 x 4 for 1x1x1 kernels), at least a tile of 128 voxels each."""
+        tiles = -(-ci // 16) * -(-co // 16) if k == 3 else -(-ci // 8) * -(-co // 4)
+        return max(128, math.ceil(nvox / math.ceil(2 * 152 / tiles)))
 
     def _ensure_part(self, B, D, H, W):
         need = 1
@@ -162,7 +163,7 @@ class UNet3D:
             lvl = {"enc1a": 0, "enc1b": 0, "enc2a": 1, "enc2b": 1, "bota": 2, "botb": 2, "dec2a": 1, "dec2b": 1,
                    "dec1a": 0, "dec1b": 0, "head": 0}[name]
             nvox = B * (D >> lvl) * (H >> lvl) * (W >> lvl)
-            kc = self._kchunk(nvox, ci * k ** 3, co)
+            kc = self._kchunk(nvox, ci, co, k)
             need = max(need, math.ceil(nvox / kc) * co * ci * k ** 3)
         if self._part is None or self._part.numel() < need:
             self._part = self.torch.empty(need, dtype=self.torch.float32, device=self.dev)
@@ -211,7 +212,7 @@ class UNet3D:
         if relu:
             _ck(lib.gt_nn_relu_bwd(_p(gy), _p(y), BF16, co, Cg, goff, B, vol, stream))
         nvox = B * vol
-        kc = self._kchunk(nvox, ci * k ** 3, co)
+        kc = self._kchunk(nvox, ci, co, k)
         _ck(lib.gt_nn_conv3d_wgrad(_p(gy), co, Cg, goff, _p(x), xdt, ci, Cx, xoff, B, D, H, W, k, kc, _p(self._part),
                                    self.gptr(name), 0, stream))
         _ck(lib.gt_nn_bias_grad(_p(gy), co, Cg, goff, B, vol, self.bptr(name, "grad"), 0, stream))

