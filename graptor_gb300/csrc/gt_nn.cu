@@ -19,23 +19,78 @@
 #include "graptor_gb300.h"
 #include "gt_nn.cuh"
 #include "gt_tc.cuh"
+#include "gt_vec.cuh"
 
 namespace {
 
 // ---------------------------------------------------------------------------
-// forward convolution: a thread computes CO_T output channels for VX voxels
-// along W; the block stages the weights of its channel tile, CI_CH input
-// channels at a time, in shared memory (converted to FP32).
+// forward convolution on the CUDA cores (float32 inputs: the data gradients; and the layers the
+// tensor cores do not take): a thread computes CO_T output channels for VX voxels along W; the
+// block stages the weights of its channel tile, CI_CH input channels at a time, in shared
+// memory (converted to FP32).
+//
+// Bound by the multiply-adds and the weights' broadcasts from shared memory (128 bytes a clock
+// and SM), so a weight serves VX voxels and the output channels go in pairs through packed
+// multiply-adds (fma.rn.f32x2, each half rounding as a scalar one; the order of every sum
+// is input channel, then tap).  16 -> 16 channels on 4 x 16 x 64 x 64 voxels, float32: 142 us with
+// 8 channels x 4 voxels and scalar multiply-adds.
 // ---------------------------------------------------------------------------
 constexpr int CI_CH = 8;
+
+// the VX voxels of a row at w0 and one neighbour on each side (0 outside the row); vec: the row
+// starts on a 16-byte boundary and W is a multiple of VX
+template <int VX, int R>
+__device__ __forceinline__ void row_load(const float *__restrict__ row, int w0, int W, bool vec,
+                                         float (&v)[VX + 2 * R]) {
+  if (vec) {
+#pragma unroll
+    for (int q = 0; q < VX; q += 4) {
+      const float4 f = __ldg(reinterpret_cast<const float4 *>(row + w0 + q));
+      v[R + q] = f.x; v[R + q + 1] = f.y; v[R + q + 2] = f.z; v[R + q + 3] = f.w;
+    }
+    if (R) {
+      v[0] = w0 > 0 ? __ldg(row + w0 - 1) : 0.f;
+      v[VX + 2 * R - 1] = w0 + VX < W ? __ldg(row + w0 + VX) : 0.f;
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < VX + 2 * R; ++q) {
+      const int w = w0 + q - R;
+      v[q] = (w >= 0 && w < W) ? row[w] : 0.f;
+    }
+  }
+}
+
+template <int VX, int R>
+__device__ __forceinline__ void row_load(const __nv_bfloat16 *__restrict__ row, int w0, int W, bool vec,
+                                         float (&v)[VX + 2 * R]) {
+  if (vec) {
+#pragma unroll
+    for (int q = 0; q < VX; q += 4) {
+      const uint2 f = __ldg(reinterpret_cast<const uint2 *>(row + w0 + q));
+      v[R + q] = __uint_as_float(f.x << 16); v[R + q + 1] = __uint_as_float(f.x & 0xffff0000u);
+      v[R + q + 2] = __uint_as_float(f.y << 16); v[R + q + 3] = __uint_as_float(f.y & 0xffff0000u);
+    }
+    if (R) {
+      v[0] = w0 > 0 ? ld(row + w0 - 1) : 0.f;
+      v[VX + 2 * R - 1] = w0 + VX < W ? ld(row + w0 + VX) : 0.f;
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < VX + 2 * R; ++q) {
+      const int w = w0 + q - R;
+      v[q] = (w >= 0 && w < W) ? ld(row + w) : 0.f;
+    }
+  }
+}
 
 template <class TI, class TO, int KS, int CO_T, int VX>
 __global__ void __launch_bounds__(128) k_conv3d(const TI *__restrict__ x, int Ci, int Cx, int x_off,
                                                 const __nv_bfloat16 *__restrict__ w,
                                                 const float *__restrict__ bias, TO *__restrict__ y, int Co, int Cy,
-                                                int co_off, Shape s, int relu, int accumulate) {
-  constexpr int K3 = KS * KS * KS, R = KS / 2;
-  __shared__ float sw[CO_T * CI_CH * K3];
+                                                int co_off, Shape s, int relu, int accumulate, int vec) {
+  constexpr int K3 = KS * KS * KS, R = KS / 2, CP = CO_T / 2;
+  __shared__ gt::f32x2 sw[CI_CH * K3 * CP];  // [input channel][tap][output channel pair]
   const int co0 = blockIdx.y * CO_T;
   const long long nvox = (long long)s.B * s.D * s.H * (s.W / VX);
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -49,18 +104,23 @@ __global__ void __launch_bounds__(128) k_conv3d(const TI *__restrict__ x, int Ci
     w0 = wq * VX;
   }
   const size_t plane = (size_t)s.H * s.W, vol = plane * s.D;
-  float acc[CO_T][VX];
+  gt::f32x2 acc2[CP][VX];
 #pragma unroll
-  for (int c = 0; c < CO_T; ++c) {
-    const float bv = (bias && co0 + c < Co) ? bias[co0 + c] : 0.f;
+  for (int c = 0; c < CP; ++c) {
+    const float b0 = (bias && co0 + 2 * c < Co) ? bias[co0 + 2 * c] : 0.f;
+    const float b1 = (bias && co0 + 2 * c + 1 < Co) ? bias[co0 + 2 * c + 1] : 0.f;
 #pragma unroll
-    for (int v = 0; v < VX; ++v) acc[c][v] = bv;
+    for (int v = 0; v < VX; ++v) acc2[c][v] = gt::pack2(b0, b1);
   }
   for (int ci0 = 0; ci0 < Ci; ci0 += CI_CH) {
     __syncthreads();
-    for (int k = threadIdx.x; k < CO_T * CI_CH * K3; k += blockDim.x) {
-      const int c = k / (CI_CH * K3), rem = k - c * CI_CH * K3, ci = rem / K3, tp = rem - ci * K3;
-      sw[k] = (co0 + c < Co && ci0 + ci < Ci) ? __bfloat162float(w[((size_t)(co0 + c) * Ci + ci0 + ci) * K3 + tp]) : 0.f;
+    for (int k = threadIdx.x; k < CI_CH * K3 * CP; k += blockDim.x) {
+      const int c = 2 * (k % CP), tp = (k / CP) % K3, ci = k / (CP * K3);
+      float wv[2];
+#pragma unroll
+      for (int o = 0; o < 2; ++o)
+        wv[o] = (co0 + c + o < Co && ci0 + ci < Ci) ? ld(w + ((size_t)(co0 + c + o) * Ci + ci0 + ci) * K3 + tp) : 0.f;
+      sw[k] = gt::pack2(wv[0], wv[1]);
     }
     __syncthreads();
     if (!active) continue;
@@ -75,27 +135,30 @@ __global__ void __launch_bounds__(128) k_conv3d(const TI *__restrict__ x, int Ci
         for (int kh = 0; kh < KS; ++kh) {
           const int hh = h + kh - R;
           if (hh < 0 || hh >= s.H) continue;
-          const TI *row = xc + (size_t)dd * plane + (size_t)hh * s.W;
-          float xv[VX + KS - 1];
+          float xv[VX + 2 * R];
+          row_load<VX, R>(xc + (size_t)dd * plane + (size_t)hh * s.W, w0, s.W, vec, xv);
+          gt::f32x2 xx[VX + 2 * R];
 #pragma unroll
-          for (int q = 0; q < VX + KS - 1; ++q) {
-            const int ww = w0 + q - R;
-            xv[q] = (ww >= 0 && ww < s.W) ? ld<TI>(row + ww) : 0.f;
-          }
+          for (int q = 0; q < VX + 2 * R; ++q) xx[q] = gt::pack2(xv[q], xv[q]);
 #pragma unroll
           for (int kw = 0; kw < KS; ++kw) {
-            const int tp = (kd * KS + kh) * KS + kw;
+            const gt::f32x2 *wt = sw + (ci * K3 + (kd * KS + kh) * KS + kw) * CP;
 #pragma unroll
-            for (int c = 0; c < CO_T; ++c) {
-              const float wv = sw[(c * CI_CH + ci) * K3 + tp];
+            for (int c = 0; c < CP; ++c) {
+              const gt::f32x2 wv = wt[c];
 #pragma unroll
-              for (int v = 0; v < VX; ++v) acc[c][v] = fmaf(wv, xv[v + kw], acc[c][v]);
+              for (int v = 0; v < VX; ++v) gt::fma2(acc2[c][v], wv, xx[v + kw]);
             }
           }
         }
       }
     }
   }
+  float acc[CO_T][VX];
+#pragma unroll
+  for (int c = 0; c < CP; ++c)
+#pragma unroll
+    for (int v = 0; v < VX; ++v) gt::unpack2(acc2[c][v], acc[2 * c][v], acc[2 * c + 1][v]);
   if (!active) return;
 #pragma unroll
   for (int c = 0; c < CO_T; ++c) {
@@ -628,22 +691,33 @@ __global__ void k_cast_b2f(const __nv_bfloat16 *__restrict__ a, float *__restric
   if (t < n) b[t] = __bfloat162float(a[t]);
 }
 
-template <class TI, class TO, int KS, int CO_T>
+template <class TI, class TO, int KS, int CO_T, int VX>
 cudaError_t conv_t(const void *x, int Ci, int Cx, int x_off, const void *w, const float *bias, void *y, int Co, int Cy,
                    int co_off, Shape s, int relu, int accumulate, cudaStream_t st) {
-  constexpr int VX = 4;
-  if (s.W % VX != 0) return cudaErrorInvalidValue;
   dim3 g(nblk((long long)s.B * s.D * s.H * (s.W / VX), 128), (Co + CO_T - 1) / CO_T);
+  const int vec = reinterpret_cast<size_t>(x) % 16 == 0;  // rows start at multiples of W >= 4 elements
   k_conv3d<TI, TO, KS, CO_T, VX><<<g, 128, 0, st>>>((const TI *)x, Ci, Cx, x_off, (const __nv_bfloat16 *)w, bias,
-                                                     (TO *)y, Co, Cy, co_off, s, relu, accumulate);
+                                                     (TO *)y, Co, Cy, co_off, s, relu, accumulate, vec);
   return cudaGetLastError();
+}
+
+// 8 channels x 8 voxels per thread where that leaves two blocks per SM, else 4 x 4 (the coarse
+// levels: 64 -> 64 channels on 4 x 4 x 16 x 16 voxels are 8 blocks of the larger tile)
+template <class TI, class TO, int KS>
+cudaError_t conv_ks(const void *x, int Ci, int Cx, int x_off, const void *w, const float *bias, void *y, int Co,
+                    int Cy, int co_off, Shape s, int relu, int accumulate, cudaStream_t st) {
+  if (s.W % 4 != 0) return cudaErrorInvalidValue;
+  const long long blocks8 = ((long long)s.B * s.D * s.H * (s.W / 8) + 127) / 128 * ((Co + 7) / 8);
+  if (s.W % 8 == 0 && Co > 4 && blocks8 >= 304)
+    return conv_t<TI, TO, KS, 8, 8>(x, Ci, Cx, x_off, w, bias, y, Co, Cy, co_off, s, relu, accumulate, st);
+  return conv_t<TI, TO, KS, 4, 4>(x, Ci, Cx, x_off, w, bias, y, Co, Cy, co_off, s, relu, accumulate, st);
 }
 
 template <class TI, class TO>
 cudaError_t conv_k(int ks, const void *x, int Ci, int Cx, int x_off, const void *w, const float *bias, void *y, int Co,
                    int Cy, int co_off, Shape s, int relu, int accumulate, cudaStream_t st) {
-  if (ks == 3) return conv_t<TI, TO, 3, 8>(x, Ci, Cx, x_off, w, bias, y, Co, Cy, co_off, s, relu, accumulate, st);
-  if (ks == 1) return conv_t<TI, TO, 1, 8>(x, Ci, Cx, x_off, w, bias, y, Co, Cy, co_off, s, relu, accumulate, st);
+  if (ks == 3) return conv_ks<TI, TO, 3>(x, Ci, Cx, x_off, w, bias, y, Co, Cy, co_off, s, relu, accumulate, st);
+  if (ks == 1) return conv_ks<TI, TO, 1>(x, Ci, Cx, x_off, w, bias, y, Co, Cy, co_off, s, relu, accumulate, st);
   return cudaErrorInvalidValue;
 }
 

@@ -48,3 +48,17 @@ def test_weight_and_bias_gradient_tiles(k, shape, ci, co):
     db = torch.ones(co, device="cuda")
     L.check(L.lib().gt_nn_bias_grad(_p(dyd), co, co + 2, 2, B, D * H * W, _p(db), 1, None))
     assert _rel(db, gb + 1) < 1e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_cuda_core_convolution_large_tile(dtype):
+    L = _lib()
+    B, D, H, W, ci, co = 2, 16, 64, 64, 3, 21  # 384 blocks of 8 channels x 8 voxels; a partial channel tile
+    g = torch.Generator().manual_seed(3)
+    x = torch.randn((B, ci, D, H, W), generator=g).to(dtype)
+    w = (torch.randn((co, ci, 3, 3, 3), generator=g) * 0.2).to(torch.bfloat16)
+    y = torch.zeros((B, co, D, H, W), device="cuda")
+    xd, wd = x.cuda(), w.cuda()
+    L.check(L.lib().gt_nn_conv3d(_p(xd), int(dtype == torch.bfloat16), ci, ci, 0, _p(wd), None, _p(y), 0, co, co, 0, B, D,
+                                 H, W, 3, 0, 0, None))
+    assert _rel(y, F.conv3d(x.double(), w.double(), padding=1)) < 1e-6
