@@ -62,3 +62,39 @@ def test_cuda_core_convolution_large_tile(dtype):
     L.check(L.lib().gt_nn_conv3d(_p(xd), int(dtype == torch.bfloat16), ci, ci, 0, _p(wd), None, _p(y), 0, co, co, 0, B, D,
                                  H, W, 3, 0, 0, None))
     assert _rel(y, F.conv3d(x.double(), w.double(), padding=1)) < 1e-6
+
+
+@pytest.mark.parametrize("W", [2, 4, 6, 8, 12, 16])
+def test_pool_upsample_relu_runs(W):
+    """W: row length of the coarse tensors."""
+    L = _lib()
+    lib = L.lib()
+    B, C, D, H = 2, 3, 2, 3
+    g = torch.Generator().manual_seed(W)
+    fine = torch.randn((B, C + 2, 2 * D, 2 * H, 2 * W), generator=g).to(torch.bfloat16)
+    coarse = torch.randn((B, C, D, H, W), generator=g).to(torch.bfloat16)
+    fd, cd = fine.cuda(), coarse.cuda()
+    out = torch.empty_like(cd)
+    L.check(lib.gt_nn_pool2(_p(fd), C + 2, 1, _p(out), C, B, D, H, W, None))
+    assert _rel(out, F.avg_pool3d(fine[:, 1:1 + C].double(), 2)) < 4e-3  # one bfloat16 rounding
+    up = fd.clone()
+    L.check(lib.gt_nn_up2(_p(cd), _p(up), C, C + 2, 1, B, 2 * D, 2 * H, 2 * W, None))
+    want = fine.clone()
+    want[:, 1:1 + C] = F.interpolate(coarse.float(), scale_factor=2, mode="nearest").to(torch.bfloat16)
+    assert torch.equal(up.cpu(), want)
+    gf = torch.randn((B, C + 2, 2 * D, 2 * H, 2 * W), generator=g)
+    gc = torch.randn((B, C, D, H, W), generator=g)
+    gfd, gcd = gf.cuda(), gc.cuda()
+    dx = torch.empty_like(gcd)
+    L.check(lib.gt_nn_up2_bwd(_p(gfd), C + 2, 1, _p(dx), C, B, D, H, W, None))
+    assert _rel(dx, 8 * F.avg_pool3d(gf[:, 1:1 + C].double(), 2)) < 1e-6
+    acc = gfd.clone()
+    L.check(lib.gt_nn_pool2_bwd(_p(gcd), _p(acc), C, C + 2, 1, B, 2 * D, 2 * H, 2 * W, None))
+    want = gf.double()
+    want[:, 1:1 + C] += 0.125 * F.interpolate(gc.double(), scale_factor=2, mode="nearest")
+    assert _rel(acc, want) < 1e-6
+    acc = gfd.clone()
+    L.check(lib.gt_nn_relu_bwd(_p(acc), _p(fd), 1, C, C + 2, 1, B, 8 * D * H * W, None))
+    want = gf.clone()
+    want[:, 1:1 + C] *= fine[:, 1:1 + C] > 0
+    assert torch.equal(acc.cpu(), want)
