@@ -29,6 +29,8 @@ cudaError_t prepare_bp_tma();
 cudaError_t launch_fwd(const IterParams &P, int disc, cudaStream_t st);
 cudaError_t launch_bp(const IterParams &P, cudaStream_t st);
 cudaError_t launch_update(const IterParams &P, int tgv, cudaStream_t st, int part);
+bool small_ok(const IterParams &P, int cpl);
+cudaError_t launch_small(const IterParams &P, int disc, int tgv, int cpl, cudaStream_t st);
 cudaError_t launch_radon(const float *img, float *sino, const float4 *ofs, int N, int nd, int nang, int S,
                          cudaStream_t st);
 cudaError_t launch_radon_ad(const float *sino, float *img, const float4 *ofs, int N, int nd, int nang, int S,
@@ -302,6 +304,7 @@ struct gt_problem {
   int schedule = 1;            // 1: p / pbar half of the primal update beside the projectors; 0: one update after
                                // them; 2: the p / pbar half fused into the next iteration's dual kernel
   bool schedule_set = false;   // chosen by gt_set_schedule (the autotuner leaves it)
+  bool small = false;          // iterations in two launches (launch_small), chosen by the autotuner
   long long iters = 0;
   bool has_data = false;
   double lsqr = 0;             // > 0: step-size constant of a variant (two-resolution solver: 36)
@@ -322,6 +325,10 @@ namespace {
 // every value by the same operations (bit-identical iterates).
 int enqueue_iteration(gt_problem *p) {
   const int tgv = p->reg == GT_TGV;
+  if (p->small) {
+    CK(gt::launch_small(p->P, p->disc, tgv, p->cpl, p->stream));
+    return GT_OK;
+  }
   CK(cudaEventRecord(p->ev_fork, p->stream));
   CK(cudaStreamWaitEvent(p->side, p->ev_fork, 0));
   CK(gt::launch_fwd(p->P, p->disc, p->side));
@@ -475,7 +482,7 @@ int upload_mu_eff(gt_problem *p) {
 // launches never touch the solve.
 using TuneKey = std::tuple<int, int, int, int, int, int, int, int, int, int>;
 std::mutex g_tune_mu;
-std::map<TuneKey, std::tuple<int, int, int, int>> g_tune;
+std::map<TuneKey, std::tuple<int, int, int, int, bool>> g_tune;
 
 int autotune(gt_problem *p) {
   const bool tgv = p->reg == GT_TGV;
@@ -498,9 +505,10 @@ int autotune(gt_problem *p) {
                (c == 7 && S == 4));
     if (which == 1)
       return !((c == 18 && S >= 96) || (c == 19 && S >= 36) || (c == 9 && S >= 16 && S <= 128) ||
-               (c == 10 && S <= 128) || (c == 11 && S <= 16));
+               (c == 10 && S <= 128) || (c == 11 && S <= 16) || (c == 12 && S == 4));
     return false;
   };
+  p->small = false;
   p->P.fwd_cfg = gt::default_fwd_shape(S);
   p->P.bp_cfg = gt::default_bp_shape(S);
   p->P.dual_cfg = gt::default_dual_shape(p->P, p->cpl);
@@ -511,7 +519,9 @@ int autotune(gt_problem *p) {
     auto it = g_tune.find(key);
     if (it != g_tune.end()) {
       int sched = 0;
-      std::tie(p->P.fwd_cfg, p->P.bp_cfg, p->P.dual_cfg, sched) = it->second;
+      bool small = false;
+      std::tie(p->P.fwd_cfg, p->P.bp_cfg, p->P.dual_cfg, sched, small) = it->second;
+      p->small = small && !p->schedule_set;
       // sched < 0: the schedule was chosen by gt_set_schedule when the shapes were
       // tuned, not timed; 0 is the measured choice at 8M voxel-channels and above
       if (!p->schedule_set) p->schedule = sched >= 0 ? sched : (p->d.vol >= (8u << 20) ? 0 : 1);
@@ -576,21 +586,26 @@ int autotune(gt_problem *p) {
   p->P.fwd_cfg = best[0];
   p->P.bp_cfg = best[1];
   p->P.dual_cfg = best[2];
-  // the schedule (TGV only: TV has no p / pbar half): graph-captured iterations of
-  // each, the faster kept; concurrency between the kernels decides, not their times
-  // alone.  Problems below 8M voxel-channels keep schedule 1 (the two schedules are
-  // within a few per cent there, e.g. 0.135 / 0.132 ms at 128^2 x 32 x 2).
+  // The form of the iteration, from graph-captured iterations of each (16, the second and third
+  // launch timed), the faster kept: concurrency between the kernels decides, not their times
+  // alone.  From 8M voxel-channels on the schedules 0 and 1 (TGV only: TV has no p / pbar half);
+  // below, where the two are within a few per cent (0.135 / 0.132 ms at 128^2 x 32 x 2), schedule
+  // 1 against the two-launch form of gt_small.cu.
   // Schedule 2 (the p half fused into the next dual kernel) is not timed: its
   // fused kernel is slower than the dual kernel and the p half together on every
   // measured workload (256^2 x 60 x 4: 1.07 ms against 0.25 + 0.16 ms), so it
-  // stays a choice of gt_set_schedule.  The graphs are timed over 16 iterations.
-  if (tgv && !p->schedule_set && p->d.vol < (8u << 20)) p->schedule = 1;
-  if (tgv && !p->schedule_set && p->d.vol >= (8u << 20)) {
-    const int nsched = 2;
-    float ms_s[3] = {1e30f, 1e30f, 1e30f};
-    for (int round = 0; round < 2 && rc == GT_OK; ++round) {
-      for (int sched = 0; sched < nsched && rc == GT_OK; ++sched) {
-        p->schedule = sched;
+  // stays a choice of gt_set_schedule.
+  if (!p->schedule_set) {
+    const bool large = p->d.vol >= (8u << 20);
+    float ms_f[2] = {1e30f, 1e30f};  // schedules 0 and 1, or schedule 1 and the two-launch form
+    auto set_form = [&](int f) {
+      p->small = !large && f == 1;
+      if (tgv) p->schedule = large ? f : 1;
+    };
+    const int nform = large ? (tgv ? 2 : 1) : (gt::small_ok(p->P, p->cpl) ? 2 : 1);
+    for (int round = 0; round < 2 && nform > 1 && rc == GT_OK; ++round) {
+      for (int f = 0; f < nform && rc == GT_OK; ++f) {
+        set_form(f);
         cudaGraphExec_t g = nullptr;
         rc = capture(p, 16, &g);
         if (rc) break;
@@ -602,24 +617,21 @@ int autotune(gt_problem *p) {
         float ms = 0.f;
         if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
         cudaGraphExecDestroy(g);
-        if (e != cudaSuccess) { rc = cuda_err(e, "autotune (schedule)", __LINE__); break; }
-        ms_s[sched] = std::min(ms_s[sched], ms / 32);
+        if (e != cudaSuccess) { rc = cuda_err(e, "autotune (iteration)", __LINE__); break; }
+        ms_f[f] = std::min(ms_f[f], ms / 32);
       }
     }
-    int bs = 0;
-    for (int sched = 1; sched < nsched; ++sched)
-      if (ms_s[sched] < ms_s[bs]) bs = sched;
-    p->schedule = bs;
-    if (bs != 2) free_fused(p);
-    if (log && rc == GT_OK)
-      fprintf(stderr, "graptor autotune schedule 0: %.4f ms, 1: %.4f ms, 2: %.4f ms per iteration\n", ms_s[0],
-              ms_s[1], ms_s[2]);
+    set_form(nform > 1 && ms_f[1] < ms_f[0] ? 1 : 0);
+    free_fused(p);
+    if (log && rc == GT_OK && nform > 1)
+      fprintf(stderr, "graptor autotune %s: %.4f ms, %s: %.4f ms per iteration\n", large ? "schedule 0" : "schedule 1",
+              ms_f[0], large ? "schedule 1" : "two launches", ms_f[1]);
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc) return rc;
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  g_tune[key] = std::make_tuple(best[0], best[1], best[2], p->schedule_set ? -1 : p->schedule);
+  g_tune[key] = std::make_tuple(best[0], best[1], best[2], p->schedule_set ? -1 : p->schedule, p->small);
   return GT_OK;
 }
 
@@ -638,6 +650,7 @@ const char *gt_version(void) { return "graptor_gb300 0.1 (sm_103a)"; }
 
 int gt_launches_per_iteration(const gt_problem *p) {
   if (!p) return 0;
+  if (p->small) return 2;
   return 3 + (p->d.C > 8 ? (p->d.C + 7) / 8 : 1) + (p->schedule == 1 && p->reg == GT_TGV ? 1 : 0);
 }
 
@@ -656,6 +669,7 @@ int gt_set_schedule(gt_problem *p, int schedule) {
   }
   p->schedule = schedule;
   p->schedule_set = true;
+  p->small = false;
   if (p->g_one) { cudaGraphExecDestroy(p->g_one); p->g_one = nullptr; }
   if (p->g_chunk) { cudaGraphExecDestroy(p->g_chunk); p->g_chunk = nullptr; }
   return GT_OK;
@@ -773,6 +787,7 @@ int gt_problem_create(const gt_desc *desc, gt_problem **out) {
 
   gt::IterParams &P = p->P;
   P.d = p->d;
+  P.npix = p->d.N * p->d.N;
   P.ofs = p->ofs; P.mu = p->mu_eff;
   {
     int rc = build_rays(P, p->tables, (int *)p->stage, p->stream);  // stage is free scratch now (>= an int per bin)
@@ -1039,6 +1054,7 @@ int gt_set_tuning(gt_problem *p, int fwd_cfg, int bp_cfg) {
     const int rc = build_pairs(p->P, p->tables, (int *)p->stage, p->stream);
     if (rc) return rc;
   }
+  p->small = false;  // the shapes asked for are the ones that run
   p->P.fwd_cfg = fwd_cfg;
   p->P.bp_cfg = bp_cfg;
   // the captured graphs hold the old launch shapes
@@ -1056,6 +1072,7 @@ int gt_set_dual_shape(gt_problem *p, int cfg) {
     return set_err(GT_ERR_ARG, "dual launch shape %d not available here", cfg);
   CK(cudaSetDevice(p->device));
   CK(cudaStreamSynchronize(p->stream));
+  p->small = false;
   p->P.dual_cfg = cfg;
   if (p->g_one) { cudaGraphExecDestroy(p->g_one); p->g_one = nullptr; }
   if (p->g_chunk) { cudaGraphExecDestroy(p->g_chunk); p->g_chunk = nullptr; }
@@ -1869,6 +1886,7 @@ int gt_subs_create(const gt_subs_desc *D, gt_subs **out) {
   auto group = [&](gt::IterParams &Q, ProjTables &t, int C, int ld, int nang, const float4 *ofs, bool inner) -> int {
     Q.d = p->d;
     Q.d.C = C; Q.d.S = ld; Q.d.nd = nd0; Q.d.nang = nang;
+    Q.npix = p->P.npix;
     Q.d.vol = NN * ld; Q.d.nbin = (size_t)nd0 * nang * ld;
     Q.ofs = ofs;
     Q.fwd_cfg = gt::default_fwd_shape(ld);

@@ -41,6 +41,7 @@ struct IterParams {
   float norming;         // 1 / normest     (update_u argument)
   float ainv0, ainv1;    // 1 / (alpha / normest^2)
   float stepsize;
+  int npix;              // pixels of the image (N*N)
   int cbase;             // first channel handled by a k_dual launch (0 unless C > 8)
   int fwd_cfg, bp_cfg;   // projector launch shapes (see launch_fwd / launch_bp)
   int dual_cfg;          // 0: k_dual, 1: k_dual_z2 (where dual_z2_ok)

@@ -23,15 +23,18 @@
 // 64 -> 39 us; 64^2 x 32: 16.4 -> 11.1 us; 177^2 x 16, 45 angles: 33 -> 25 us.
 //
 // k_fwd_staged: one, two or four slices.  A thread per ray would read the ray table
-// uncoalesced (one sector per lane and entry); here the warps of a block read the
-// entries of 32 rays in runs of 32 and gather their pixels into shared memory, and
-// one warp adds each ray's products in order.  128^2 x 1, 60 angles: 51 -> 10.4 us.
+// uncoalesced (one sector per lane and entry) in a bare chain of loads; here the warps of a
+// block read the entries of 32 rays in runs, gather their pixels into shared memory, and
+// one warp adds each ray's products in order.  128^2 x 1, 60 angles: 51 us with a thread per
+// ray, 12 us.  (A warp for itself with two rays has less latency and no barrier, but adds with two
+// lanes: the iterations of several problems side by side got slower.)
 //
 // All kernels add each ray's terms in the reference's order (rows, then x) with the
 // reference's weights (fused multiply-add), so all shapes give identical iterates.
 #include <cuda_runtime.h>
 
 #include "gt_common.cuh"
+#include "gt_flat.cuh"
 #include "gt_geom.cuh"
 #include "gt_vec.cuh"
 
@@ -102,38 +105,6 @@ __global__ void k_pair_fill(const float4 *__restrict__ ofs, int N, int nd, int n
 // ---------------------------------------------------------------------------
 // sums
 // ---------------------------------------------------------------------------
-// one ray from the ray table, UNR entries in flight; the next group's entries are fetched
-// while the current group's pixels are on their way
-template <int VW, int UNR>
-__device__ __forceinline__ void ray_sum(const float *__restrict__ img, size_t S, const int2 *__restrict__ ent, int n,
-                                        int off2, VecAcc<VW> &acc) {
-  int2 nx[UNR];
-#pragma unroll
-  for (int u = 0; u < UNR; ++u) nx[u] = n > 0 ? __ldg(ent + min(u, n - 1)) : make_int2(0, 0);
-  int e = 0;
-  for (; e + UNR <= n; e += UNR) {
-    float w[UNR];
-    Vec<VW> v[UNR];
-#pragma unroll
-    for (int u = 0; u < UNR; ++u) {
-      v[u].load(img + (size_t)nx[u].x * S, off2);
-      w[u] = __int_as_float(nx[u].y);
-    }
-#pragma unroll
-    for (int u = 0; u < UNR; ++u) nx[u] = __ldg(ent + min(e + UNR + u, n - 1));
-#pragma unroll
-    for (int u = 0; u < UNR; ++u) acc.fma(w[u], v[u]);
-  }
-#pragma unroll
-  for (int u = 0; u < UNR - 1; ++u) {  // the rest: its entries are in nx
-    if (e + u < n) {
-      Vec<VW> v;
-      v.load(img + (size_t)nx[u].x * S, off2);
-      acc.fma(__int_as_float(nx[u].y), v);
-    }
-  }
-}
-
 // two rays from the pair table
 template <int VW, int UNR>
 __device__ __forceinline__ void pair_sum(const float *__restrict__ img, size_t S, const int2 *__restrict__ ent, int n,
@@ -167,34 +138,6 @@ __device__ __forceinline__ void pair_sum(const float *__restrict__ img, size_t S
       add(__int_as_float(nx[u].y), v);
     }
   }
-}
-
-// K u and the data dual of bin b (j * nd + i), slices s0 ..; vb: see Vec::store
-template <int DISC, int VW>
-__device__ __forceinline__ void data_step(const IterParams &P, const VecAcc<VW> &acc, long long b, int s0, bool vb) {
-  const Dims d = P.d;
-  const float sd = P.sigma_data;
-  const size_t q = (size_t)b * d.S + s0;
-  float a[VW], lam[VW], f[VW];
-  acc.get(a);
-  Vec<VW>::store(P.ku + q, a, vb);
-  if constexpr (DISC == DATA_NONE) return;
-  Vec<VW>::loadw(P.lam + q, lam, vb);
-  Vec<VW>::loadw(P.f + q, f, vb);
-#pragma unroll
-  for (int k = 0; k < VW; ++k) {
-    const int s = VW == 8 ? s0 + (k < 4 ? k : 124 + k) : s0 + k;
-    const float m = s < d.S ? __ldg(P.mu + s / d.Nz) : 0.f;
-    if (DISC == KL) {
-      const float sv = lam[k] + sd * a[k];
-      const float wv = sv - m;
-      const float dv = wv * wv + 4.f * sd * f[k] * m;
-      lam[k] = sv - 0.5f * (wv + sqrtf(dv));
-    } else {
-      lam[k] = (lam[k] + sd * (a[k] - f[k])) * m;
-    }
-  }
-  Vec<VW>::store(P.lam + q, lam, vb);
 }
 
 // ---------------------------------------------------------------------------
@@ -242,8 +185,8 @@ __global__ void __launch_bounds__(AG *BG * 32, MINB) k_fwd_pair(const IterParams
     }
   }
   if (s0 >= d.S) return;
-  data_step<DISC, VW>(P, acc[0], b0, s0, vb);
-  if (i0 + 1 < d.nd) data_step<DISC, VW>(P, acc[1], b0 + 1, s0, vb);
+  data_step<VW>(P, DISC, acc[0], b0, s0, vb);
+  if (i0 + 1 < d.nd) data_step<VW>(P, DISC, acc[1], b0 + 1, s0, vb);
 }
 
 template <int VW, int UNR, int AG, int BG, int MINB>
@@ -260,17 +203,7 @@ void fwd_pair(const IterParams &P, int disc, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 template <int DISC, int VW, int UNR, int NT>
 __global__ void __launch_bounds__(NT) k_fwd_flat(const IterParams P) {
-  const Dims d = P.d;
-  const int ng = d.S / VW;
-  const long long t = (long long)blockIdx.x * NT + threadIdx.x;
-  if (t >= (long long)ng * d.nd * d.nang) return;
-  const long long b = t / ng;
-  const int s0 = (int)(t - b * ng) * VW;
-  const long long r0 = __ldg(P.ray_start + b);
-  VecAcc<VW> acc;
-  acc.zero();
-  ray_sum<VW, UNR>(P.ubar + s0, d.S, P.ray_ent + r0, (int)(__ldg(P.ray_start + b + 1) - r0), 0, acc);
-  data_step<DISC, VW>(P, acc, b, s0, false);
+  fwd_flat_body<VW, UNR>(P, DISC, (long long)blockIdx.x * NT + threadIdx.x);
 }
 
 template <int VW, int UNR, int NT>
@@ -282,76 +215,20 @@ void fwd_flat(const IterParams &P, int disc, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
-// k_fwd_staged: S = VW slices; a block's 8 warps stage the entries of 32 adjacent rays of an
-// angle, CH at a time and double-buffered, and warp 0 (lane = ray) adds them in order
+// k_fwd_staged: S = VW slices (fwd_staged_body)
 // ---------------------------------------------------------------------------
-template <int DISC, int VW, int CH>
+template <int DISC, int VW>
 __global__ void __launch_bounds__(256) k_fwd_staged(const IterParams P) {
-  __shared__ float sw[2][32][CH + 1];
-  __shared__ Vec<VW> sv[2][32][CH + 1];
-  const Dims d = P.d;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nb = (d.nd + 31) / 32, j = blockIdx.x / nb, i0 = (blockIdx.x - j * nb) * 32;
-  const long long *__restrict__ start = P.ray_start + (size_t)j * d.nd;
-  const int2 *ent[4];
-  int n[4];
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int i = min(i0 + warp * 4 + r, d.nd - 1);
-    const long long r0 = __ldg(start + i);
-    ent[r] = P.ray_ent + r0;
-    n[r] = i0 + warp * 4 + r < d.nd ? (int)(__ldg(start + i + 1) - r0) : 0;
-  }
-  const int il = min(i0 + lane, d.nd - 1);
-  const int mine = i0 + lane < d.nd ? (int)(__ldg(start + il + 1) - __ldg(start + il)) : 0;
-  const int nc = (__reduce_max_sync(0xffffffffu, mine) + CH - 1) / CH;
-  float w[4][CH / 32];
-  Vec<VW> v[4][CH / 32];
-  auto fetch = [&](int c) {
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int k = 0; k < CH / 32; ++k) {
-        const int e = c * CH + k * 32 + lane;
-        if (e < n[r]) {
-          const int2 q = __ldg(ent[r] + e);
-          w[r][k] = __int_as_float(q.y);
-          v[r][k].load(P.ubar + (size_t)q.x * VW, 0);
-        }
-      }
-  };
-  if (nc > 0) fetch(0);
-  VecAcc<VW> acc;
-  acc.zero();
-  // a buffer is written again two chunks later: warp 0 has passed the barrier of the chunk
-  // in between by then, after it read this one
-  for (int c = 0; c < nc; ++c) {
-    const int b = c & 1;
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int k = 0; k < CH / 32; ++k)
-        if (c * CH + k * 32 + lane < n[r]) {
-          sw[b][warp * 4 + r][k * 32 + lane] = w[r][k];
-          sv[b][warp * 4 + r][k * 32 + lane] = v[r][k];
-        }
-    __syncthreads();
-    if (c + 1 < nc) fetch(c + 1);
-    if (warp == 0) {
-      const int m = min(CH, mine - c * CH);
-#pragma unroll 8
-      for (int k = 0; k < m; ++k) acc.fma(sw[b][lane][k], sv[b][lane][k]);
-    }
-  }
-  if (warp == 0 && i0 + lane < d.nd) data_step<DISC, VW>(P, acc, (long long)j * d.nd + i0 + lane, 0, false);
+  __shared__ FwdStage<VW> sh;
+  fwd_staged_body<VW>(P, DISC, blockIdx.x, sh);
 }
 
-template <int VW, int CH>
+template <int VW>
 void fwd_staged(const IterParams &P, int disc, cudaStream_t st) {
-  const unsigned g = (unsigned)P.d.nang * ((P.d.nd + 31) / 32);
-  if (disc == KL) k_fwd_staged<KL, VW, CH><<<g, 256, 0, st>>>(P);
-  else if (disc == L2) k_fwd_staged<L2, VW, CH><<<g, 256, 0, st>>>(P);
-  else k_fwd_staged<DATA_NONE, VW, CH><<<g, 256, 0, st>>>(P);
+  const unsigned g = blocks((long long)P.d.nd * P.d.nang, FS_RAYS);
+  if (disc == KL) k_fwd_staged<KL, VW><<<g, 256, 0, st>>>(P);
+  else if (disc == L2) k_fwd_staged<L2, VW><<<g, 256, 0, st>>>(P);
+  else k_fwd_staged<DATA_NONE, VW><<<g, 256, 0, st>>>(P);
 }
 
 }  // namespace
@@ -387,9 +264,9 @@ cudaError_t launch_fwd_flat(const IterParams &P, int disc, int vw, cudaStream_t 
 
 // k_fwd_staged (S = 1, 2 or 4)
 cudaError_t launch_fwd_staged(const IterParams &P, int disc, cudaStream_t st) {
-  if (P.d.S == 4) fwd_staged<4, 32>(P, disc, st);
-  else if (P.d.S == 2) fwd_staged<2, 32>(P, disc, st);
-  else fwd_staged<1, 64>(P, disc, st);
+  if (P.d.S == 4) fwd_staged<4>(P, disc, st);
+  else if (P.d.S == 2) fwd_staged<2>(P, disc, st);
+  else fwd_staged<1>(P, disc, st);
   return cudaGetLastError();
 }
 

@@ -25,6 +25,10 @@ __device__ __forceinline__ void fma2(f32x2 &acc, f32x2 w, f32x2 v) {
 template <int VW>
 struct Vec {
   f32x2 v[VW / 2];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int k = 0; k < VW / 2; ++k) v[k] = 0ull;
+  }
   __device__ __forceinline__ void load(const float *__restrict__ p, int off2) {
     if constexpr (VW >= 4) {
       const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2 *>(p));
@@ -68,6 +72,7 @@ struct Vec {
 template <>
 struct Vec<1> {
   float v;
+  __device__ __forceinline__ void clear() { v = 0.f; }
   __device__ __forceinline__ void load(const float *__restrict__ p, int) { v = __ldg(p); }
   static __device__ __forceinline__ void loadw(const float *p, float (&r)[1], bool) { r[0] = *p; }
   static __device__ __forceinline__ void store(float *p, const float (&r)[1], bool) { *p = r[0]; }

@@ -109,3 +109,28 @@ def test_operator_norm_matches_fp64_power_iteration(N, nd, deg):
         ne = p.scalars["normest"]
     want = np.sqrt(x.sum())
     assert abs(ne - want) <= 1e-6 * want, (ne, want)
+
+
+@pytest.mark.parametrize("dim,N,nd,Nz,C,reg,cpl,disc", [
+    (2, 33, 33, 1, 1, "TGV", "UNCORR", "KL"), (2, 30, 41, 2, 1, "TV", "FROB", "L2"), (2, 17, 17, 1, 4, "TGV", "FROB", "L2"),
+    (3, 21, 21, 7, 1, "TGV", "FROB", "KL"), (3, 24, 19, 5, 3, "TGV", "UNCORR", "L2"), (3, 26, 26, 8, 4, "TV", "FROB", "KL")])
+def test_two_launch_iteration_equals_separate_launches(dim, N, nd, Nz, C, reg, cpl, disc):
+    """The two-launch form of small problems (whichever form the tuning picks) against schedule
+    0, with the primal weight and the precise primal mode, over runs that end inside and at a graph chunk."""
+    from graptor_gb300.solver import Problem
+    ang = np.deg2rad(np.linspace(-80, 85, 13))
+    f = np.abs(np.random.default_rng(N).standard_normal((C * Nz, ang.size, nd))).astype(np.float32)
+    fields = ("u", "ubar", "v", "lambda", "ku") + (("p", "pbar", "w") if reg == "TGV" else ())
+    got = []
+    for forced in (False, True):
+        with Problem(dim, N, Nz, C, nd, ang, (4, 1), [0.2] * C, disc, reg, cpl, 1.0, 11.0) as p:
+            if forced:
+                p.set_schedule(0)
+            p.set_data(f)
+            p.set_precise_primal()
+            p.run(5).synchronize()
+            p.set_primal_weight(3.0)
+            p.run(37).synchronize()
+            got.append({k: p.get(k) for k in fields + ("ulo",)})
+    for k in got[0]:
+        np.testing.assert_array_equal(got[0][k], got[1][k], err_msg=k)
