@@ -202,7 +202,7 @@ void fwd_pair(const IterParams &P, int disc, cudaStream_t st) {
 // k_fwd_flat: thread = (ray, VW slices)
 // ---------------------------------------------------------------------------
 template <int DISC, int VW, int UNR, int NT>
-__global__ void __launch_bounds__(NT) k_fwd_flat(const IterParams P) {
+__global__ void __launch_bounds__(NT, 1) k_fwd_flat(const IterParams P) {
   fwd_flat_body<VW, UNR>(P, DISC, (long long)blockIdx.x * NT + threadIdx.x);
 }
 
@@ -215,10 +215,61 @@ void fwd_flat(const IterParams &P, int disc, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
+// k_fwd_pair_flat: thread = (pair of bins, 4 slices)
+// ---------------------------------------------------------------------------
+constexpr int PF_G = 4;  // adjacent pairs that stay together; their groups go from the centre outwards
+
+template <int DISC, int UNR>
+__global__ void __launch_bounds__(64, 1) k_fwd_pair_flat(const IterParams P) {
+  const Dims d = P.d;
+  const int ng = d.S / 4, np = (d.nd + 1) / 2, nb = (np + PF_G - 1) / PF_G;
+  const long long t = (long long)blockIdx.x * 64 + threadIdx.x, o = div_pos(t, ng);
+  const int s0 = (int)(t - o * ng) * 4, b = (int)(o / PF_G), k = b / d.nang, j = b - k * d.nang, h = nb / 2;
+  const int bb = (nb & 1) ? ((k & 1) ? h - (k + 1) / 2 : h + k / 2) : ((k & 1) ? h + k / 2 : h - 1 - k / 2);
+  const int q = bb * PF_G + (int)(o % PF_G);
+  if (k >= nb || q >= np) return;
+  const int i0 = 2 * q;
+  const long long b0 = (long long)j * d.nd + i0;
+  const long long e0 = __ldg(P.pair_start + (size_t)j * np + q);
+  const int n = (int)(__ldg(P.pair_start + (size_t)j * np + q + 1) - e0);
+  const float *__restrict__ img = P.ubar + s0;
+  VecAcc<4> acc[2];
+  acc[0].zero();
+  acc[1].zero();
+  bool exact = n == 0;  // see k_fwd_pair
+  if (!exact) {
+    pair_sum<4, UNR>(img, d.S, P.pair_ent + e0, n, (float)i0, 0, acc);
+    exact = !acc[0].finite() || !acc[1].finite();
+  }
+  if (exact) {
+#pragma unroll 1
+    for (int r = 0; r < 2 && i0 + r < d.nd; ++r) {
+      const long long r0 = __ldg(P.ray_start + b0 + r);
+      VecAcc<4> a;
+      a.zero();
+      ray_sum<4, 1>(img, d.S, P.ray_ent + r0, (int)(__ldg(P.ray_start + b0 + r + 1) - r0), 0, a);
+      if (r == 0) acc[0] = a;
+      else acc[1] = a;
+    }
+  }
+  data_step<4>(P, DISC, acc[0], b0, s0, false);
+  if (i0 + 1 < d.nd) data_step<4>(P, DISC, acc[1], b0 + 1, s0, false);
+}
+
+template <int UNR>
+void fwd_pair_flat(const IterParams &P, int disc, cudaStream_t st) {
+  const long long np = (P.d.nd + 1) / 2, pairs = (np + PF_G - 1) / PF_G * PF_G * P.d.nang;
+  const unsigned g = blocks(pairs * (P.d.S / 4), 64);
+  if (disc == KL) k_fwd_pair_flat<KL, UNR><<<g, 64, 0, st>>>(P);
+  else if (disc == L2) k_fwd_pair_flat<L2, UNR><<<g, 64, 0, st>>>(P);
+  else k_fwd_pair_flat<DATA_NONE, UNR><<<g, 64, 0, st>>>(P);
+}
+
+// ---------------------------------------------------------------------------
 // k_fwd_staged: S = VW slices (fwd_staged_body)
 // ---------------------------------------------------------------------------
 template <int DISC, int VW>
-__global__ void __launch_bounds__(256) k_fwd_staged(const IterParams P) {
+__global__ void __launch_bounds__(256, 1) k_fwd_staged(const IterParams P) {
   __shared__ FwdStage<VW> sh;
   fwd_staged_body<VW>(P, DISC, blockIdx.x, sh);
 }
@@ -251,6 +302,12 @@ cudaError_t launch_pair_fill(const float4 *ofs, int N, int nd, int nang, const l
 cudaError_t launch_fwd_pair(const IterParams &P, int disc, int vw, cudaStream_t st) {
   if (vw == 8) fwd_pair<8, 2, 2, 2, 8>(P, disc, st);
   else fwd_pair<4, 8, 1, 4, 6>(P, disc, st);
+  return cudaGetLastError();
+}
+
+// k_fwd_pair_flat (S a multiple of 4)
+cudaError_t launch_fwd_pair_flat(const IterParams &P, int disc, cudaStream_t st) {
+  fwd_pair_flat<8>(P, disc, st);
   return cudaGetLastError();
 }
 

@@ -2234,6 +2234,7 @@ static void fwd_vw(const IterParams &P, int disc, cudaStream_t st) {
 
 cudaError_t launch_fwd_pair(const IterParams &P, int disc, int vw, cudaStream_t st);
 cudaError_t launch_fwd_flat(const IterParams &P, int disc, int vw, cudaStream_t st);
+cudaError_t launch_fwd_pair_flat(const IterParams &P, int disc, cudaStream_t st);
 cudaError_t launch_fwd_staged(const IterParams &P, int disc, cudaStream_t st);
 cudaError_t launch_bp_tap(const IterParams &P, int vw, cudaStream_t st);
 cudaError_t launch_bp_flat(const IterParams &P, int vw, cudaStream_t st);
@@ -2266,7 +2267,9 @@ cudaError_t launch_fwd(const IterParams &P, int disc, cudaStream_t st) {
     case 7:
       if (S == 4) return launch_fwd_staged(P, disc, st);
       return launch_fwd_flat(P, disc, 4, st);
-    case 8: case 9: return launch_fwd_flat(P, disc, 4, st);
+    case 9: return launch_fwd_flat(P, disc, 4, st);
+    case 8:  // without the pair table the flat shape
+      return P.pair_start ? launch_fwd_pair_flat(P, disc, st) : launch_fwd_flat(P, disc, 4, st);
     case 10: case 11:  // without the pair table the ray-table shape
       if (P.pair_start) return launch_fwd_pair(P, disc, P.fwd_cfg == 10 ? 8 : 4, st);
       fwd_vw<8, 4, 4>(P, disc, st);

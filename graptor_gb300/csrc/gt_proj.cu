@@ -217,7 +217,7 @@ void bp_tap(const IterParams &P, cudaStream_t st) {
 }
 
 template <int VW, int UA, int NT>
-__global__ void __launch_bounds__(NT) k_bp_flat(const IterParams P) {
+__global__ void __launch_bounds__(NT, 1) k_bp_flat(const IterParams P) {
   int pix, s0;
   float r[VW];
   if (!bp_flat_body<VW, UA>(P, (long long)blockIdx.x * NT + threadIdx.x, pix, s0, r)) return;
@@ -230,7 +230,7 @@ void bp_flat(const IterParams &P, cudaStream_t st) {
 }
 
 template <int VW>
-__global__ void __launch_bounds__(128) k_bp_staged(const IterParams P) {
+__global__ void __launch_bounds__(128, 1) k_bp_staged(const IterParams P) {
   __shared__ BpStage<VW> sh[4];
   const int warp = threadIdx.x >> 5;
   int pix;
@@ -270,9 +270,9 @@ cudaError_t launch_bp_tap(const IterParams &P, int vw, cudaStream_t st) {
 
 // k_bp_flat with vw slices per thread (4, 2 or 1, a divisor of S)
 cudaError_t launch_bp_flat(const IterParams &P, int vw, cudaStream_t st) {
-  if (vw == 4) bp_flat<4, 8, 64>(P, st);
-  else if (vw == 2) bp_flat<2, 8, 128>(P, st);
-  else bp_flat<1, 8, 128>(P, st);
+  if (vw == 4) bp_flat<4, 4, 64>(P, st);
+  else if (vw == 2) bp_flat<2, 8, 64>(P, st);
+  else bp_flat<1, 8, 64>(P, st);
   return cudaGetLastError();
 }
 
