@@ -5,6 +5,7 @@
 #include <math.h>
 
 #include "gt_common.cuh"
+#include "gt_round.cuh"
 
 namespace gt {
 
@@ -16,12 +17,33 @@ namespace gt {
 // catastrophically when the off-diagonal entry is small, so their results depend
 // on rounding: they are written with explicitly rounded operations (no fused
 // multiply-add), in the reference's order, and with hypot / atan / cos / cube
-// evaluated in double and rounded once (as the host C library's float versions
-// are, to within their last bit).
+// as evaluated in double and rounded once (as the host C library's float versions
+// are, to within their last bit).  gt_round.cuh gives those values without FP64 but for
+// about one call in 10^4, which is left to the functions here.
 __device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fs(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ float hyp(float a, float b) { return (float)sqrt((double)a * a + (double)b * b); }
+static __device__ __noinline__ float hyp_exact(float a, float b) { return (float)sqrt((double)a * a + (double)b * b); }
+static __device__ __noinline__ float cos_exact(float x) { return (float)cos((double)x); }
+static __device__ __noinline__ float atan_exact(float y) { return (float)atan((double)y); }
+static __device__ __noinline__ float cube_exact(float c) { return (float)((double)c * c * c); }
+
+__device__ __forceinline__ float hyp(float a, float b) {
+  float r;
+  return hyp_round(a, b, r) ? r : hyp_exact(a, b);
+}
+__device__ __forceinline__ float cos_f(float x) {
+  float r;
+  return cos_round(x, r) ? r : cos_exact(x);
+}
+__device__ __forceinline__ float atan_f(float y) {
+  float r;
+  return atan_round(y, r) ? r : atan_exact(y);
+}
+__device__ __forceinline__ float cube_f(float c) {
+  float r;
+  return cube_round(c, r) ? r : cube_exact(c);
+}
 
 // nuclear 2-D (update_NormV_Nucl, radon_tgv_primal_dual_2d.py:124-204): spectral
 // projection of the C x 2 matrix A of one pixel via the 2x2 matrix A^T A = [a b; b c].
@@ -82,14 +104,14 @@ __device__ __forceinline__ void eig3d(float a, float b, float c, float d, float 
   const float c0 = fs(fs(fa(fa(fm(fm(a, f), f), fm(fm(b, e), e)), fm(fm(c, d), d)), fm(fm(a, b), c)),
                       fm(fm(fm(2.f, d), e), f));
   float p = (float)((double)fm(c2, c2) - 3.0 * (double)c1);
-  const float cube = (float)((double)c2 * c2 * c2);
+  const float cube = cube_f(c2);
   const float q = fa(fs(fm(-13.5f, c0), cube), fm(fm(4.5f, c2), c1));
   const float inner = fm(27.f, fa(fm(fm(fm(0.25f, c1), c1), fs(p, c1)), fm(c0, fa(q, fm(6.75f, c0)))));
-  float phi = fm(1.f / 3.f, (float)atan((double)(sqrtf(inner) / q)));
+  float phi = fm(1.f / 3.f, atan_f(sqrtf(inner) / q));
   if (q < 0.f) phi = fa(phi, pi / 3.f);
-  const float x1 = fm(2.f, (float)cos((double)phi));
-  const float x2 = fm(2.f, (float)cos((double)fa(phi, fm(2.f, pi) / 3.f)));
-  const float x3 = fm(2.f, (float)cos((double)fs(phi, fm(2.f, pi) / 3.f)));
+  const float x1 = fm(2.f, cos_f(phi));
+  const float x2 = fm(2.f, cos_f(fa(phi, fm(2.f, pi) / 3.f)));
+  const float x3 = fm(2.f, cos_f(fs(phi, fm(2.f, pi) / 3.f)));
   p = sqrtf(p) / 3.f;
   c2 = c2 / 3.f;
   out[0] = fs(fm(p, x1), c2); out[1] = fs(fm(p, x2), c2); out[2] = fs(fm(p, x3), c2);
