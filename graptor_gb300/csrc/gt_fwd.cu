@@ -105,9 +105,11 @@ __global__ void k_pair_fill(const float4 *__restrict__ ofs, int N, int nd, int n
 // ---------------------------------------------------------------------------
 // sums
 // ---------------------------------------------------------------------------
-// two rays from the pair table
+// two rays from the pair table; false where a product of a zero weight and an infinity or NaN may
+// have reached the wrong ray (looked at after the first group too: once an iterate is NaN
+// everywhere, as the nuclear projection's can be, the sums from the ray table follow at once)
 template <int VW, int UNR>
-__device__ __forceinline__ void pair_sum(const float *__restrict__ img, size_t S, const int2 *__restrict__ ent, int n,
+__device__ __forceinline__ bool pair_sum(const float *__restrict__ img, size_t S, const int2 *__restrict__ ent, int n,
                                          float fi0, int off2, VecAcc<VW> (&acc)[2]) {
   auto add = [&](float t, const Vec<VW> &v) {
     acc[0].fma(fmaxf(0.f, 1.0f - fabsf(__fsub_rn(t, fi0))), v);
@@ -129,6 +131,7 @@ __device__ __forceinline__ void pair_sum(const float *__restrict__ img, size_t S
     for (int u = 0; u < UNR; ++u) nx[u] = __ldg(ent + min(e + UNR + u, n - 1));
 #pragma unroll
     for (int u = 0; u < UNR; ++u) add(t[u], v[u]);
+    if (e == 0 && !(acc[0].finite() && acc[1].finite())) return false;
   }
 #pragma unroll
   for (int u = 0; u < UNR - 1; ++u) {
@@ -138,6 +141,7 @@ __device__ __forceinline__ void pair_sum(const float *__restrict__ img, size_t S
       add(__int_as_float(nx[u].y), v);
     }
   }
+  return acc[0].finite() && acc[1].finite();
 }
 
 // ---------------------------------------------------------------------------
@@ -169,9 +173,7 @@ __global__ void __launch_bounds__(AG *BG * 32, MINB) k_fwd_pair(const IterParams
   acc[1].zero();
   bool exact = n == 0;  // no list: from the ray table (no entries there either for rays off the image)
   if (!exact) {
-    pair_sum<VW, UNR>(img, S, P.pair_ent + e0, n, (float)i0, off2, acc);
-    // a product of a zero weight and an infinity or NaN must not reach the other ray
-    exact = !acc[0].finite() || !acc[1].finite();
+    exact = !pair_sum<VW, UNR>(img, S, P.pair_ent + e0, n, (float)i0, off2, acc);
   }
   if (exact) {
 #pragma unroll 1
@@ -179,7 +181,7 @@ __global__ void __launch_bounds__(AG *BG * 32, MINB) k_fwd_pair(const IterParams
       const long long r0 = __ldg(P.ray_start + b0 + r);
       VecAcc<VW> a;
       a.zero();
-      ray_sum<VW, 1>(img, S, P.ray_ent + r0, (int)(__ldg(P.ray_start + b0 + r + 1) - r0), off2, a);
+      ray_sum<VW, VW == 8 ? 1 : 4>(img, S, P.ray_ent + r0, (int)(__ldg(P.ray_start + b0 + r + 1) - r0), off2, a);
       if (r == 0) acc[0] = a;
       else acc[1] = a;
     }
@@ -238,8 +240,7 @@ __global__ void __launch_bounds__(64, 1) k_fwd_pair_flat(const IterParams P) {
   acc[1].zero();
   bool exact = n == 0;  // see k_fwd_pair
   if (!exact) {
-    pair_sum<4, UNR>(img, d.S, P.pair_ent + e0, n, (float)i0, 0, acc);
-    exact = !acc[0].finite() || !acc[1].finite();
+    exact = !pair_sum<4, UNR>(img, d.S, P.pair_ent + e0, n, (float)i0, 0, acc);
   }
   if (exact) {
 #pragma unroll 1
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(64, 1) k_fwd_pair_flat(const IterParams P) {
       const long long r0 = __ldg(P.ray_start + b0 + r);
       VecAcc<4> a;
       a.zero();
-      ray_sum<4, 1>(img, d.S, P.ray_ent + r0, (int)(__ldg(P.ray_start + b0 + r + 1) - r0), 0, a);
+      ray_sum<4, 8>(img, d.S, P.ray_ent + r0, (int)(__ldg(P.ray_start + b0 + r + 1) - r0), 0, a);
       if (r == 0) acc[0] = a;
       else acc[1] = a;
     }
