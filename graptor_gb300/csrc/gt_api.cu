@@ -232,7 +232,7 @@ int build_rays(gt::IterParams &P, ProjTables &t, int *scratch, cudaStream_t st) 
   return GT_OK;
 }
 
-// optional (forward shapes 10 and 11): without room for it those shapes use the ray table
+// optional (forward shapes 8, 10 and 11): without room for it those shapes use the ray table
 int build_pairs(gt::IterParams &P, ProjTables &t, int *scratch, cudaStream_t st) {
   if (t.pairs || !P.ray_start) return GT_OK;
   const gt::Dims &d = P.d;
@@ -494,9 +494,9 @@ int autotune(gt_problem *p) {
                      std::min(kMaxCfg, gt::num_dual_configs(p->P))};
   // Shapes left out of the tuning (all stay selectable by gt_set_tuning), to bound
   // its time on batches of many distinct problems: of the back projection all but the
-  // row-tile shapes (18, 19, 9) and the flat ones (10, 11), each in the range of slice
+  // row-tile shapes (18, 19, 9) and the flat ones (10, 11, 12), each in the range of slice
   // counts where it can win (times at default_bp_shape; the one-pixel and TMA shapes
-  // never do); of the forward projection all but the pair shapes (10, 11), the flat ones
+  // never do); of the forward projection all but the pair shapes (10, 11, 8), the flat ones
   // (9, 5) and the staged one (7), likewise (times at default_fwd_shape).
   const int S = p->d.S;
   auto skipped = [&](int which, int c) {
@@ -590,7 +590,7 @@ int autotune(gt_problem *p) {
   // launch timed), the faster kept: concurrency between the kernels decides, not their times
   // alone.  From 8M voxel-channels on the schedules 0 and 1 (TGV only: TV has no p / pbar half);
   // below, where the two are within a few per cent (0.135 / 0.132 ms at 128^2 x 32 x 2), schedule
-  // 1 against the two-launch form of gt_small.cu.
+  // 1, and with 1, 2 or 4 slices the two-launch form of gt_small.cu against it.
   // Schedule 2 (the p half fused into the next dual kernel) is not timed: its
   // fused kernel is slower than the dual kernel and the p half together on every
   // measured workload (256^2 x 60 x 4: 1.07 ms against 0.25 + 0.16 ms), so it

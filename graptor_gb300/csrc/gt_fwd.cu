@@ -18,9 +18,15 @@
 // Three and four bins per warp load fewer pixels still but took 399 and 530 us: their
 // zero-weight products and registers cost more than the loads saved.
 //
+// k_fwd_pair_flat: a thread owns a pair of bins and 4 slices, threads of a warp run on over
+// pairs: 56 to 128 slices do not fill the lanes of a warp per pair.  128^2, 71 angles, 64 slices:
+// 33 us (k_fwd_flat 38, k_fwd_pair 58); 92 slices: 53 us (61, 61).  With one thread in two fewer
+// than k_fwd_flat it loses below that: 48 slices 34.8 against 37 us, 32 (64^2) 14.4 against 10.4.
+//
 // k_fwd_flat: a thread owns one ray and VW slices, threads of a warp run on over rays;
-// with few slices a warp holds several rays and no lane idles.  128^2 x 64, 71 angles:
-// 64 -> 39 us; 64^2 x 32: 16.4 -> 11.1 us; 177^2 x 16, 45 angles: 33 -> 25 us.
+// with few slices a warp holds several rays and no lane idles.  Bound by the latency of its
+// loads, 12 in flight.  64^2 x 32, 71 angles: 10.4 us (16.4 with a warp per ray); 177^2 x 16, 45
+// angles: 24.4 us (33); 101^2 x 40, 33 angles: 15.3 us.
 //
 // k_fwd_staged: one, two or four slices.  A thread per ray would read the ray table
 // uncoalesced (one sector per lane and entry) in a bare chain of loads; here the warps of a

@@ -2241,11 +2241,11 @@ cudaError_t launch_bp_flat(const IterParams &P, int vw, cudaStream_t st);
 cudaError_t launch_bp_staged(const IterParams &P, cudaStream_t st);
 
 // default forward shape (no autotuning).  us of k_fwd_pair with 8 / 4 slices per lane, of
-// k_fwd_flat with 4 slices per thread and of the ray-table kernel (the best of 0..4, 14):
-// 16 slices (177^2, 45 angles) - / 73 / 25 / 33; 32 (64^2, 71) - / 21 / 11 / 16; 40 (101^2, 45)
-// - / 29 / 18 / 25; 64 (128^2, 71) - / 61 / 38 / 64; 92 (128^2, 71) - / 61 / 62 / 68; 240 (256^2,
-// 71) 333 / 395 / 417 / 386; 384 (512^2, 141) 5044 / 4404 / 8130 / 7795 (there 8 per lane
-// leave a quarter of the lanes idle).
+// k_fwd_pair_flat, of k_fwd_flat with 4 slices per thread and of the ray-table kernel (the best of
+// 0..4, 14): 16 slices (177^2, 45 angles) - / 70 / 34 / 24 / 33; 32 (64^2, 71) - / 20 / 14 / 10 / 16;
+// 64 (128^2, 71) - / 58 / 33 / 38 / 64; 92 (128^2, 71) 83 / 61 / 53 / 61 / 68; 240 (256^2, 71) 333 / 360
+// / 359 / 426 / 386; 384 (512^2, 141) 5044 / 4404 / - / 8130 / 7795 (there 8 per lane leave a quarter
+// of the lanes idle).
 int default_fwd_shape(int S) {
   if (S == 4) return 7;
   if (S <= 92) return 9;
@@ -2287,14 +2287,14 @@ static void bp_vw(const IterParams &P, cudaStream_t st) {
 
 // default back-projection shape (no autotuning).  256^2 and smaller, us of k_bp_tap with
 // 8 / 4 / 2 slices per lane and k_bp_flat with 4 slices per thread: 16 slices (177^2, 45
-// angles) 73 / 45 / 41 / 18; 32 (64^2, 71) 39 / 33 / 31 / 14; 40 (101^2, 45) 33 / 25 / 25 / 17;
-// 64 (128^2, 71) 74 / 41 / 36 / 45; 92 (128^2, 71) 74 / 43 / 62 / 62; 240 (256^2, 71)
-// 213 / 242 / 362 / 558; 384 (512^2, 141) 2912 / 2628 / 4050 / 6856 (there 8 per lane leave
+// angles) 73 / 45 / 41 / 14; 32 (64^2, 71) 39 / 33 / 31 / 12; 40 (101^2, 33) - / 19 / 19 / 10;
+// 64 (128^2, 71) 74 / 42 / 36 / 35; 92 (128^2, 71) 74 / 43 / 62 / 50; 240 (256^2, 71)
+// 213 / 242 / 361 / 440; 384 (512^2, 141) 2912 / 2628 / 4050 / 6856 (there 8 per lane leave
 // a quarter of the lanes idle).
 int default_bp_shape(int S) {
   if (S == 4) return 12;
   if (S <= 48) return 10;
-  if (S <= 64) return 9;
+  if (S <= 64) return 9;  // alone as k_bp_flat, beside other work faster (three at once: 22 us each against 28)
   const int w8 = (S + 255) / 256 * 256, w4 = (S + 127) / 128 * 128;
   return S >= 192 && w8 <= w4 + w4 / 8 ? 18 : 19;
 }

@@ -32,8 +32,8 @@ namespace {
 // Bound by the multiply-adds and the weights' broadcasts from shared memory (128 bytes a clock
 // and SM), so a weight serves VX voxels and the output channels go in pairs through packed
 // multiply-adds (fma.rn.f32x2, each half rounding as a scalar one; the order of every sum
-// is input channel, then tap).  16 -> 16 channels on 4 x 16 x 64 x 64 voxels, float32: 142 us with
-// 8 channels x 4 voxels and scalar multiply-adds.
+// is input channel, then tap).  16 -> 16 channels on 4 x 16 x 64 x 64 voxels, float32: 116 us; 142 us
+// with 8 channels x 4 voxels and scalar multiply-adds.
 // ---------------------------------------------------------------------------
 constexpr int CI_CH = 8;
 

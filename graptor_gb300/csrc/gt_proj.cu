@@ -23,8 +23,8 @@
 // k_bp_flat: a thread owns one pixel and VW slices, threads of a warp run on over pixels.
 // With few slices per pixel a warp per tile leaves lanes idle; here a warp holds
 // several pixels and the geometry is computed on the fly, UA angles at a time so that
-// 2 UA loads are in flight.  64^2, 71 angles, 32 slices: 14.4 us against 26.7 us with
-// one slice per thread; 177^2, 45 angles, 16 slices: 18.5 against 37 us.
+// 2 UA loads are in flight.  64^2, 71 angles, 32 slices: 12.3 us (26.7 with one slice per thread,
+// 25.9 with the loads one after another); 177^2, 45 angles, 16 slices: 14.4 us (37, 20.5).
 //
 // k_bp_staged: one, two or four slices; a warp computes the geometry and loads the taps of
 // 8 pixels and 32 angles at once into shared memory, 8 lanes add them in order (a thread per

@@ -5,8 +5,10 @@
 // the FP32 rate: that took most of its dual update.  Here
 // a value is computed as an unevaluated sum h + l of two floats with a relative error below
 // 2^-38 (bounds at each function), and accepted where every real number that close to h + l
-// rounds to h (Ziv's test).  Otherwise, about once in 2^12 calls, the function returns false
-// and the caller evaluates in double; so results are the same in all bits.
+// rounds to h (Ziv's test).  Otherwise, about once in 10^4 calls, the function returns false
+// and the caller evaluates in double; so results are the same in all bits.  NaN goes through
+// as NaN.  Dual update of 128^2 x 30 x 3: 64 -> 54 us after 100 iterations, 120 -> 58 us once
+// the iterate is NaN, as the reference's projection can make it.
 //
 // Sums and products of such pairs: T. J. Dekker, "A floating-point technique for extending the
 // available precision", Numer. Math. 18 (1971); the series are Taylor's.  Built with
