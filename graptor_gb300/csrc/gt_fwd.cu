@@ -19,9 +19,10 @@
 // zero-weight products and registers cost more than the loads saved.
 //
 // k_fwd_pair_flat: a thread owns a pair of bins and 4 slices, threads of a warp run on over
-// pairs: 56 to 128 slices do not fill the lanes of a warp per pair.  128^2, 71 angles, 64 slices:
-// 33 us (k_fwd_flat 38, k_fwd_pair 58); 92 slices: 53 us (61, 61).  With one thread in two fewer
-// than k_fwd_flat it loses below that: 48 slices 34.8 against 37 us, 32 (64^2) 14.4 against 10.4.
+// pairs: 80 to 128 slices do not fill the lanes of a warp per pair.  128^2, 71 angles, 92 slices:
+// 53 us (k_fwd_flat 61, k_fwd_pair 61).  With half the threads of k_fwd_flat it gains nothing
+// below that: 64 slices 33 us with the image in L2 but 48 us with cold caches (38, 45), 32 (64^2)
+// 14.4 us (10.4).
 //
 // k_fwd_flat: a thread owns one ray and VW slices, threads of a warp run on over rays;
 // with few slices a warp holds several rays and no lane idles.  Bound by the latency of its
