@@ -114,16 +114,18 @@ __global__ void __launch_bounds__(256, 2) k_wgrad3(const float *__restrict__ dy,
     }
     __syncthreads();
     const float *rows[3] = {&T.x[(d + 2) % 3][0][0][ci], &T.x[d % 3][0][0][ci], &T.x[(d + 1) % 3][0][0][ci]};
+    // Only the tile's voxels inside the volume: the others' dY is 0, but 0 times an infinite X
+    // would be NaN.
+    const int hv = min(HR, s.H - h0), wv = min(WB, s.W - w0);
 #pragma unroll 1
-    for (int hr = group * (HR / 2); hr < (group + 1) * (HR / 2); ++hr) {
+    for (int hr = group * (HR / 2); hr < min((group + 1) * (HR / 2), hv); ++hr) {
       float win[9][3];  // X at (kd, kh) and three neighbours along the row
 #pragma unroll
       for (int k = 0; k < 9; ++k) {
         win[k][1] = rows[k / 3][(hr + k % 3) * XR];
         win[k][2] = rows[k / 3][(hr + k % 3) * XR + XS];
       }
-#pragma unroll
-      for (int ww = 0; ww < WB; ++ww) {
+      auto voxel = [&](int ww) {
         const float2 g = *reinterpret_cast<const float2 *>(&T.dy[hr][ww][2 * cp]);
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
@@ -136,6 +138,13 @@ __global__ void __launch_bounds__(256, 2) k_wgrad3(const float *__restrict__ dy,
             acc[1][3 * k + q] = fmaf(g.y, win[k][q], acc[1][3 * k + q]);
           }
         }
+      };
+      if (wv == WB) {
+#pragma unroll
+        for (int ww = 0; ww < WB; ++ww) voxel(ww);
+      } else {
+#pragma unroll 1
+        for (int ww = 0; ww < wv; ++ww) voxel(ww);
       }
     }
   }

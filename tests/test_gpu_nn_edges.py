@@ -1,0 +1,54 @@
+"""Weight gradients where rows and columns of a volume end inside a tile: what is not finite
+reaches the taps that use it and no others."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _p(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+def _wgrad(x, dy):
+    """dW[co][ci][kd][kh][kw] in float64, each tap over the voxels whose neighbour is inside."""
+    D, H, W = x.shape[2:]
+    out = np.zeros((dy.shape[1], x.shape[1], 3, 3, 3))
+    for t in np.ndindex(3, 3, 3):
+        a = [slice(max(0, 1 - k), min(n, n + 1 - k)) for k, n in zip(t, (D, H, W))]  # voxels of dY
+        b = [slice(s.start + k - 1, s.stop + k - 1) for s, k in zip(a, t)]           # their neighbours
+        with np.errstate(invalid="ignore"):
+            out[(slice(None), slice(None)) + t] = np.einsum("bodhw,bidhw->oi", dy[(slice(None), slice(None), *a)],
+                                                            x[(slice(None), slice(None), *b)])
+    return out
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [(1, 2, 9, 20), (1, 3, 6, 72), (2, 1, 5, 8), (1, 2, 8, 32)])
+def test_infinite_activation_reaches_its_own_taps_only(shape, dtype):
+    """Tiles of 8 x 16 and 4 x 32 voxels, ragged in rows, in columns, in both and in neither; infinite
+    activations on the last row and column, dY positive (so that no tap sees infinity minus infinity)."""
+    from graptor_gb300 import _lib as L
+    B, D, H, W = shape
+    ci, co = 3, 2
+    g = torch.Generator().manual_seed(W)
+    x = torch.randn((B, ci, D, H, W), generator=g).to(dtype)
+    x[0, 0, 0, H - 1, W - 1] = float("inf")
+    x[0, 1, D - 1, H - 1, W // 2] = float("inf")
+    x[0, 2, 0, H // 2, W - 1] = float("inf")
+    dy = torch.rand((B, co, D, H, W), generator=g) + 0.1
+    want = _wgrad(x.double().numpy(), dy.double().numpy())
+    assert np.isinf(want).any() and np.isfinite(want).any()
+    xd, dyd = x.cuda(), dy.cuda()
+    part, out = torch.empty(co * ci * 27, device="cuda"), torch.empty((co, ci, 3, 3, 3), device="cuda")
+    L.check(L.lib().gt_nn_conv3d_wgrad(_p(dyd), co, co, 0, _p(xd), int(dtype == torch.bfloat16), ci, ci, 0, B, D, H, W, 3,
+                                       B * D * H * W, _p(part), _p(out), 0, None))
+    got = out.double().cpu().numpy()
+    fin = np.isfinite(want)
+    np.testing.assert_array_equal(np.isfinite(got), fin)
+    np.testing.assert_array_equal(got[~fin], want[~fin])
+    # float32 sums of n <= 1296 products of |x| dY: n 2^-24 times the sum of magnitudes, some 900
+    assert np.abs(got[fin] - want[fin]).max() <= 0.07
