@@ -324,6 +324,8 @@ int gt_nn_conv3d_wgrad(const float *dy, int Co, int Cdy, int dy_off, const void 
   if (!dy || !x || !part || !g || kchunk < 1 || dy_off < 0 || dy_off + Co > Cdy || x_off < 0 || x_off + Ci > Cx)
     return gt::set_error(GT_ERR_ARG, "gt_nn_conv3d_wgrad: bad argument");
   const long long nvox = (long long)B * D * H * W;
+  if (B < 1 || D < 1 || H < 1 || W < 1 || Co < 1 || Ci < 1)
+    return gt::set_error(GT_ERR_ARG, "gt_nn_conv3d_wgrad: empty batch, volume or channel range");
   const long long nchunk = (nvox + kchunk - 1) / kchunk;
   if (nchunk > 65535) return gt::set_error(GT_ERR_ARG, "gt_nn_conv3d_wgrad: kchunk too small (more than 65535 chunks)");
   if ((ksize != 1 && ksize != 3) || (x_dtype != 0 && x_dtype != 1))
