@@ -47,8 +47,7 @@ __global__ void __launch_bounds__(256, 2) k_wgrad3(const float *__restrict__ dy,
   const int ci0 = blockIdx.x * WG_C, co0 = blockIdx.y * WG_C;
   const int group = threadIdx.x >> 7, ci = threadIdx.x & 15, cp = (threadIdx.x >> 4) & 7;
   const int nw = (s.W + WB - 1) / WB, nh = (s.H + HR - 1) / HR;
-  const int plane = s.H * s.W;
-  const long long vol = (long long)plane * s.D;
+  const long long vol = (long long)s.H * s.W * s.D;
   float acc[2][27];
 #pragma unroll
   for (int t = 0; t < 27; ++t) acc[0][t] = acc[1][t] = 0.f;
@@ -64,7 +63,7 @@ __global__ void __launch_bounds__(256, 2) k_wgrad3(const float *__restrict__ dy,
     constexpr int STEP = 256 / WB;
     float gq[WG_V * WG_C / 256];
     {
-      const float *p = dy + ((long long)b * Cdy + dy_off + co0) * vol + (long long)d * plane + h0 * s.W + w0 + lw;
+      const float *p = dy + ((long long)b * Cdy + dy_off + co0) * vol + ((long long)d * s.H + h0) * s.W + w0 + lw;
 #pragma unroll
       for (int k = 0; k < WG_V * WG_C / 256; ++k) {
         const int q = lq + k * STEP, c = q / HR, hr = q % HR;
@@ -81,7 +80,7 @@ __global__ void __launch_bounds__(256, 2) k_wgrad3(const float *__restrict__ dy,
     for (int zd = (t == t0 || d == 0) ? d - 1 : d + 1; zd <= d + 1; ++zd) {
       float(*X)[WB + 2][XS] = T.x[(zd + 3) % 3];
       const bool in_d = zd >= 0 && zd < s.D;
-      const TX *p = x + ((long long)b * Cx + x_off + ci0) * vol + (long long)zd * plane + (h0 - 1) * s.W + w0;
+      const TX *p = x + ((long long)b * Cx + x_off + ci0) * vol + ((long long)zd * s.H + h0 - 1) * s.W + w0;
       constexpr int ROWS = (HR + 2) * WG_C, NK = ROWS / STEP;
       static_assert(ROWS % STEP == 0 && 2 * ROWS <= 2 * 256, "staging");
       float v[NK], e[2];

@@ -52,3 +52,25 @@ def test_infinite_activation_reaches_its_own_taps_only(shape, dtype):
     np.testing.assert_array_equal(got[~fin], want[~fin])
     # float32 sums of n <= 1296 products of |x| dY: n 2^-24 times the sum of magnitudes, some 900
     assert np.abs(got[fin] - want[fin]).max() <= 0.07
+
+
+@pytest.mark.parametrize("W", [32, 16])
+def test_plane_of_more_than_2_31_voxels(W):
+    """Voxel offsets inside a plane do not fit 32 bits: a pair of voxels and their products at both ends."""
+    from graptor_gb300 import _lib as L
+    H = (1 << 31) // W + 9
+    x = torch.zeros((H, W), dtype=torch.bfloat16, device="cuda")
+    dy = torch.zeros((H, W), device="cuda")
+    x[0, 1], x[H - 2, 3], x[H - 1, W - 1] = 2.0, 3.0, 5.0
+    dy[1, 2], dy[H - 1, 2], dy[H - 1, W - 1] = 0.5, 0.25, 4.0
+    want = torch.zeros((3, 3))
+    # dW[kh][kw] = sum of dY[h][w] X[h + kh - 1][w + kw - 1]
+    want[0, 0] += 0.5 * 2.0
+    want[0, 2] += 0.25 * 3.0
+    want[1, 1] += 4.0 * 5.0
+    kchunk = -(-H * W // 608)
+    part, out = torch.empty(608 * 27, device="cuda"), torch.empty((3, 3, 3), device="cuda")
+    L.check(L.lib().gt_nn_conv3d_wgrad(_p(dy), 1, 1, 0, _p(x), 1, 1, 1, 0, 1, 1, H, W, 3, kchunk, _p(part), _p(out), 0,
+                                       None))
+    got = out.cpu()
+    assert torch.equal(got[1], want) and not got[0].any() and not got[2].any()
