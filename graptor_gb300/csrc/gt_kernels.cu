@@ -23,6 +23,7 @@
 
 #include "gt_common.cuh"
 #include "gt_dual.cuh"
+#include "gt_fix.cuh"
 #include "gt_geom.cuh"
 #include "gt_tma.cuh"
 #include "gt_update.cuh"
@@ -1675,16 +1676,11 @@ __global__ void k_fill(T *__restrict__ x, size_t n, T v) {
 // ===========================================================================
 // FP64 operator-norm power iteration (radon_normest, 3-D :1018-1030), one slice
 // ===========================================================================
-// Geometry in fixed point, FIX = 44 fraction bits: FP64 arithmetic runs at a sixty-fourth of the
-// FP32 rate here, and computed in FP64 the detector coordinate, its floor, fraction and
-// weights were nearly all of the projectors' time (128^2, 71 angles: 0.45 ms per round).
-// The coordinate t = x X + y Y + off is a sum of 64-bit integers (|t| < 2^18, rounding of
-// X, Y and off 3e-14 each, as that of an FP64 t of a few hundred), its bin a shift and its
-// fraction a mantissa; only the sums stay FP64 operations.  Wider geometries take FIX = 30
-// (|t| < 2^32; an FP64 t beyond 2^18 has no more than 35 fraction bits itself).
-template <int FIX>
-__device__ __forceinline__ long long to_fix(double v) { return __double2ll_rn(v * (double)(1ll << FIX)); }
-
+// Geometry in fixed point (gt_fix.cuh): FP64 arithmetic runs at a sixty-fourth of the FP32 rate
+// here, and computed in FP64 the detector coordinate, its floor, fraction and weights were
+// nearly all of the projectors' time (128^2, 71 angles: 0.45 ms per round).  The coordinate's
+// bin is a shift and its fraction a mantissa; only the sums stay FP64 operations.  FIX = 0:
+// FP64 geometry, for coordinates of 2^18 and more.
 // f 2^-FIX for 0 <= f <= 2^FIX, exactly
 template <int FIX>
 __device__ __forceinline__ double from_fix(long long f) {
@@ -1705,9 +1701,13 @@ __global__ void k_radon64_warp(const double *__restrict__ img, double *__restric
   if (ray >= (long long)nd * nang) return;  // whole warps leave together
   const int j = (int)(ray / nd), i = (int)(ray - (long long)j * nd);
   const dvec4 o = ofs[j];
-  const long long X = to_fix<FIX>(o.x), Y = to_fix<FIX>(o.y), off = to_fix<FIX>(o.z) - (long long)i * FIX_ONE;
+  FixAngle a{};
+  if constexpr (FIX > 0) {
+    a = fix_angle<FIX>(o.x, o.y, o.z);
+    a.off.hi -= i * FIX_ONE;  // t - i
+  }
   double acc = 0.0;
-  for (int y = lane; y < N; y += 32) {
+  for (int y = isfinite(o.x + o.y + o.z) ? lane : N; y < N; y += 32) {  // an angle of NaN takes no pixel
     const double dd = y * o.y + o.z;
     int xl, xh;
     if (o.x == 0.0) {
@@ -1718,11 +1718,18 @@ __global__ void k_radon64_warp(const double *__restrict__ img, double *__restric
       xl = (int)((i + 1 - dd) * o.w); xh = (int)((i - 1 - dd) * o.w);
     }
     xl = max(xl - 1, 0); xh = min(xh + 1, N - 1);
-    long long c = xl * X + y * Y + off;  // t - i
     const double *__restrict__ row = img + (size_t)y * N;
-    for (int x = xl; x <= xh; ++x, c += X) {
-      const long long wgt = FIX_ONE - (c < 0 ? -c : c);
-      if (wgt > 0) acc = __fma_rn(from_fix<FIX>(wgt), row[x], acc);
+    if constexpr (FIX > 0) {
+      FixNum c = fix_at(a, xl, y);
+      for (int x = xl; x <= xh; ++x, fix_step(c, a.X)) {
+        const long long wgt = FIX_ONE - (c.hi < 0 ? -c.hi : c.hi);
+        if (wgt > 0) acc = __fma_rn(from_fix<FIX>(wgt), row[x], acc);
+      }
+    } else {
+      for (int x = xl; x <= xh; ++x) {
+        const double wgt = 1.0 - fabs(x * o.x + dd - i);
+        if (wgt > 0.0) acc = __fma_rn(wgt, row[x], acc);
+      }
     }
   }
 #pragma unroll
@@ -1736,31 +1743,40 @@ __global__ void __launch_bounds__(128) k_radon_ad64(const double *__restrict__ s
                                                     const dvec4 *__restrict__ ofs, int N, int nd, int nang) {
   constexpr long long FIX_ONE = 1ll << FIX;
   constexpr int ANG = 128;
-  __shared__ long long sx[ANG], sy[ANG], so[ANG];
+  __shared__ FixAngle sa[FIX > 0 ? ANG : 1];
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = t / N, x = t - y * N;
-  const long long end = (long long)nd * FIX_ONE;
   double acc = 0.0;
-  for (int j0 = 0; j0 < nang; j0 += ANG) {
-    __syncthreads();
-    for (int k = threadIdx.x; k < min(ANG, nang - j0); k += blockDim.x) {
-      const dvec4 o = ofs[j0 + k];
-      sx[k] = to_fix<FIX>(o.x);
-      sy[k] = to_fix<FIX>(o.y);
-      so[k] = to_fix<FIX>(o.z);
-    }
-    __syncthreads();
-    if (t >= N * N) continue;
-    const int m = min(ANG, nang - j0);
+  auto taps = [&](int j, int il, double p) {
+    const double *__restrict__ row = sino + (size_t)j * nd;
+    if (il >= 0) acc = __fma_rn(1.0 - p, row[il], acc);
+    if (il <= nd - 2) acc = __fma_rn(p, row[il + 1], acc);
+  };
+  if constexpr (FIX > 0) {
+    const long long end = (long long)nd * FIX_ONE;
+    for (int j0 = 0; j0 < nang; j0 += ANG) {
+      __syncthreads();
+      for (int k = threadIdx.x; k < min(ANG, nang - j0); k += blockDim.x) {
+        const dvec4 o = ofs[j0 + k];
+        // an angle of NaN: every pixel off the detector
+        sa[k] = isfinite(o.x + o.y + o.z) ? fix_angle<FIX>(o.x, o.y, o.z) : FixAngle{{0, 0}, {0, 0}, {-2 * FIX_ONE, 0}};
+      }
+      __syncthreads();
+      if (t >= N * N) continue;
+      const int m = min(ANG, nang - j0);
 #pragma unroll 4
-    for (int k = 0; k < m; ++k) {
-      const long long c = x * sx[k] + y * sy[k] + so[k];
-      if (c > -FIX_ONE && c < end) {
-        const int il = (int)(c >> FIX);
-        const double p = from_fix<FIX>(c & (FIX_ONE - 1));
-        const double *__restrict__ row = sino + (size_t)(j0 + k) * nd;
-        if (il >= 0) acc = __fma_rn(1.0 - p, row[il], acc);
-        if (il <= nd - 2) acc = __fma_rn(p, row[il + 1], acc);
+      for (int k = 0; k < m; ++k) {
+        const long long c = fix_at(sa[k], x, y).hi;
+        if (c > -FIX_ONE && c < end) taps(j0 + k, (int)(c >> FIX), from_fix<FIX>(c & (FIX_ONE - 1)));
+      }
+    }
+  } else if (t < N * N) {
+    for (int j = 0; j < nang; ++j) {
+      const dvec4 o = ofs[j];
+      const double tt = x * o.x + y * o.y + o.z;
+      if (tt > -1.0 && tt < nd) {
+        const double fl = floor(tt);
+        taps(j, (int)fl, tt - fl);
       }
     }
   }
@@ -2631,6 +2647,13 @@ cudaError_t fill_f32(float *x, size_t n, float v, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// x <- R^T R x of one slice
+template <int FIX>
+static void radon64(double *d_img, double *d_sino, const dvec4 *ofs, int N, int nd, int nang, cudaStream_t st) {
+  k_radon64_warp<FIX><<<blocks_for(32LL * nd * nang, 256), 256, 0, st>>>(d_img, d_sino, ofs, N, nd, nang);
+  k_radon_ad64<FIX><<<blocks_for((long long)N * N, 128), 128, 0, st>>>(d_sino, d_img, ofs, N, nd, nang);
+}
+
 // power iteration: up to `rounds` rounds of  s = sum(img); img /= s; img = R^T R img
 // from the all-ones image, stopping once two consecutive sums agree to 1e-10;
 // returns sqrt(s) (the reference's 10 rounds from randn, in FP32).
@@ -2654,13 +2677,11 @@ cudaError_t normest64(const dvec4 *ofs, int N, int nd, int nang, int rounds, dou
       prev = s;
     }
     k_scale64<<<64, 256, 0, st>>>(d_img, n, d_part + nb);
-    const unsigned gf = blocks_for(32LL * nd * nang, 256), gb = blocks_for((long long)n, 128);
-    if ((long long)nd + 2LL * N < (1 << 18)) {
-      k_radon64_warp<44><<<gf, 256, 0, st>>>(d_img, d_sino, ofs, N, nd, nang);
-      k_radon_ad64<44><<<gb, 128, 0, st>>>(d_sino, d_img, ofs, N, nd, nang);
-    } else {
-      k_radon64_warp<30><<<gf, 256, 0, st>>>(d_img, d_sino, ofs, N, nd, nang);
-      k_radon_ad64<30><<<gb, 128, 0, st>>>(d_sino, d_img, ofs, N, nd, nang);
+    switch (fix_bits((long long)nd + 2LL * N)) {  // |t|, |off| <= nd / 2 + N
+      case 52: radon64<52>(d_img, d_sino, ofs, N, nd, nang, st); break;
+      case 48: radon64<48>(d_img, d_sino, ofs, N, nd, nang, st); break;
+      case 44: radon64<44>(d_img, d_sino, ofs, N, nd, nang, st); break;
+      default: radon64<0>(d_img, d_sino, ofs, N, nd, nang, st); break;
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
