@@ -1682,6 +1682,7 @@ struct gt_subs {
   int *m_start = nullptr, *m_idx = nullptr, *mt_start = nullptr, *mt_idx = nullptr;
   float *m_val = nullptr, *mt_val = nullptr;
   double *part = nullptr;
+  float *scratch = nullptr, *stage = nullptr;
   cudaGraphExec_t g_one = nullptr, g_chunk = nullptr;
   double normest = 0;
   float sigma_data = 0;
@@ -1840,6 +1841,12 @@ int gt_subs_create(const gt_subs_desc *D, gt_subs **out) {
   const size_t o_ms = take(4 * start.size()), o_mi = take(4 * idx.size()), o_mv = take(4 * val.size());
   const size_t o_ts = take(4 * tstart.size()), o_ti = take(4 * tidx.size()), o_tv = take(4 * tval.size());
   const size_t o_part = take(8 * 256);
+  // an int or float per bin of either series, fine or coarse detector; staging of any field that is
+  // copied in or out (the inner problem's buffer is sized by its own series)
+  const size_t o_scr = take(4 * (size_t)std::max(D->nang0, D->nang1) * std::max(nd0, D->nd1));
+  const size_t staged = std::max({NN, (size_t)D->nang0 * nd0 * s->S0, (size_t)D->nang1 * nd0 * s->S1, nblo});
+  const bool own_stage = staged > std::max(p->d.vol, p->d.nbin);
+  const size_t o_stage = take(own_stage ? 4 * staged : 0);
   if ((e = cudaMalloc(&s->block, off)) != cudaSuccess) {
     cudaGetLastError();
     gt_subs_destroy(s);
@@ -1855,6 +1862,8 @@ int gt_subs_create(const gt_subs_desc *D, gt_subs **out) {
   s->m_start = (int *)(b + o_ms); s->m_idx = (int *)(b + o_mi); s->m_val = (float *)(b + o_mv);
   s->mt_start = (int *)(b + o_ts); s->mt_idx = (int *)(b + o_ti); s->mt_val = (float *)(b + o_tv);
   s->part = (double *)(b + o_part);
+  s->scratch = (float *)(b + o_scr);
+  s->stage = own_stage ? (float *)(b + o_stage) : p->stage;
   // angle tables: both series on the fine detector (radon_struct with n_detectors = Nx0, :926-931)
   auto table = [&](const double *ang, int nang, float4 *dst) -> int {
     std::vector<double> t64;
@@ -1893,7 +1902,7 @@ int gt_subs_create(const gt_subs_desc *D, gt_subs **out) {
     Q.ofs = ofs;
     Q.fwd_cfg = gt::default_fwd_shape(ld);
     Q.bp_cfg = gt::default_bp_shape(ld);
-    int *scratch = (int *)s->ku1;  // an int per bin of the geometry; written by every projection
+    int *scratch = (int *)s->scratch;
     int r = GT_OK;
     if (inner) {  // the inner problem's own geometry: its tables
       Q.ray_start = p->P.ray_start; Q.ray_ent = p->P.ray_ent; Q.tap_hdr = p->P.tap_hdr; Q.tap_frac = p->P.tap_frac;
@@ -1932,16 +1941,16 @@ int gt_subs_set_data(gt_subs *s, const float *f0, const float *f1, int make_feas
   const size_t nb0 = (size_t)s->nang0 * nd0 * s->S0, nblo = (size_t)s->nang1 * s->nd1 * s->S1lo;
   // host layout [S][bins] -> device [bins][S]
   if (s->C0) {
-    CK(cudaMemcpyAsync(p->stage, f0, 4 * nb0, cudaMemcpyHostToDevice, p->stream));
-    CK(gt::launch_transpose(p->stage, s->f0, s->S0, s->nang0 * nd0, s->nang0 * nd0, ld0, p->stream));
+    CK(cudaMemcpyAsync(s->stage, f0, 4 * nb0, cudaMemcpyHostToDevice, p->stream));
+    CK(gt::launch_transpose(s->stage, s->f0, s->S0, s->nang0 * nd0, s->nang0 * nd0, ld0, p->stream));
   }
-  CK(cudaMemcpyAsync(p->stage, f1, 4 * nblo, cudaMemcpyHostToDevice, p->stream));
-  CK(gt::launch_transpose(p->stage, s->f1, s->S1lo, s->nang1 * s->nd1, s->nang1 * s->nd1, s->S1lo, p->stream));
+  CK(cudaMemcpyAsync(s->stage, f1, 4 * nblo, cudaMemcpyHostToDevice, p->stream));
+  CK(gt::launch_transpose(s->stage, s->f1, s->S1lo, s->nang1 * s->nd1, s->nang1 * s->nd1, s->S1lo, p->stream));
   if (make_feasible) {
     // Make_function_feasible (3dsubsample :466-476): bins where the projection of the
     // all-ones slice is <= 0 are zeroed (the low-resolution data uses the mask of the
     // fine detector, restricted to its own bins)
-    float *ones = p->stage, *r1 = p->ku;
+    float *ones = s->stage, *r1 = s->scratch;
     CK(gt::fill_f32(ones, (size_t)s->N * s->N, 1.f, p->stream));
     if (s->C0) {
       CK(gt::launch_radon(ones, r1, s->ofs0, s->N, nd0, s->nang0, 1, p->stream));
@@ -2062,8 +2071,8 @@ int gt_subs_get(gt_subs *s, int which, float *host) {
     default: return set_err(GT_ERR_ARG, "unknown field %d", which);
   }
   if (cols == 0) return GT_OK;
-  CK(gt::launch_transpose(src, p->stage, rows, cols, ld, rows, p->stream));
-  CK(cudaMemcpyAsync(host, p->stage, 4 * (size_t)rows * cols, cudaMemcpyDeviceToHost, p->stream));
+  CK(gt::launch_transpose(src, s->stage, rows, cols, ld, rows, p->stream));
+  CK(cudaMemcpyAsync(host, s->stage, 4 * (size_t)rows * cols, cudaMemcpyDeviceToHost, p->stream));
   CK(cudaStreamSynchronize(p->stream));
   return GT_OK;
 }

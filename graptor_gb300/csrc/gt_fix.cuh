@@ -5,7 +5,7 @@
 // rounding of X and Y: t is off by at most 2^-(FIX + 1) from its last rounding and (x + y + 1)
 // 2^-(FIX + 33) from X, Y and off.  In FP64 it is off by half an ulp of x X, of x X + y Y and of t,
 // 2^-45 each from 2^8 on; fix_bits chooses FIX so that the fixed-point t is nowhere worse: errors of up to
-// 1.2e-16 against 8e-14 for a 256^2 image and as many bins, 1.8e-15 against 1.7e-13 for 512^2.
+// 1.2e-16 against 8e-14 for a 256^2 image and as many bins, 1.8e-15 against 1.3e-13 for 512^2.
 #pragma once
 #include <math.h>
 
