@@ -1046,10 +1046,9 @@ void *gt_problem_stream(gt_problem *p) { return p ? (void *)p->stream : nullptr;
 
 int gt_set_tuning(gt_problem *p, int fwd_cfg, int bp_cfg) {
   if (!p) return set_err(GT_ERR_ARG, "null argument");
-  if (fwd_cfg < 0 || fwd_cfg >= gt::num_proj_configs(p->Sr, 0) || bp_cfg < 0 ||
-      bp_cfg >= gt::num_proj_configs(p->Sr, 1))
-    return set_err(GT_ERR_ARG, "launch configuration out of range (%d forward, %d back-projection configurations)",
-                   gt::num_proj_configs(p->Sr, 0), gt::num_proj_configs(p->Sr, 1));
+  const int nf = gt::num_proj_configs(p->d.S, 0), nb = gt::num_proj_configs(p->d.S, 1);
+  if (fwd_cfg < 0 || fwd_cfg >= nf || bp_cfg < 0 || bp_cfg >= nb)
+    return set_err(GT_ERR_ARG, "launch configuration out of range (%d forward, %d back-projection configurations)", nf, nb);
   CK(cudaSetDevice(p->device));
   CK(cudaStreamSynchronize(p->stream));
   if (fwd_cfg == 8 || fwd_cfg == 10 || fwd_cfg == 11) {

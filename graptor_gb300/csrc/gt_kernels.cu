@@ -2236,8 +2236,8 @@ cudaError_t launch_dual_fused(const IterParams &P, int tgv, int cpl, cudaStream_
 // gt_proj.cu).
 // Otherwise one fixed shape.
 int num_proj_configs(int S, int which) {
-  if (S % 4 != 0) return 1;
-  return which == 0 ? 20 : 20;
+  (void)which;
+  return S % 4 != 0 ? 1 : 20;
 }
 
 template <int VW, int UNR, int MINB = 1>
@@ -2263,6 +2263,7 @@ cudaError_t launch_bp_staged(const IterParams &P, cudaStream_t st);
 // / 359 / 426 / 386; 384 (512^2, 141) 5044 / 4404 / - / 8130 / 7795 (there 8 per lane leave a quarter
 // of the lanes idle).
 int default_fwd_shape(int S) {
+  if (S % 4 != 0) return 0;  // the one shape (num_proj_configs)
   if (S == 4) return 7;
   if (S <= 92) return 9;
   const int w8 = (S + 255) / 256 * 256, w4 = (S + 127) / 128 * 128;
@@ -2308,6 +2309,7 @@ static void bp_vw(const IterParams &P, cudaStream_t st) {
 // 213 / 242 / 361 / 440; 384 (512^2, 141) 2912 / 2628 / 4050 / 6856 (there 8 per lane leave
 // a quarter of the lanes idle).
 int default_bp_shape(int S) {
+  if (S % 4 != 0) return 0;  // the one shape (num_proj_configs)
   if (S == 4) return 12;
   if (S <= 48) return 10;
   if (S <= 64) return 9;  // alone as k_bp_flat, beside other work faster (three at once: 22 us each against 28)
