@@ -677,33 +677,15 @@ int gt_set_schedule(gt_problem *p, int schedule) {
   return GT_OK;
 }
 
-int gt_problem_create(const gt_desc *desc, gt_problem **out) {
-  if (!desc || !out) return set_err(GT_ERR_ARG, "null argument");
-  *out = nullptr;
-  const gt_desc &D = *desc;
-  if (D.dim != 2 && D.dim != 3) return set_err(GT_ERR_ARG, "dim must be 2 or 3 (got %d)", D.dim);
-  if (D.N < 1 || D.Nz < 1 || D.C < 1 || D.nd < 1 || D.nang < 1)
-    return set_err(GT_ERR_ARG, "sizes must be positive (N=%d Nz=%d C=%d nd=%d nang=%d)", D.N, D.Nz, D.C, D.nd, D.nang);
-  if (D.coupling != GT_UNCORR && D.C > 8)
-    return set_err(GT_ERR_ARG, "coupled regularisation supports at most 8 channels (got %d)", D.C);
-  if (D.discrepancy != GT_KL && D.discrepancy != GT_L2) return set_err(GT_ERR_ARG, "bad discrepancy");
-  if (D.regularisation != GT_TV && D.regularisation != GT_TGV) return set_err(GT_ERR_ARG, "bad regularisation");
-  if (D.coupling < GT_UNCORR || D.coupling > GT_NUCL) return set_err(GT_ERR_ARG, "bad coupling");
-  if (!D.angles || !D.mu) return set_err(GT_ERR_ARG, "angles and mu are required");
-  if (!(D.stepsize > 0.f)) return set_err(GT_ERR_ARG, "stepsize must be positive");
-  if (D.regularisation == GT_TGV && !(D.alpha0 > 0 && D.alpha1 > 0)) return set_err(GT_ERR_ARG, "alpha must be positive");
-  if (D.regularisation == GT_TV && !(D.alpha1 > 0)) return set_err(GT_ERR_ARG, "alpha1 must be positive");
-  const long long Sr = (long long)D.Nz * D.C;
-  if ((long long)D.N * D.N > (1LL << 30) || Sr > (1LL << 20) || (long long)D.nd * D.nang > (1LL << 30))
-    return set_err(GT_ERR_ARG, "problem too large for 32-bit pixel / bin indices");
-  const long long S = padded_slices((int)Sr);
+// a problem of Sr slices, S of them in memory (checked arguments)
+static int create_problem(const gt_desc &D, int Sr, int S, gt_problem **out) {
   const long long vol = (long long)D.N * D.N * S, nbin = (long long)D.nd * D.nang * S;
 
   gt_problem *p = new (std::nothrow) gt_problem();
   if (!p) return set_err(GT_ERR_OOM, "host allocation failed");
   p->device = D.device;
-  p->d.dim = D.dim; p->d.N = D.N; p->d.Nz = D.Nz; p->d.C = D.C; p->d.S = (int)S;
-  p->Sr = (int)Sr;
+  p->d.dim = D.dim; p->d.N = D.N; p->d.Nz = D.Nz; p->d.C = D.C; p->d.S = S;
+  p->Sr = Sr;
   p->d.nd = D.nd; p->d.nang = D.nang; p->d.vol = (size_t)vol; p->d.nbin = (size_t)nbin;
   p->disc = D.discrepancy; p->reg = D.regularisation; p->cpl = D.coupling;
   p->K = D.dim; p->KW = D.dim == 3 ? 6 : 3;
@@ -810,6 +792,31 @@ int gt_problem_create(const gt_desc *desc, gt_problem **out) {
   }
   *out = p;
   return GT_OK;
+}
+
+int gt_problem_create(const gt_desc *desc, gt_problem **out) {
+  if (!desc || !out) return set_err(GT_ERR_ARG, "null argument");
+  *out = nullptr;
+  const gt_desc &D = *desc;
+  if (D.dim != 2 && D.dim != 3) return set_err(GT_ERR_ARG, "dim must be 2 or 3 (got %d)", D.dim);
+  if (D.N < 1 || D.Nz < 1 || D.C < 1 || D.nd < 1 || D.nang < 1)
+    return set_err(GT_ERR_ARG, "sizes must be positive (N=%d Nz=%d C=%d nd=%d nang=%d)", D.N, D.Nz, D.C, D.nd, D.nang);
+  if (D.coupling != GT_UNCORR && D.C > 8)
+    return set_err(GT_ERR_ARG, "coupled regularisation supports at most 8 channels (got %d)", D.C);
+  if (D.discrepancy != GT_KL && D.discrepancy != GT_L2) return set_err(GT_ERR_ARG, "bad discrepancy");
+  if (D.regularisation != GT_TV && D.regularisation != GT_TGV) return set_err(GT_ERR_ARG, "bad regularisation");
+  if (D.coupling < GT_UNCORR || D.coupling > GT_NUCL) return set_err(GT_ERR_ARG, "bad coupling");
+  if (!D.angles || !D.mu) return set_err(GT_ERR_ARG, "angles and mu are required");
+  if (!(D.stepsize > 0.f)) return set_err(GT_ERR_ARG, "stepsize must be positive");
+  if (D.regularisation == GT_TGV && !(D.alpha0 > 0 && D.alpha1 > 0)) return set_err(GT_ERR_ARG, "alpha must be positive");
+  if (D.regularisation == GT_TV && !(D.alpha1 > 0)) return set_err(GT_ERR_ARG, "alpha1 must be positive");
+  const long long Sr = (long long)D.Nz * D.C;
+  if ((long long)D.N * D.N > (1LL << 30) || Sr > (1LL << 20) || (long long)D.nd * D.nang > (1LL << 30))
+    return set_err(GT_ERR_ARG, "problem too large for 32-bit pixel / bin indices");
+  int rc = create_problem(D, (int)Sr, padded_slices((int)Sr), out);
+  // no room for the padding (0.23 KB per pixel and more at S = 5): as without it, by slower kernels
+  if (rc == GT_ERR_OOM && padded_slices((int)Sr) != Sr) rc = create_problem(D, (int)Sr, (int)Sr, out);
+  return rc;
 }
 
 void gt_problem_destroy(gt_problem *p) {
@@ -1768,13 +1775,8 @@ void gt_subs_destroy(gt_subs *s) {
   delete s;
 }
 
-int gt_subs_create(const gt_subs_desc *D, gt_subs **out) {
-  if (!D || !out) return set_err(GT_ERR_ARG, "null argument");
-  *out = nullptr;
-  if (D->N < 1 || D->Nz < 1 || D->C0 < 0 || D->C1 < 1 || D->C0 + D->C1 > 8 || D->nang0 < (D->C0 ? 1 : 0) ||
-      D->nang1 < 1 || D->nd1 < 1 || D->Nz1 < 1 || !(D->pixel_ratio > 0) || !D->angles1 || (D->C0 && !D->angles0) ||
-      !D->mu || (D->coupling != GT_FROB && D->coupling != GT_UNCORR))
-    return set_err(GT_ERR_ARG, "gt_subs_create: invalid description");
+// pad: slices padded in memory (padded_slices); D is checked
+static int create_subs(const gt_subs_desc *D, bool pad, gt_subs **out) {
   gt_subs *s = new (std::nothrow) gt_subs();
   if (!s) return set_err(GT_ERR_OOM, "host allocation failed");
   s->C0 = D->C0; s->C1 = D->C1; s->Nz = D->Nz; s->Nz1 = D->Nz1; s->nd1 = D->nd1; s->N = D->N;
@@ -1788,7 +1790,8 @@ int gt_subs_create(const gt_subs_desc *D, gt_subs **out) {
   d.stepsize = D->stepsize; d.alpha0 = D->alpha0; d.alpha1 = D->alpha1; d.mu = D->mu;
   d.discrepancy = D->discrepancy; d.regularisation = D->regularisation; d.coupling = D->coupling;
   d.normest = 1.0; d.device = D->device; d.stream = D->stream; d.autotune = 0;
-  int rc = gt_problem_create(&d, &s->p);
+  const int Sr = d.Nz * d.C;
+  int rc = pad ? gt_problem_create(&d, &s->p) : create_problem(d, Sr, Sr, &s->p);
   if (rc) { delete s; return rc; }
   s->p->lsqr = 36.0;
   gt_problem *p = s->p;
@@ -1826,7 +1829,7 @@ int gt_subs_create(const gt_subs_desc *D, gt_subs **out) {
   }
   // device block
   const size_t NN = (size_t)D->N * D->N;
-  const int ld0 = padded_slices(s->S0), ld1 = padded_slices(s->S1);
+  const int ld0 = pad ? padded_slices(s->S0) : s->S0, ld1 = pad ? padded_slices(s->S1) : s->S1;
   const size_t nb0 = (size_t)D->nang0 * nd0 * ld0, nb1 = (size_t)D->nang1 * nd0 * ld1,
                nblo = (size_t)D->nang1 * D->nd1 * s->S1lo;
   size_t off = 0;
@@ -1928,6 +1931,18 @@ int gt_subs_create(const gt_subs_desc *D, gt_subs **out) {
   s->normest = D->normest;
   *out = s;
   return GT_OK;
+}
+
+int gt_subs_create(const gt_subs_desc *D, gt_subs **out) {
+  if (!D || !out) return set_err(GT_ERR_ARG, "null argument");
+  *out = nullptr;
+  if (D->N < 1 || D->Nz < 1 || D->C0 < 0 || D->C1 < 1 || D->C0 + D->C1 > 8 || D->nang0 < (D->C0 ? 1 : 0) ||
+      D->nang1 < 1 || D->nd1 < 1 || D->Nz1 < 1 || !(D->pixel_ratio > 0) || !D->angles1 || (D->C0 && !D->angles0) ||
+      !D->mu || (D->coupling != GT_FROB && D->coupling != GT_UNCORR))
+    return set_err(GT_ERR_ARG, "gt_subs_create: invalid description");
+  int rc = create_subs(D, true, out);
+  if (rc == GT_ERR_OOM) rc = create_subs(D, false, out);  // as in gt_problem_create
+  return rc;
 }
 
 // f0: [C0*Nz][nang0][N], f1: [C1*Nz1][nang1][nd1] (s = c*Nz + z); resets the iterates
