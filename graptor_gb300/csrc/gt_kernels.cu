@@ -1703,8 +1703,12 @@ __global__ void k_radon64_warp(const double *__restrict__ img, double *__restric
   const dvec4 o = ofs[j];
   FixAngle a{};
   if constexpr (FIX > 0) {
-    a = fix_angle<FIX>(o.x, o.y, o.z);
-    a.off.hi -= i * FIX_ONE;  // t - i
+    // the warp's first three lanes convert one number each
+    const FixNum f = to_fix<FIX>(lane == 0 ? o.x : lane == 1 ? o.y : o.z);
+    auto of = [&](int l) { return FixNum{__shfl_sync(0xffffffffu, f.hi, l), __shfl_sync(0xffffffffu, f.lo, l)}; };
+    const FixNum X = of(0), Y = of(1), off = of(2);
+    a = fix_angle(X, Y, off);
+    a.off -= i * FIX_ONE;  // t - i
   }
   double acc = 0.0;
   for (int y = isfinite(o.x + o.y + o.z) ? lane : N; y < N; y += 32) {  // an angle of NaN takes no pixel
@@ -1721,7 +1725,7 @@ __global__ void k_radon64_warp(const double *__restrict__ img, double *__restric
     const double *__restrict__ row = img + (size_t)y * N;
     if constexpr (FIX > 0) {
       FixNum c = fix_at(a, xl, y);
-      for (int x = xl; x <= xh; ++x, fix_step(c, a.X)) {
+      for (int x = xl; x <= xh; ++x, fix_step(c, a)) {
         const long long wgt = FIX_ONE - (c.hi < 0 ? -c.hi : c.hi);
         if (wgt > 0) acc = __fma_rn(from_fix<FIX>(wgt), row[x], acc);
       }
@@ -1759,7 +1763,8 @@ __global__ void __launch_bounds__(128) k_radon_ad64(const double *__restrict__ s
       for (int k = threadIdx.x; k < min(ANG, nang - j0); k += blockDim.x) {
         const dvec4 o = ofs[j0 + k];
         // an angle of NaN: every pixel off the detector
-        sa[k] = isfinite(o.x + o.y + o.z) ? fix_angle<FIX>(o.x, o.y, o.z) : FixAngle{{0, 0}, {0, 0}, {-2 * FIX_ONE, 0}};
+        sa[k] = isfinite(o.x + o.y + o.z) ? fix_angle(to_fix<FIX>(o.x), to_fix<FIX>(o.y), to_fix<FIX>(o.z))
+                                          : FixAngle{0, 0, -2 * FIX_ONE, 0, 0, 0};
       }
       __syncthreads();
       if (t >= N * N) continue;

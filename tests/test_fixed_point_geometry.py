@@ -13,10 +13,10 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 SRC = """
 #include "gt_fix.cuh"
 template <int FIX> static void at(long n, const double *o, const int *x0, const int *x, const int *y, long long *out) {
-  const gt::FixAngle a = gt::fix_angle<FIX>(o[0], o[1], o[2]);
+  const gt::FixAngle a = gt::fix_angle(gt::to_fix<FIX>(o[0]), gt::to_fix<FIX>(o[1]), gt::to_fix<FIX>(o[2]));
   for (long k = 0; k < n; ++k) {  // from x0 to x by steps
     gt::FixNum t = gt::fix_at(a, x0[k], y[k]);
-    for (int q = x0[k]; q < x[k]; ++q) gt::fix_step(t, a.X);
+    for (int q = x0[k]; q < x[k]; ++q) gt::fix_step(t, a);
     out[k] = t.hi;
   }
 }
@@ -71,6 +71,6 @@ def test_coordinates_are_no_further_off_than_in_fp64(lib, N, nd):
         for k in range(n):
             exact = int(x[k]) * Fraction(o[0]) + int(y[k]) * Fraction(o[1]) + Fraction(o[2])
             err = abs(Fraction(int(out[k]), 2 ** fix) - exact)
-            assert err <= Fraction(1, 2 ** (fix + 1)) + Fraction(int(x[k]) + int(y[k]) + 1, 2 ** (fix + 33))
+            assert err <= Fraction(1, 2 ** (fix + 1)) + Fraction(int(x[k]) + int(y[k]) + 1, 2 ** (fix + 17))
             worst_fix, worst_64 = max(worst_fix, err), max(worst_64, abs(Fraction(float(t64[k])) - exact))
     assert worst_fix <= worst_64, (float(worst_fix), float(worst_64))
