@@ -476,6 +476,56 @@ int upload_mu_eff(gt_problem *p) {
   return GT_OK;
 }
 
+// The form of the iteration, from graph-captured iterations of each (16, the second and third
+// launch timed), the faster kept: concurrency between the kernels decides, not their times
+// alone.  From 8M voxel-channels on the schedules 0 and 1 (TGV only: TV has no p / pbar half);
+// below, where the two are within a few per cent (0.135 / 0.132 ms at 128^2 x 32 x 2), schedule
+// 1, and with 1, 2 or 4 slices the two-launch form of gt_small.cu against it.
+// Schedule 2 (the p half fused into the next dual kernel) is not timed: its
+// fused kernel is slower than the dual kernel and the p half together on every
+// measured workload (256^2 x 60 x 4: 1.07 ms against 0.25 + 0.16 ms), so it
+// stays a choice of gt_set_schedule.
+int tune_form(gt_problem *p) {
+  const bool tgv = p->reg == GT_TGV, log = std::getenv("GRAPTOR_TUNE_LOG") != nullptr;
+  cudaEvent_t e0, e1;
+  CK(cudaEventCreate(&e0));
+  CK(cudaEventCreate(&e1));
+  int rc = GT_OK;
+  const bool large = p->d.vol >= (8u << 20);
+  float ms_f[2] = {1e30f, 1e30f};  // schedules 0 and 1, or schedule 1 and the two-launch form
+  auto set_form = [&](int f) {
+    p->small = !large && f == 1;
+    if (tgv) p->schedule = large ? f : 1;
+  };
+  const int nform = large ? (tgv ? 2 : 1) : (gt::small_ok(p->P, p->cpl) ? 2 : 1);
+  for (int round = 0; round < 2 && nform > 1 && rc == GT_OK; ++round) {
+    for (int f = 0; f < nform && rc == GT_OK; ++f) {
+      set_form(f);
+      cudaGraphExec_t g = nullptr;
+      rc = capture(p, 16, &g);
+      if (rc) break;
+      cudaError_t e = cudaGraphLaunch(g, p->stream);
+      if (e == cudaSuccess) e = cudaEventRecord(e0, p->stream);
+      for (int r = 0; r < 2 && e == cudaSuccess; ++r) e = cudaGraphLaunch(g, p->stream);
+      if (e == cudaSuccess) e = cudaEventRecord(e1, p->stream);
+      if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+      float ms = 0.f;
+      if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+      cudaGraphExecDestroy(g);
+      if (e != cudaSuccess) { rc = cuda_err(e, "autotune (iteration)", __LINE__); break; }
+      ms_f[f] = std::min(ms_f[f], ms / 32);
+    }
+  }
+  set_form(nform > 1 && ms_f[1] < ms_f[0] ? 1 : 0);
+  free_fused(p);
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  if (log && rc == GT_OK && nform > 1)
+    fprintf(stderr, "graptor autotune %s: %.4f ms, %s: %.4f ms per iteration\n", large ? "schedule 0" : "schedule 1",
+            ms_f[0], large ? "schedule 1" : "two launches", ms_f[1]);
+  return rc;
+}
+
 // ---------------------------------------------------------------------------
 // Autotuner: times every launch shape of k_fwd and k_bp (gt_kernels.cu,
 // launch_fwd / launch_bp) with CUDA events on the problem's own buffers and keeps
@@ -484,7 +534,12 @@ int upload_mu_eff(gt_problem *p) {
 // launches never touch the solve.
 using TuneKey = std::tuple<int, int, int, int, int, int, int, int, int, int>;
 std::mutex g_tune_mu;
-std::map<TuneKey, std::tuple<int, int, int, int, bool>> g_tune;
+struct TuneVal {
+  int fwd = 0, bp = 0, dual = 0;
+  int schedule = -1;  // -1: the form of the iteration was chosen by gt_set_schedule and not timed
+  bool small = false;
+};
+std::map<TuneKey, TuneVal> g_tune;
 
 int autotune(gt_problem *p) {
   const bool tgv = p->reg == GT_TGV;
@@ -503,33 +558,51 @@ int autotune(gt_problem *p) {
   const int S = p->d.S;
   auto skipped = [&](int which, int c) {
     if (which == 0)
-      return !((c == 10 && S > 128) || (c == 11 && S >= kPairSlices) || (c == 8 && S >= kPairSlices && S <= 128) || (c == 9 && S <= 128) || (c == 5 && S <= 32) ||
-               (c == 7 && S == 4));
+      return !((c == 10 && S > 128) || (c == 11 && S >= kPairSlices) || (c == 8 && S >= kPairSlices && S <= 128) ||
+               (c == 9 && S <= 128) || (c == 5 && S <= 32) || (c == 7 && S == 4));
     if (which == 1)
       return !((c == 18 && S >= 96) || (c == 19 && S >= 36) || (c == 9 && S >= 16 && S <= 128) ||
                (c == 10 && S <= 128) || (c == 11 && S <= 16) || (c == 12 && S == 4));
     return false;
   };
-  p->small = false;
+  if (!p->schedule_set) p->small = false;
   p->P.fwd_cfg = gt::default_fwd_shape(S);
   p->P.bp_cfg = gt::default_bp_shape(S);
   p->P.dual_cfg = gt::default_dual_shape(p->P, p->cpl);
   if ((nc[0] <= 1 && nc[1] <= 1 && nc[2] <= 1) || !p->autotune) return GT_OK;
   const TuneKey key{p->d.dim, p->d.N, p->d.S, p->d.nd, p->d.nang, p->disc, p->d.C, p->d.Nz, p->reg, p->cpl};
+  TuneVal tuned{};
+  bool hit = false;
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
     if (it != g_tune.end()) {
-      int sched = 0;
-      bool small = false;
-      std::tie(p->P.fwd_cfg, p->P.bp_cfg, p->P.dual_cfg, sched, small) = it->second;
-      p->small = small && !p->schedule_set;
-      // sched < 0: the schedule was chosen by gt_set_schedule when the shapes were
-      // tuned, not timed; 0 is the measured choice at 8M voxel-channels and above
-      if (!p->schedule_set) p->schedule = sched >= 0 ? sched : (p->d.vol >= (8u << 20) ? 0 : 1);
+      tuned = it->second;
+      hit = true;
+    }
+  }
+  auto keep = [&]() {  // an entry whose form is timed stays
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    TuneVal &t = g_tune[key];
+    t = TuneVal{p->P.fwd_cfg, p->P.bp_cfg, p->P.dual_cfg, p->schedule_set ? t.schedule : p->schedule,
+                p->schedule_set ? t.small : p->small};
+  };
+  if (hit) {
+    p->P.fwd_cfg = tuned.fwd;
+    p->P.bp_cfg = tuned.bp;
+    p->P.dual_cfg = tuned.dual;
+    if (p->schedule_set) {
       if (p->schedule == 2 && ensure_fused(p) != GT_OK) p->schedule = 0;  // no room for the second set
       return GT_OK;
     }
+    if (tuned.schedule >= 0) {
+      p->schedule = tuned.schedule;
+      p->small = tuned.small;
+      return GT_OK;
+    }
+    const int rc = tune_form(p);
+    if (rc == GT_OK) keep();
+    return rc;
   }
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
@@ -580,61 +653,15 @@ int autotune(gt_problem *p) {
       for (int c = 0; c < nc[which] && nc[which] > 1; ++c)
         fprintf(stderr, "graptor autotune %s cfg %d: %.4f ms%s\n", names[which], c, ms_cfg[which][c],
                 c == best[which] ? " *" : "");
-  if (rc) {
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    return rc;
-  }
-  p->P.fwd_cfg = best[0];
-  p->P.bp_cfg = best[1];
-  p->P.dual_cfg = best[2];
-  // The form of the iteration, from graph-captured iterations of each (16, the second and third
-  // launch timed), the faster kept: concurrency between the kernels decides, not their times
-  // alone.  From 8M voxel-channels on the schedules 0 and 1 (TGV only: TV has no p / pbar half);
-  // below, where the two are within a few per cent (0.135 / 0.132 ms at 128^2 x 32 x 2), schedule
-  // 1, and with 1, 2 or 4 slices the two-launch form of gt_small.cu against it.
-  // Schedule 2 (the p half fused into the next dual kernel) is not timed: its
-  // fused kernel is slower than the dual kernel and the p half together on every
-  // measured workload (256^2 x 60 x 4: 1.07 ms against 0.25 + 0.16 ms), so it
-  // stays a choice of gt_set_schedule.
-  if (!p->schedule_set) {
-    const bool large = p->d.vol >= (8u << 20);
-    float ms_f[2] = {1e30f, 1e30f};  // schedules 0 and 1, or schedule 1 and the two-launch form
-    auto set_form = [&](int f) {
-      p->small = !large && f == 1;
-      if (tgv) p->schedule = large ? f : 1;
-    };
-    const int nform = large ? (tgv ? 2 : 1) : (gt::small_ok(p->P, p->cpl) ? 2 : 1);
-    for (int round = 0; round < 2 && nform > 1 && rc == GT_OK; ++round) {
-      for (int f = 0; f < nform && rc == GT_OK; ++f) {
-        set_form(f);
-        cudaGraphExec_t g = nullptr;
-        rc = capture(p, 16, &g);
-        if (rc) break;
-        cudaError_t e = cudaGraphLaunch(g, p->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(e0, p->stream);
-        for (int r = 0; r < 2 && e == cudaSuccess; ++r) e = cudaGraphLaunch(g, p->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(e1, p->stream);
-        if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-        float ms = 0.f;
-        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-        cudaGraphExecDestroy(g);
-        if (e != cudaSuccess) { rc = cuda_err(e, "autotune (iteration)", __LINE__); break; }
-        ms_f[f] = std::min(ms_f[f], ms / 32);
-      }
-    }
-    set_form(nform > 1 && ms_f[1] < ms_f[0] ? 1 : 0);
-    free_fused(p);
-    if (log && rc == GT_OK && nform > 1)
-      fprintf(stderr, "graptor autotune %s: %.4f ms, %s: %.4f ms per iteration\n", large ? "schedule 0" : "schedule 1",
-              ms_f[0], large ? "schedule 1" : "two launches", ms_f[1]);
-  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc) return rc;
-  std::lock_guard<std::mutex> lk(g_tune_mu);
-  g_tune[key] = std::make_tuple(best[0], best[1], best[2], p->schedule_set ? -1 : p->schedule, p->small);
-  return GT_OK;
+  p->P.fwd_cfg = best[0];
+  p->P.bp_cfg = best[1];
+  p->P.dual_cfg = best[2];
+  if (!p->schedule_set) rc = tune_form(p);
+  if (rc == GT_OK) keep();
+  return rc;
 }
 
 }  // namespace

@@ -64,3 +64,28 @@ def test_flat_pair_shape_on_edges_and_infinities(N, nd, Nz, C):
     for a, b in got[1:]:
         np.testing.assert_array_equal(a, got[0][0])
         np.testing.assert_array_equal(b, got[0][1])
+
+
+FORM = """
+import numpy as np
+from graptor_gb300.solver import Problem
+ang = np.deg2rad(np.linspace(-80, 85, 11))
+for schedule in (0, None, None):
+    with Problem(2, 24, 1, 1, 24, ang, (4, 1), [0.2], normest=11.0) as p:
+        if schedule is not None:
+            p.set_schedule(schedule)
+        p.set_data(np.ones((1, 11, 24), np.float32)).run(3).synchronize()
+"""
+
+
+def test_a_chosen_schedule_does_not_stand_for_later_problems():
+    """The first problem of a size has its schedule set and its form of the iteration not timed: the second
+    one times it, the third takes the result."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", FORM], cwd=root, env=dict(os.environ, GRAPTOR_TUNE_LOG="1"),
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    assert r.stderr.count("two launches:") == 1, r.stderr
