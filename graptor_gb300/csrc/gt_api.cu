@@ -306,7 +306,7 @@ struct gt_problem {
   int schedule = 1;            // 1: p / pbar half of the primal update beside the projectors; 0: one update after
                                // them; 2: the p / pbar half fused into the next iteration's dual kernel
   bool schedule_set = false;   // chosen by gt_set_schedule (the autotuner leaves it)
-  bool small = false;          // iterations in two launches (launch_small), chosen by the autotuner
+  bool small = false;          // schedule 3: iterations in two launches (launch_small); `schedule` is 1 then
   long long iters = 0;
   bool has_data = false;
   double lsqr = 0;             // > 0: step-size constant of a variant (two-resolution solver: 36)
@@ -685,9 +685,11 @@ int gt_launches_per_iteration(const gt_problem *p) {
 
 int gt_set_schedule(gt_problem *p, int schedule) {
   if (!p) return set_err(GT_ERR_ARG, "null argument");
-  if (schedule < 0 || schedule > 2) return set_err(GT_ERR_ARG, "schedule must be 0, 1 or 2 (got %d)", schedule);
+  if (schedule < 0 || schedule > 3) return set_err(GT_ERR_ARG, "schedule must be 0, 1, 2 or 3 (got %d)", schedule);
   if (schedule == 2 && !fused_available(p))
     return set_err(GT_ERR_ARG, "schedule 2 needs 3-D TGV, Frobenius or uncorrelated coupling, C <= 4 and Nz even");
+  if (schedule == 3 && !gt::small_ok(p->P, p->cpl))
+    return set_err(GT_ERR_ARG, "schedule 3 needs 1, 2 or 4 slices (3 count as 4), C <= 4 and Frobenius or uncorrelated coupling");
   CK(cudaSetDevice(p->device));
   CK(cudaStreamSynchronize(p->stream));
   if (schedule == 2) {
@@ -696,9 +698,9 @@ int gt_set_schedule(gt_problem *p, int schedule) {
   } else {
     free_fused(p);
   }
-  p->schedule = schedule;
+  p->schedule = schedule == 3 ? 1 : schedule;
   p->schedule_set = true;
-  p->small = false;
+  p->small = schedule == 3;
   if (p->g_one) { cudaGraphExecDestroy(p->g_one); p->g_one = nullptr; }
   if (p->g_chunk) { cudaGraphExecDestroy(p->g_chunk); p->g_chunk = nullptr; }
   return GT_OK;
@@ -1116,7 +1118,7 @@ int gt_set_dual_shape(gt_problem *p, int cfg) {
 
 int gt_get_dual_shape(gt_problem *p) { return p ? p->P.dual_cfg : -1; }
 
-int gt_get_schedule(gt_problem *p) { return p ? p->schedule : -1; }
+int gt_get_schedule(gt_problem *p) { return p ? (p->small ? 3 : p->schedule) : -1; }
 
 int gt_set_precise_primal(gt_problem *p, int on) {
   if (!p) return set_err(GT_ERR_ARG, "null argument");

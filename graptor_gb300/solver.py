@@ -183,7 +183,8 @@ class Problem:
     def set_schedule(self, schedule: int):
         """1: the p / pbar half of the primal update beside the projectors (default);
         0: the whole primal update after them; 2: the p / pbar half fused into the
-        next iteration's dual kernel (3-D TGV; see gt_set_schedule)."""
+        next iteration's dual kernel (3-D TGV); 3: the iteration in two launches (up
+        to 4 slices; see gt_set_schedule)."""
         L.check(L.lib().gt_set_schedule(self._h, int(schedule)))
         return self
 

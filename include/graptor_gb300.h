@@ -134,10 +134,14 @@ GT_API int gt_get_dual_shape(gt_problem *p);
  * v, w), which writes p, v, w to a second buffer set (12 floats per voxel-channel,
  * allocated by this call or the autotuner); the sets alternate within a run of
  * gt_run and every gt_run ends on the problem's own set with the state of plain
- * iterations.  The reference enqueues update_u then update_p after radon_ad
+ * iterations; 3 (1, 2 or 4 slices C Nz, 3 counting as 4, Frobenius or uncorrelated
+ * coupling, C <= 4): the iteration in two launches, the forward projection beside
+ * the dual update and the back projection inside the primal update; forcing a
+ * launch shape afterwards goes back to schedule 1.  The reference enqueues update_u then update_p after radon_ad
  * (:1194-1221); all schedules give bit-identical iterates.  The autotuner
- * (gt_set_data) times them as graph-captured iterations and keeps the fastest,
- * unless gt_set_schedule chose one; gt_get_schedule returns the current. */
+ * (gt_set_data) times 0 and 1 (from 8M voxel-channels on) or 1 and 3 (below, where 3
+ * applies) as graph-captured iterations and keeps the faster, unless
+ * gt_set_schedule chose one; gt_get_schedule returns the current. */
 GT_API int gt_set_schedule(gt_problem *p, int schedule);
 /* Precise primal mode (no counterpart in the reference, off by default).  The
  * reference stores u in float32, so a primal step smaller than half an ulp of u
