@@ -941,6 +941,11 @@ __device__ __forceinline__ bool map_thread(long long units, int S, long long &un
   return map_thread<VW>((long long)blockIdx.x, units, S, unit, sl);
 }
 
+// slices that the threads of a shape cover: with one slice per thread only the caller's, which
+// leaves the padding as it is, zero; the vector shapes run over it
+template <int VW>
+__host__ __device__ __forceinline__ int slices_of(const Dims &d) { return VW == 1 ? d.C * d.Nz : d.S; }
+
 template <int VW>
 static inline long long threads_for(long long units, int S) {
   return (VW == 8 || VW == 4) ? units * ((S + VW * 32 - 1) / (VW * 32)) * 32 : units * (S / VW);
@@ -1092,7 +1097,7 @@ __device__ __forceinline__ void fwd_body(const IterParams &P, long long bid) {
   const Dims d = P.d;
   long long unit;
   Slices<VW> sl;
-  if (!map_thread<VW>(bid, (long long)d.nd * d.nang, d.S, unit, sl)) return;
+  if (!map_thread<VW>(bid, (long long)d.nd * d.nang, slices_of<VW>(d), unit, sl)) return;
   const int b = (int)unit;
   const int j = b / d.nd, i = b - j * d.nd;
   float acc[VW];
@@ -1233,7 +1238,7 @@ __device__ __forceinline__ void bp_body(const IterParams &P, long long bid) {
   const Dims d = P.d;
   long long unit;
   Slices<VW> sl;
-  if (!map_thread<VW>(bid, (long long)d.N * d.N, d.S, unit, sl)) return;
+  if (!map_thread<VW>(bid, (long long)d.N * d.N, slices_of<VW>(d), unit, sl)) return;
   const int pix = (int)unit;
   float acc[VW];
   const int y = pix / d.N, x = pix - y * d.N;
@@ -2247,7 +2252,7 @@ int num_proj_configs(int S, int which) {
 
 template <int VW, int UNR, int MINB = 1>
 static void fwd_vw(const IterParams &P, int disc, cudaStream_t st) {
-  const unsigned g = blocks_for(threads_for<VW>((long long)P.d.nd * P.d.nang, P.d.S), 256);
+  const unsigned g = blocks_for(threads_for<VW>((long long)P.d.nd * P.d.nang, slices_of<VW>(P.d)), 256);
   if (disc == KL) k_fwd<KL, VW, UNR, MINB><<<g, 256, 0, st>>>(P);
   else if (disc == L2) k_fwd<L2, VW, UNR, MINB><<<g, 256, 0, st>>>(P);
   else k_fwd<DATA_NONE, VW, UNR, MINB><<<g, 256, 0, st>>>(P);
@@ -2304,7 +2309,7 @@ cudaError_t launch_fwd(const IterParams &P, int disc, cudaStream_t st) {
 
 template <int VW, int AU, int UA = 2>
 static void bp_vw(const IterParams &P, cudaStream_t st) {
-  k_bp<VW, AU, UA><<<blocks_for(threads_for<VW>((long long)P.d.N * P.d.N, P.d.S), 256), 256, 0, st>>>(P);
+  k_bp<VW, AU, UA><<<blocks_for(threads_for<VW>((long long)P.d.N * P.d.N, slices_of<VW>(P.d)), 256), 256, 0, st>>>(P);
 }
 
 // default back-projection shape (no autotuning).  256^2 and smaller, us of k_bp_tap with
@@ -2429,7 +2434,7 @@ long long batch_blocks(const Dims &d, int ph) {
   const int sh = batch_shape(d);
   auto proj = [&](long long units) {
     return blocks_for(sh == 2 ? threads_for<8>(units, d.S) : sh == 1 ? threads_for<4>(units, d.S)
-                                                                     : threads_for<1>(units, d.S), 256);
+                                                                     : threads_for<1>(units, slices_of<1>(d)), 256);
   };
   switch (ph) {
     case 0: return blocks_for((long long)d.N * d.N * d.Nz, 256);
