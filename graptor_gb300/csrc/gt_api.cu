@@ -31,9 +31,9 @@ cudaError_t launch_bp(const IterParams &P, cudaStream_t st);
 cudaError_t launch_update(const IterParams &P, int tgv, cudaStream_t st, int part);
 bool small_ok(const IterParams &P, int cpl);
 cudaError_t launch_small(const IterParams &P, int disc, int tgv, int cpl, cudaStream_t st);
-cudaError_t launch_radon(const float *img, float *sino, const float4 *ofs, int N, int nd, int nang, int S,
+cudaError_t launch_radon(const float *img, float *sino, const float4 *ofs, int N, int nd, int nang, int S, int ld,
                          cudaStream_t st);
-cudaError_t launch_radon_ad(const float *sino, float *img, const float4 *ofs, int N, int nd, int nang, int S,
+cudaError_t launch_radon_ad(const float *sino, float *img, const float4 *ofs, int N, int nd, int nang, int S, int ld,
                             cudaStream_t st);
 cudaError_t launch_transpose(const float *in, float *out, int rows, int cols, int ld_in, int ld_out,
                              cudaStream_t st);
@@ -879,7 +879,7 @@ int gt_set_data(gt_problem *p, const float *f_host, int make_feasible) {
     // (R 1 <= 0) are zeroed in every slice.  ku is free scratch here.
     float *ones = p->stage, *r1 = p->ku;
     CK(gt::fill_f32(ones, (size_t)d.N * d.N, 1.f, p->stream));
-    CK(gt::launch_radon(ones, r1, p->ofs, d.N, d.nd, d.nang, 1, p->stream));
+    CK(gt::launch_radon(ones, r1, p->ofs, d.N, d.nd, d.nang, 1, 1, p->stream));
     CK(gt::launch_feasible(p->f, r1, nb1, d.S, p->stream));
   }
   // operator norm (radon_normest, 3-D :1018-1030): injected, or FP64 power iteration
@@ -1061,14 +1061,15 @@ int gt_dual_from_primal_ex(gt_problem *p, int flags, float empty_weight) {
   const float cap = (flags & GT_DUAL_CAP100) ? 100.f : ((flags & GT_DUAL_CAP10) ? 10.f : 0.f);
   CK(cudaSetDevice(p->device));
   // K u into the ku buffer (the next iteration's forward projection overwrites it)
-  CK(gt::launch_radon(p->u, p->ku, p->ofs, p->d.N, p->d.nd, p->d.nang, p->d.S, p->stream));
+  CK(gt::launch_radon(p->u, p->ku, p->ofs, p->d.N, p->d.nd, p->d.nang, p->Sr, p->d.S, p->stream));
   if ((flags & GT_DUAL_REPAIR) && p->disc == GT_KL) {
     // lift u along rays with data that the image misses: u, ubar += R^T r (stage holds
     // the image-sized correction), then project again
     CK(gt::launch_missed_rays(p->ku, p->f, p->ku, (long long)p->d.nbin, p->d.N, p->stream));
-    CK(gt::launch_radon_ad(p->ku, p->stage, p->ofs, p->d.N, p->d.nd, p->d.nang, p->d.S, p->stream));
+    if (p->d.S != p->Sr) CK(cudaMemsetAsync(p->stage, 0, sizeof(float) * p->d.vol, p->stream));  // the padding
+    CK(gt::launch_radon_ad(p->ku, p->stage, p->ofs, p->d.N, p->d.nd, p->d.nang, p->Sr, p->d.S, p->stream));
     CK(gt::launch_add2(p->u, p->ubar, p->stage, (long long)p->d.vol, p->stream));
-    CK(gt::launch_radon(p->u, p->ku, p->ofs, p->d.N, p->d.nd, p->d.nang, p->d.S, p->stream));
+    CK(gt::launch_radon(p->u, p->ku, p->ofs, p->d.N, p->d.nd, p->d.nang, p->Sr, p->d.S, p->stream));
   }
   if (flags & GT_DUAL_NO_RESET) return GT_OK;  // only the lift
   CK(gt::launch_lambda_fixed(p->lam, p->ku, p->f, p->mu64, (long long)p->d.nd * p->d.nang, p->d.S, p->d.Nz, p->disc,
@@ -1392,7 +1393,8 @@ static int run_projector(bool forward, const float *in, float *out, const double
   CK(cudaMalloc(&ofs, sizeof(float4) * nang));
   cudaError_t e = cudaMemcpyAsync(ofs, t32.data(), sizeof(float4) * nang, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess)
-    e = forward ? gt::launch_radon(in, out, ofs, N, nd, nang, S, st) : gt::launch_radon_ad(in, out, ofs, N, nd, nang, S, st);
+    e = forward ? gt::launch_radon(in, out, ofs, N, nd, nang, S, S, st)
+                : gt::launch_radon_ad(in, out, ofs, N, nd, nang, S, S, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   cudaFree(ofs);
   if (e != cudaSuccess) return cuda_err(e, forward ? "radon" : "radon_ad", __LINE__);
@@ -1996,10 +1998,10 @@ int gt_subs_set_data(gt_subs *s, const float *f0, const float *f1, int make_feas
     float *ones = s->stage, *r1 = s->scratch;
     CK(gt::fill_f32(ones, (size_t)s->N * s->N, 1.f, p->stream));
     if (s->C0) {
-      CK(gt::launch_radon(ones, r1, s->ofs0, s->N, nd0, s->nang0, 1, p->stream));
+      CK(gt::launch_radon(ones, r1, s->ofs0, s->N, nd0, s->nang0, 1, 1, p->stream));
       CK(gt::launch_feasible(s->f0, r1, s->nang0 * nd0, ld0, p->stream));
     }
-    CK(gt::launch_radon(ones, r1, s->ofs1, s->N, nd0, s->nang1, 1, p->stream));
+    CK(gt::launch_radon(ones, r1, s->ofs1, s->N, nd0, s->nang1, 1, 1, p->stream));
     std::vector<float> mask((size_t)s->nang1 * nd0);
     CK(cudaMemcpyAsync(mask.data(), r1, 4 * mask.size(), cudaMemcpyDeviceToHost, p->stream));
     CK(cudaStreamSynchronize(p->stream));

@@ -1421,30 +1421,31 @@ __global__ void __launch_bounds__(256) k_update(const IterParams P) {
 }
 
 // ===========================================================================
-// standalone projectors
+// standalone projectors: S slices of fields with ld values per pixel and bin (the values past
+// S are left as they are)
 // ===========================================================================
 template <int VW>
 __global__ void k_radon(const float *__restrict__ img, float *__restrict__ sino, const float4 *__restrict__ ofs,
-                        int N, int nd, int nang, int S) {
+                        int N, int nd, int nang, int S, int ld) {
   long long unit;
   Slices<VW> sl;
   if (!map_thread<VW>((long long)nd * nang, S, unit, sl)) return;
   const int b = (int)unit, j = b / nd, i = b - j * nd;
   float acc[VW];
-  radon_ray<VW>(img, S, N, __ldg(ofs + j), i, sl, acc);
-  sl.store(sino + (size_t)b * S, acc);
+  radon_ray<VW>(img, ld, N, __ldg(ofs + j), i, sl, acc);
+  sl.store(sino + (size_t)b * ld, acc);
 }
 
 template <int VW>
 __global__ void k_radon_ad(const float *__restrict__ sino, float *__restrict__ img, const float4 *__restrict__ ofs,
-                           int N, int nd, int nang, int S) {
+                           int N, int nd, int nang, int S, int ld) {
   long long unit;
   Slices<VW> sl;
   if (!map_thread<VW>((long long)N * N, S, unit, sl)) return;
   const int pix = (int)unit, y = pix / N, x = pix - y * N;
   float acc[VW];
-  radon_ad_pixel<VW>(sino, S, nd, nang, ofs, (float)x, (float)y, sl, acc);
-  sl.store(img + (size_t)pix * S, acc);
+  radon_ad_pixel<VW>(sino, ld, nd, nang, ofs, (float)x, (float)y, sl, acc);
+  sl.store(img + (size_t)pix * ld, acc);
 }
 
 // out[c][r] = in[r][c]: host layout [S][X] <-> device layout [X][S], 32x32 tiles,
@@ -2527,23 +2528,23 @@ static int proj_width(const void *a, const void *b, int S) {
   return vw;
 }
 
-cudaError_t launch_radon(const float *img, float *sino, const float4 *ofs, int N, int nd, int nang, int S,
+cudaError_t launch_radon(const float *img, float *sino, const float4 *ofs, int N, int nd, int nang, int S, int ld,
                          cudaStream_t st) {
   const long long units = (long long)nd * nang;
   const int vw = proj_width(img, sino, S);
-  if (vw == 8) k_radon<8><<<blocks_for(threads_for<8>(units, S), 256), 256, 0, st>>>(img, sino, ofs, N, nd, nang, S);
-  else if (vw == 2) k_radon<2><<<blocks_for(threads_for<2>(units, S), 256), 256, 0, st>>>(img, sino, ofs, N, nd, nang, S);
-  else k_radon<1><<<blocks_for(threads_for<1>(units, S), 256), 256, 0, st>>>(img, sino, ofs, N, nd, nang, S);
+  if (vw == 8) k_radon<8><<<blocks_for(threads_for<8>(units, S), 256), 256, 0, st>>>(img, sino, ofs, N, nd, nang, S, ld);
+  else if (vw == 2) k_radon<2><<<blocks_for(threads_for<2>(units, S), 256), 256, 0, st>>>(img, sino, ofs, N, nd, nang, S, ld);
+  else k_radon<1><<<blocks_for(threads_for<1>(units, S), 256), 256, 0, st>>>(img, sino, ofs, N, nd, nang, S, ld);
   return cudaGetLastError();
 }
 
-cudaError_t launch_radon_ad(const float *sino, float *img, const float4 *ofs, int N, int nd, int nang, int S,
+cudaError_t launch_radon_ad(const float *sino, float *img, const float4 *ofs, int N, int nd, int nang, int S, int ld,
                             cudaStream_t st) {
   const long long units = (long long)N * N;
   const int vw = proj_width(img, sino, S);
-  if (vw == 8) k_radon_ad<8><<<blocks_for(threads_for<8>(units, S), 256), 256, 0, st>>>(sino, img, ofs, N, nd, nang, S);
-  else if (vw == 2) k_radon_ad<2><<<blocks_for(threads_for<2>(units, S), 256), 256, 0, st>>>(sino, img, ofs, N, nd, nang, S);
-  else k_radon_ad<1><<<blocks_for(threads_for<1>(units, S), 256), 256, 0, st>>>(sino, img, ofs, N, nd, nang, S);
+  if (vw == 8) k_radon_ad<8><<<blocks_for(threads_for<8>(units, S), 256), 256, 0, st>>>(sino, img, ofs, N, nd, nang, S, ld);
+  else if (vw == 2) k_radon_ad<2><<<blocks_for(threads_for<2>(units, S), 256), 256, 0, st>>>(sino, img, ofs, N, nd, nang, S, ld);
+  else k_radon_ad<1><<<blocks_for(threads_for<1>(units, S), 256), 256, 0, st>>>(sino, img, ofs, N, nd, nang, S, ld);
   return cudaGetLastError();
 }
 
