@@ -722,6 +722,7 @@ static int create_problem(const gt_desc &D, int Sr, int S, gt_problem **out) {
   p->alpha0 = D.alpha0; p->alpha1 = D.alpha1; p->ne_in = D.normest;
   p->autotune = D.autotune != 0;
   p->mu.assign(D.mu, D.mu + D.C);
+  p->mu.resize(D.C + kMuPad, 1.0);
   angle_table(D.angles, D.N, D.nd, D.nang, p->ofs64h);
 
   auto fail = [&](int rc) { gt_problem_destroy(p); return rc; };
@@ -905,10 +906,7 @@ int gt_set_data(gt_problem *p, const float *f_host, int make_feasible) {
     const int rc = upload_mu_eff(p);
     if (rc) return rc;
   }
-  std::vector<double> m64(p->mu);
-  m64.resize(d.C + kMuPad, 1.0);
-  CK(cudaMemcpyAsync(p->mu64, m64.data(), sizeof(double) * m64.size(), cudaMemcpyHostToDevice, p->stream));
-  CK(cudaStreamSynchronize(p->stream));  // m64 is a host buffer
+  CK(cudaMemcpyAsync(p->mu64, p->mu.data(), sizeof(double) * p->mu.size(), cudaMemcpyHostToDevice, p->stream));
   p->P.ne64 = p->ne;
   // pick the projector launch shapes (uses lambda / ku / kstar as scratch: they are reset below)
   {
