@@ -23,6 +23,7 @@ import argparse
 import contextlib
 import io
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -73,12 +74,35 @@ def algorithmic_bytes(V, Sb):
             "k_dual_fused": 100 * V}
 
 
-def gather_bytes(N, nang, S):
-    """Bytes a projector moves through L1 per launch: every (pixel, angle) pair
-    has two interpolation taps of S floats (k_bp reads two sinogram bins per pixel
-    and angle; k_fwd reads two image pixels per ray and row, about as many pairs).
-    The model counts every pair as inside the detector, an upper bound."""
-    return 2 * 4 * N * N * nang * S
+def gather_bytes(kernel, shape, N, nd, angles, S):
+    """Bytes that one launch of a projector ("k_fwd" or "k_bp", launch shape as in
+    gt_set_tuning) gathers through L1: S floats per load.  One load per pixel and ray, or
+    per pixel and detector tap, of which a pixel has two per angle inside the detector;
+    the pair kernels (forward 8, 10, 11) load a pixel once for both rays of a pair, the row
+    tiles (back 9, 18, 19) each bin once for the four pixels of a tile whose bins step by
+    0 or 1 in one direction."""
+    x = np.arange(N, dtype=np.float64)
+    loads = 0
+    for a in np.asarray(angles, np.float64):
+        X, Y = math.cos(a), math.sin(a)
+        t = x[None, :] * X + x[:, None] * Y + ((nd - 1) / 2 - (X + Y) * (N - 1) / 2)
+        lo = np.floor(t).astype(np.int64)
+        inside = (t > -1) & (t < nd)
+        first, second = inside & (lo >= 0), inside & (lo <= nd - 2)  # which of a pixel's two bins exist
+        taps = first.astype(np.int64) + second
+        if kernel == "k_fwd" and shape in (8, 10, 11):
+            loads += int((taps - (first & second & (lo % 2 == 0))).sum())
+        elif kernel == "k_bp" and shape in (9, 18, 19):
+            pad = -N % 4
+            def tiles(v):
+                return np.pad(v, ((0, 0), (0, pad)), mode="edge").reshape(N, -1, 4)
+            step = np.diff(tiles(lo), axis=2)
+            whole = tiles(taps).min(axis=2) == 2
+            whole &= ((step == 0) | (step == 1)).all(axis=2) | ((step == 0) | (step == -1)).all(axis=2)
+            loads += int(np.where(whole, 2 + np.abs(step).sum(axis=2), tiles(taps).sum(axis=2)).sum())
+        else:
+            loads += int(taps.sum())
+    return 4 * S * loads
 
 
 # L1 data path: 128 B per clock per SM, 152 SMs, 2.07 GHz maximum SM clock (nominal)
@@ -317,7 +341,9 @@ def run_ours(args, rank, world, local):
     top = max(kms, key=kms.get)
     hbm, peak_kind = peaks()
     achieved = alg[top] / (kms[top] / 1e3) / 1e9
-    traffic = ncu_traffic(top)
+    tuning = prob.tuning
+    shape = tuning[{"k_fwd": "fwd_cfg", "k_bp": "bp_cfg"}.get(top, "dual_cfg")]
+    traffic = ncu_traffic(top, shape)
     it_ms = ms / args.steps
     solver_gbs = alg["iteration"] / (it_ms / 1e3) / 1e9
     launches = prob.launches_per_iteration * args.steps
@@ -326,12 +352,11 @@ def run_ours(args, rank, world, local):
             "algorithmic_bytes_per_launch": alg[top], "ms_per_launch": kms[top]}
     if top in ("k_fwd", "k_bp"):
         # a projector gathers from L2-resident operands: its limit is the L1 data path
-        gb = gather_bytes(N, nang, S)
+        gb = gather_bytes(top, shape, N, N, ang, S)
         roof["l1"] = {"achieved": gb / (kms[top] / 1e3) / 1e9, "peak": L1_NOMINAL_GBS, "unit": "GB/s",
                       "frac": gb / (kms[top] / 1e3) / 1e9 / L1_NOMINAL_GBS, "peak_source": "nominal",
                       "gather_bytes_per_launch": gb}
     ne = prob.scalars["normest"]
-    tuning = prob.tuning
     prob.close()
 
     # ---- end to end through the reference-facing entry point, host buffers
@@ -625,7 +650,6 @@ def time_to_gap_compare(rank, world, local, nseeds, weights=None, N=None, Nz=Non
     keep the reference's steps and float32 u, the regime the network was trained
     on): the primal weight of the step pair and u held as two floats (needed below
     the float32 plateau of the gap, a few 1e-4)."""
-    import math
 
     import torch
 
@@ -779,14 +803,15 @@ def run_warmstart(args, rank, world, local):
             "fell_back_to_cold": r["fell_back_to_cold"], "gpu_launches": r["gpu_launches"]}
 
 
-def ncu_traffic(kernel):
-    """DRAM bytes per launch of `kernel` from the committed ncu summary, if present."""
+def ncu_traffic(kernel, shape):
+    """DRAM bytes per launch of `kernel` from the committed ncu summary, if it holds the
+    launch shape that runs (the update's halves have none)."""
     path = os.path.join(ROOT, "profiles", "ncu_traffic.txt")
     try:
         for line in open(path):
             parts = line.split()
-            if len(parts) >= 2 and parts[0] == kernel and not line.startswith("#"):
-                return float(parts[1])
+            if len(parts) >= 3 and parts[0] == kernel and parts[1] == str(shape) and not line.startswith("#"):
+                return float(parts[2])
     except OSError:
         pass
     return None
