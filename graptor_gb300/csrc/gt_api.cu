@@ -73,7 +73,7 @@ int default_fwd_shape(int S);
 long long tap_entries(int N, int nd, int nang);
 cudaError_t launch_tap_fill(const float4 *ofs, int N, int nd, int nang, unsigned *hdr, float4 *frac, cudaStream_t st);
 int default_bp_shape(int S);
-int num_proj_configs(int S, int which);
+int num_proj_configs(int S);
 bool dual_z2_ok(const IterParams &P, int tgv, int cpl);
 int num_dual_configs(const IterParams &P);
 bool dual_cl_ok(const IterParams &P, int cpl);
@@ -140,7 +140,9 @@ constexpr int kPairSlices = 80;
 
 // Slices per pixel in memory.  The vector kernels (projectors, primal update) move four
 // slices per load, so a count that is not a multiple of 4 is padded with zero slices,
-// which every kernel leaves zero.  One and two slices stay as they are.
+// which every kernel leaves zero (TGV, 71 angles, us an iteration without and with padding: 64^2 x
+// 3 29 / 14, 5 29 / 22, 9 32 / 26; 256^2 x 5 147 / 92, 9 160 / 121, 17 236 / 161; 1024^2 x 5 1333 / 1062, the
+// projectors' part of it).  One and two slices stay as they are.
 int padded_slices(int S) { return S <= 2 ? S : (S + 3) & ~3; }
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -236,7 +238,7 @@ int build_rays(gt::IterParams &P, ProjTables &t, int *scratch, cudaStream_t st) 
 
 // optional (forward shapes 8, 10 and 11): without room for it those shapes use the ray table
 int build_pairs(gt::IterParams &P, ProjTables &t, int *scratch, cudaStream_t st) {
-  if (t.pairs || !P.ray_start) return GT_OK;
+  if (t.pairs) return GT_OK;
   const gt::Dims &d = P.d;
   long long *start = nullptr;
   int2 *ent = nullptr;
@@ -546,8 +548,8 @@ int autotune(gt_problem *p) {
   // every dual shape is tuned: at 256^2 x 60 x 4 the order of the shapes timed
   // alone is their order inside the overlapped iteration
   constexpr int kMaxCfg = 32;
-  const int nc[3] = {std::min(kMaxCfg, gt::num_proj_configs(p->d.S, 0)),
-                     std::min(kMaxCfg, gt::num_proj_configs(p->d.S, 1)),
+  const int nc[3] = {std::min(kMaxCfg, gt::num_proj_configs(p->d.S)),
+                     std::min(kMaxCfg, gt::num_proj_configs(p->d.S)),
                      std::min(kMaxCfg, gt::num_dual_configs(p->P))};
   // Shapes left out of the tuning (all stay selectable by gt_set_tuning), to bound
   // its time on batches of many distinct problems: of the back projection all but the
@@ -1081,9 +1083,9 @@ void *gt_problem_stream(gt_problem *p) { return p ? (void *)p->stream : nullptr;
 
 int gt_set_tuning(gt_problem *p, int fwd_cfg, int bp_cfg) {
   if (!p) return set_err(GT_ERR_ARG, "null argument");
-  const int nf = gt::num_proj_configs(p->d.S, 0), nb = gt::num_proj_configs(p->d.S, 1);
-  if (fwd_cfg < 0 || fwd_cfg >= nf || bp_cfg < 0 || bp_cfg >= nb)
-    return set_err(GT_ERR_ARG, "launch configuration out of range (%d forward, %d back-projection configurations)", nf, nb);
+  const int n = gt::num_proj_configs(p->d.S);
+  if (fwd_cfg < 0 || fwd_cfg >= n || bp_cfg < 0 || bp_cfg >= n)
+    return set_err(GT_ERR_ARG, "launch configuration out of range (%d of each projector)", n);
   CK(cudaSetDevice(p->device));
   CK(cudaStreamSynchronize(p->stream));
   if (fwd_cfg == 8 || fwd_cfg == 10 || fwd_cfg == 11) {

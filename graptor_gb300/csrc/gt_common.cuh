@@ -46,7 +46,7 @@ struct IterParams {
   int fwd_cfg, bp_cfg;   // projector launch shapes (see launch_fwd / launch_bp)
   int dual_cfg;          // 0: k_dual, 1: k_dual_z2 (where dual_z2_ok)
   const float4 *ofs;     // [nang] (X, Y, offset, Xinv)
-  const long long *ray_start;  // [nd*nang + 1] ray table offsets (null: walk rays on the fly)
+  const long long *ray_start;  // [nd*nang + 1] ray table offsets
   const int2 *ray_ent;         // (pixel, weight bits) entries of all rays
   const long long *pair_start; // [nang*ceil(nd/2) + 1] offsets of the pair table of k_fwd_pair (null: none)
   const int2 *pair_ent;        // (pixel, bits of the detector coordinate) entries of all pairs of bins

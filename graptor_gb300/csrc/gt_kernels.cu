@@ -1099,14 +1099,9 @@ __device__ __forceinline__ void fwd_body(const IterParams &P, long long bid) {
   Slices<VW> sl;
   if (!map_thread<VW>(bid, (long long)d.nd * d.nang, slices_of<VW>(d), unit, sl)) return;
   const int b = (int)unit;
-  const int j = b / d.nd, i = b - j * d.nd;
   float acc[VW];
-  if (P.ray_start) {
-    const long long r0 = __ldg(P.ray_start + b), r1 = __ldg(P.ray_start + b + 1);
-    radon_table<VW, false, UNR>(P.ubar, d.S, P.ray_ent + r0, (int)(r1 - r0), sl, acc);
-  } else {
-    radon_ray<VW>(P.ubar, d.S, d.N, __ldg(P.ofs + j), i, sl, acc);
-  }
+  const long long r0 = __ldg(P.ray_start + b), r1 = __ldg(P.ray_start + b + 1);
+  radon_table<VW, false, UNR>(P.ubar, d.S, P.ray_ent + r0, (int)(r1 - r0), sl, acc);
   const size_t q = (size_t)b * d.S;
   sl.store(P.ku + q, acc);
   if constexpr (DISC == DATA_NONE) return;
@@ -2235,9 +2230,9 @@ cudaError_t launch_dual_fused(const IterParams &P, int tgv, int cpl, cudaStream_
 // Tunable launch shapes of the projector kernels (chosen per problem shape by the
 // autotuner in gt_api.cu), for S a multiple of 4.
 // k_fwd configs: 0..4 = (slices per lane, ray-table entries in flight) = (8, 4), (8, 8),
-// (4, 4), (4, 8), (1, 4); 12..19 = (8, 4) with registers capped for 4 resident blocks;
-// 10, 11 the pair kernel k_fwd_pair with 8 and 4 slices per lane; 9 (and 8), 5, 6 the
-// flat kernel k_fwd_flat with 4, 2 and 1 slices per thread; 7 the staged kernel (S = 4,
+// (4, 4), (4, 8), (1, 4); 12..19 all (8, 4) with registers capped for 4 resident blocks;
+// 10, 11 the pair kernel k_fwd_pair with 8 and 4 slices per lane, 8 k_fwd_pair_flat; 9, 5, 6
+// the flat kernel k_fwd_flat with 4, 2 and 1 slices per thread; 7 the staged kernel (S = 4,
 // else 9) (gt_fwd.cu).
 // k_bp configs 0..8 = (slices per lane, angles per step) of the one-pixel kernel = (8, 2),
 // (8, 4), (4, 2), (4, 4), (8, 1), (4, 1), (8, 2), (4, 2), (1, 1); 16 and 17 are 4 with its
@@ -2245,9 +2240,8 @@ cudaError_t launch_dual_fused(const IterParams &P, int tgv, int cpl, cudaStream_
 // the row-tile kernel k_bp_tap with 8, 4 and 2 slices per lane, 10 (and 13), 11, 12 the
 // flat kernel k_bp_flat with 4, 2 and 1 slices per thread (12 with S = 4: the staged kernel;
 // gt_proj.cu).
-// Otherwise one fixed shape.
-int num_proj_configs(int S, int which) {
-  (void)which;
+// Otherwise (1 and 2 slices, or no room for the padding) one fixed shape.
+int num_proj_configs(int S) {
   return S % 4 != 0 ? 1 : 20;
 }
 
@@ -2267,12 +2261,16 @@ cudaError_t launch_bp_tap(const IterParams &P, int vw, cudaStream_t st);
 cudaError_t launch_bp_flat(const IterParams &P, int vw, cudaStream_t st);
 cudaError_t launch_bp_staged(const IterParams &P, cudaStream_t st);
 
-// default forward shape (no autotuning).  us of k_fwd_pair with 8 / 4 slices per lane, of
-// k_fwd_pair_flat, of k_fwd_flat with 4 slices per thread and of the ray-table kernel (the best of
-// 0..4, 14): 16 slices (177^2, 45 angles) - / 70 / 34 / 24 / 33; 32 (64^2, 71) - / 20 / 14 / 10 / 16;
-// 64 (128^2, 71) - / 58 / 33 / 38 / 64; 92 (128^2, 71) 83 / 61 / 53 / 61 / 68; 240 (256^2, 71) 333 / 360
-// / 359 / 426 / 386; 384 (512^2, 141) 5044 / 4404 / - / 8130 / 7795 (there 8 per lane leave a quarter
-// of the lanes idle).
+// default forward shape (no autotuning: gt_desc.autotune = 0, and the groups of the two-resolution
+// solver).  us of k_fwd_flat with 4 slices per thread (9) / k_fwd_pair_flat (8) / k_fwd_pair with 4 (11)
+// and 8 (10) slices per lane, 71 angles: 64^2 x 32 10 / 14 / 20 / -; 128^2 x 64 45 / 50 / 72 / 97; 80
+// 57 / 51 / 74 / 97; 96 61 / 65 / 74 / 98; 128 71 / 71 / 74 / 96; 160 90 / 80 / 111 / 98; 192 102 / 97 / 110
+// / 98; 240 126 / 110 / 113 / 101; 256^2 x 80 179 / 152 / 211 / 327; 128 237 / 208 / 215 / 329; 160 302 / 259
+// / 375 / 336; 192 348 / 302 / 378 / 338; 240 443 / 373 / 384 / 350; 512^2 x 384, 141 angles 8130 / - / 4404 /
+// 5044 (there 8 per lane leave a quarter of the lanes idle).  The ray-table kernel never wins (386 us at
+// 256^2 x 240).  Up to 92 slices the flat kernel, which needs no pair table; then the pair kernel, with
+// 8 per lane from 192 on unless its last chunk is mostly idle.  8 would be up to 30 % faster from 80 to 192
+// slices; it is left to the tuner (up to 128).
 int default_fwd_shape(int S) {
   if (S % 4 != 0) return 0;  // the one shape (num_proj_configs)
   if (S == 4) return 7;
@@ -2284,7 +2282,7 @@ int default_fwd_shape(int S) {
 cudaError_t launch_fwd(const IterParams &P, int disc, cudaStream_t st) {
   const int S = P.d.S;
   if (S <= 2) return launch_fwd_staged(P, disc, st);
-  if (S % 4 != 0) return launch_fwd_flat(P, disc, S % 2 == 0 ? 2 : 1, st);
+  if (S % 4 != 0) return launch_fwd_flat(P, disc, S % 2 == 0 ? 2 : 1, st);  // no room for the padding
   switch (P.fwd_cfg) {
     case 1: fwd_vw<8, 8>(P, disc, st); break;
     case 2: fwd_vw<4, 4>(P, disc, st); break;
@@ -2323,7 +2321,8 @@ int default_bp_shape(int S) {
   if (S % 4 != 0) return 0;  // the one shape (num_proj_configs)
   if (S == 4) return 12;
   if (S <= 48) return 10;
-  if (S <= 64) return 9;  // alone as k_bp_flat, beside other work faster (three at once: 22 us each against 28)
+  // alone as k_bp_flat; with several problems at once, as in batches, faster (three: 22 us each against 28)
+  if (S <= 64) return 9;
   const int w8 = (S + 255) / 256 * 256, w4 = (S + 127) / 128 * 128;
   return S >= 192 && w8 <= w4 + w4 / 8 ? 18 : 19;
 }
@@ -2331,7 +2330,7 @@ int default_bp_shape(int S) {
 cudaError_t launch_bp(const IterParams &P, cudaStream_t st) {
   const int S = P.d.S;
   if (S <= 2) return launch_bp_staged(P, st);
-  if (S % 4 != 0) return launch_bp_flat(P, S % 2 == 0 ? 2 : 1, st);
+  if (S % 4 != 0) return launch_bp_flat(P, S % 2 == 0 ? 2 : 1, st);  // no room for the padding
   switch (P.bp_cfg) {
     case 0: bp_vw<8, 2>(P, st); break;
     case 1: bp_vw<8, 4>(P, st); break;

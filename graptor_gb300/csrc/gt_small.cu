@@ -15,9 +15,10 @@
 // gt_update.cuh), so the iterates are identical.  K* lambda is not written.
 //
 // 128^2 x 1 slice, 60 angles, per iteration: alone 15.3 us with separate launches, 13.9 us in
-// this form; three problems side by side 10.2 -> 7.6 us.  With more slices separate launches
-// win: a launch's blocks all hold the registers of its larger half (64^2 x 32, three problems
-// side by side: 11.9 us an iteration with separate launches, 13.4 us in this form).
+// this form; three problems at once (as slices and batches of small problems are solved) 10.2 ->
+// 7.6 us.  With more slices separate launches win there: a launch's blocks all hold the
+// registers of its larger half (64^2 x 32, three problems at once: 11.9 us an iteration with
+// separate launches, 13.4 us in this form).  The tuner times a problem alone.
 #include <cuda_runtime.h>
 
 #include "gt_common.cuh"
@@ -92,7 +93,7 @@ void bp_update_s(const IterParams &P, cudaStream_t st) {
 }  // namespace
 
 bool small_ok(const IterParams &P, int cpl) {
-  return cpl != NUCL && (P.d.S <= 2 || P.d.S == 4) && P.d.C <= 4 && P.ray_start;
+  return cpl != NUCL && (P.d.S <= 2 || P.d.S == 4) && P.d.C <= 4;
 }
 
 cudaError_t launch_small(const IterParams &P, int disc, int tgv, int cpl, cudaStream_t st) {

@@ -267,8 +267,9 @@ GT_API int gt_batch_set_active(gt_batch *b, int k, int active);
  * concurrent chains.  Mode 1 (fused): per iteration four launches, each over the
  * work units of every active member (dual update, forward projection + data
  * prox, back projection, primal update), every member with one fixed launch
- * shape; for many small problems, where per-member launches leave the GPU
- * underfilled.  Mode 1 needs every member to share the dimension, the
+ * shape.  Mode 0 is the faster one wherever measured (64 problems of up to 128^2 x 8
+ * x 4: 0.81 ms an iteration against 1.33 ms); mode 1 has four graph nodes per
+ * iteration whatever the number of members, and its shapes need no tuning.  It needs every member to share the dimension, the
  * regularisation and the coupling (Frobenius or uncorrelated, <= 8 channels);
  * it returns GT_ERR_ARG otherwise.  Iterates are identical in both modes. */
 GT_API int gt_batch_set_mode(gt_batch *b, int mode);
