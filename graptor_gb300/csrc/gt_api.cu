@@ -140,9 +140,9 @@ constexpr int kPairSlices = 80;
 
 // Slices per pixel in memory.  The vector kernels (projectors, primal update) move four
 // slices per load, so a count that is not a multiple of 4 is padded with zero slices,
-// which every kernel leaves zero (TGV, 71 angles, us an iteration without and with padding: 64^2 x
-// 3 29 / 14, 5 29 / 22, 9 32 / 26; 256^2 x 5 147 / 92, 9 160 / 121, 17 236 / 161; 1024^2 x 5 1333 / 1062, the
-// projectors' part of it).  One and two slices stay as they are.
+// which every kernel leaves zero.  TGV, 71 angles, us an iteration with the projectors for any
+// count and no padding / with the vector ones: 64^2 x 3 29 / 14, 5 29 / 22, 9 32 / 26; 256^2 x 5 147 / 92, 9
+// 160 / 121, 17 236 / 161; 1024^2 x 5 1333 / 1062.  One and two slices stay as they are.
 int padded_slices(int S) { return S <= 2 ? S : (S + 3) & ~3; }
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
