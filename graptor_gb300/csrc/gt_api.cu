@@ -69,10 +69,12 @@ cudaError_t launch_ray_fill(const float4 *ofs, int N, int nd, int nang, const lo
 cudaError_t launch_pair_count(const float4 *ofs, int N, int nd, int nang, int *count, cudaStream_t st);
 cudaError_t launch_pair_fill(const float4 *ofs, int N, int nd, int nang, const long long *start, int2 *ent,
                              cudaStream_t st);
-int default_fwd_shape(int S);
+int default_fwd_shape(const Dims &d);
+long long flat_rays(const Dims &d);
+long long flat_pixels(const Dims &d);
 long long tap_entries(int N, int nd, int nang);
 cudaError_t launch_tap_fill(const float4 *ofs, int N, int nd, int nang, unsigned *hdr, float4 *frac, cudaStream_t st);
-int default_bp_shape(int S);
+int default_bp_shape(const Dims &d);
 int num_proj_configs(int S);
 bool dual_z2_ok(const IterParams &P, int tgv, int cpl);
 int num_dual_configs(const IterParams &P);
@@ -558,18 +560,20 @@ int autotune(gt_problem *p) {
   // never do); of the forward projection all but the pair shapes (10, 11, 8), the flat ones
   // (9, 5) and the staged one (7), likewise (times at default_fwd_shape).
   const int S = p->d.S;
+  // the flat shapes with more slices where the others leave the GPU idle
+  const bool flat_f = S <= 128 || gt::flat_rays(p->d) < (1 << 19), flat_b = S <= 128 || gt::flat_pixels(p->d) < (1 << 18);
   auto skipped = [&](int which, int c) {
     if (which == 0)
-      return !((c == 10 && S > 128) || (c == 11 && S >= kPairSlices) || (c == 8 && S >= kPairSlices && S <= 128) ||
-               (c == 9 && S <= 128) || (c == 5 && S <= 32) || (c == 7 && S == 4));
+      return !((c == 10 && S > 128) || (c == 11 && S >= kPairSlices) || (c == 8 && S >= kPairSlices && flat_f) ||
+               (c == 9 && flat_f) || (c == 5 && S <= 32) || (c == 7 && S == 4));
     if (which == 1)
       return !((c == 18 && S >= 96) || (c == 19 && S >= 36) || (c == 9 && S >= 16 && S <= 128) ||
-               (c == 10 && S <= 128) || (c == 11 && S <= 16) || (c == 12 && S == 4));
+               (c == 10 && flat_b) || (c == 11 && S <= 16) || (c == 12 && S == 4));
     return false;
   };
   if (!p->schedule_set) p->small = false;
-  p->P.fwd_cfg = gt::default_fwd_shape(S);
-  p->P.bp_cfg = gt::default_bp_shape(S);
+  p->P.fwd_cfg = gt::default_fwd_shape(p->d);
+  p->P.bp_cfg = gt::default_bp_shape(p->d);
   p->P.dual_cfg = gt::default_dual_shape(p->P, p->cpl);
   if ((nc[0] <= 1 && nc[1] <= 1 && nc[2] <= 1) || !p->autotune) return GT_OK;
   const TuneKey key{p->d.dim, p->d.N, p->d.S, p->d.nd, p->d.nang, p->disc, p->d.C, p->d.Nz, p->reg, p->cpl};
@@ -1933,8 +1937,8 @@ static int create_subs(const gt_subs_desc *D, bool pad, gt_subs **out) {
     Q.npix = p->P.npix;
     Q.d.vol = NN * ld; Q.d.nbin = (size_t)nd0 * nang * ld;
     Q.ofs = ofs;
-    Q.fwd_cfg = gt::default_fwd_shape(ld);
-    Q.bp_cfg = gt::default_bp_shape(ld);
+    Q.fwd_cfg = gt::default_fwd_shape(Q.d);
+    Q.bp_cfg = gt::default_bp_shape(Q.d);
     int *scratch = (int *)s->scratch;
     int r = GT_OK;
     if (inner) {  // the inner problem's own geometry: its tables

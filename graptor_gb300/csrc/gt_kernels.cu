@@ -2261,6 +2261,10 @@ cudaError_t launch_bp_tap(const IterParams &P, int vw, cudaStream_t st);
 cudaError_t launch_bp_flat(const IterParams &P, int vw, cudaStream_t st);
 cudaError_t launch_bp_staged(const IterParams &P, cudaStream_t st);
 
+// threads of the flat kernels with 4 slices each
+long long flat_rays(const Dims &d) { return (long long)d.nd * d.nang * (d.S / 4); }
+long long flat_pixels(const Dims &d) { return (long long)d.N * d.N * (d.S / 4); }
+
 // default forward shape (no autotuning: gt_desc.autotune = 0, and the groups of the two-resolution
 // solver).  us of k_fwd_flat with 4 slices per thread (9) / k_fwd_pair_flat (8) / k_fwd_pair with 4 (11)
 // and 8 (10) slices per lane, 71 angles: 64^2 x 32 10 / 14 / 20 / -; 128^2 x 64 45 / 50 / 72 / 97; 80
@@ -2271,12 +2275,19 @@ cudaError_t launch_bp_staged(const IterParams &P, cudaStream_t st);
 // 256^2 x 240).  Up to 92 slices the flat kernel, which needs no pair table; then the pair kernel, with
 // 8 per lane from 192 on unless its last chunk is mostly idle.  8 would be up to 30 % faster from 80 to 192
 // slices; it is left to the tuner (up to 128).
-int default_fwd_shape(int S) {
+// Small problems with many slices (a tilt series of a small image): a warp per pair of bins leaves most
+// of the GPU idle, so below 2^17 threads of the flat kernel (one block of 64 on every SM, some
+// 13 times over) that one, up to 2^18 where the pair kernel's chunks of 128 slices are not
+// nearly filled, and 8 slices per lane only from 3000 warps on: 20^2 x 192, 40 angles 8 (16 with 10), 48^2 x 256,
+// 40 angles 18 (29 with 10), 96^2 x 192, 40 angles 36 / 42 with 11 / 53 with 10; 48^2 x 452, 100 angles 53 / 49 / 43.
+int default_fwd_shape(const Dims &d) {
+  const int S = d.S;
   if (S % 4 != 0) return 0;  // the one shape (num_proj_configs)
   if (S == 4) return 7;
-  if (S <= 92) return 9;
-  const int w8 = (S + 255) / 256 * 256, w4 = (S + 127) / 128 * 128;
-  return S >= 192 && w8 <= w4 + w4 / 8 ? 10 : 11;
+  const int c4 = (S + 127) / 128, c8 = (S + 255) / 256;
+  const long long flat = flat_rays(d);
+  if (S <= 92 || flat < (1 << 17) || (flat < (1 << 18) && 10 * S < 1024 * c4)) return 9;
+  return S >= 192 && 16 * c8 <= 9 * c4 && (long long)(d.nd + 1) / 2 * d.nang * c8 >= 3000 ? 10 : 11;
 }
 
 cudaError_t launch_fwd(const IterParams &P, int disc, cudaStream_t st) {
@@ -2317,14 +2328,18 @@ static void bp_vw(const IterParams &P, cudaStream_t st) {
 // 64 (128^2, 71) 74 / 42 / 36 / 35; 92 (128^2, 71) 74 / 43 / 62 / 50; 240 (256^2, 71)
 // 213 / 242 / 361 / 440; 384 (512^2, 141) 2912 / 2628 / 4050 / 6856 (there 8 per lane leave
 // a quarter of the lanes idle).
-int default_bp_shape(int S) {
+// Below 2^18 threads of the flat kernel (64^2 x 252) a warp per row tile leaves the GPU idle: at 40 angles 20^2 x
+// 192 10 us with the flat kernel, 22 with 4, 27 with 8 slices per lane; 64^2 x 128 14 / 23 / 26; 96^2 x 92 23 / 25 / 29;
+// at 2^18 and above 64^2 x 452 35 / 29 / 29; 96^2 x 192 35 / 27 / 29; 128^2 x 92 31 / 27 / 47.
+int default_bp_shape(const Dims &d) {
+  const int S = d.S;
   if (S % 4 != 0) return 0;  // the one shape (num_proj_configs)
   if (S == 4) return 12;
-  if (S <= 48) return 10;
+  if (S <= 48 || flat_pixels(d) < (1 << 18)) return 10;
   // alone as k_bp_flat; with several problems at once, as in batches, faster (three: 22 us each against 28)
   if (S <= 64) return 9;
-  const int w8 = (S + 255) / 256 * 256, w4 = (S + 127) / 128 * 128;
-  return S >= 192 && w8 <= w4 + w4 / 8 ? 18 : 19;
+  const int c4 = (S + 127) / 128, c8 = (S + 255) / 256;
+  return S >= 192 && 16 * c8 <= 9 * c4 && (long long)d.N * ((d.N + 3) / 4) * c8 >= 3000 ? 18 : 19;
 }
 
 cudaError_t launch_bp(const IterParams &P, cudaStream_t st) {

@@ -89,3 +89,27 @@ def test_a_chosen_schedule_does_not_stand_for_later_problems():
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     assert r.stderr.count("two launches:") == 1, r.stderr
+
+
+@pytest.mark.parametrize("N,nd,nang,Nz,C,fwd,bp", [
+    (19, 12, 41, 53, 1, 9, 10), (13, 13, 3, 113, 4, 9, 10), (20, 40, 11, 65, 2, 9, 10),  # small images, many slices
+    (64, 64, 20, 92, 1, 9, 10), (64, 64, 20, 64, 3, 9, 10),  # below 2^18 threads per projector
+    (64, 65, 64, 64, 2, 11, 10), (72, 72, 60, 48, 4, 9, 10), (64, 70, 84, 64, 4, 11, 19),  # above one or both
+    (64, 70, 88, 64, 4, 10, 19), (112, 112, 10, 48, 4, 9, 18)])  # 3000 warps with 8 slices per lane
+def test_default_shapes_of_small_images_with_many_slices(N, nd, nang, Nz, C, fwd, bp):
+    """Both sides of the lines of the default shapes: the shapes as stated there, and the iterates of the
+    default and of the tuned shapes those of the one-ray and one-pixel kernels."""
+    got = []
+    for autotune, forced in ((False, True), (False, False), (True, False)):
+        f, p = _problem(N, nd, nang, Nz, C, autotune=autotune)
+        with p:
+            p.set_data(f)
+            if forced:
+                p.set_tuning(0, 4)
+            elif not autotune:
+                assert (p.tuning["fwd_cfg"], p.tuning["bp_cfg"]) == (fwd, bp)
+            p.run(4).synchronize()
+            got.append([p.get(k) for k in ("u", "ku", "lambda")])
+    for g in got[1:]:
+        for a, b in zip(g, got[0]):
+            np.testing.assert_array_equal(a, b)
