@@ -142,10 +142,17 @@ constexpr int kPairSlices = 80;
 
 // Slices per pixel in memory.  The vector kernels (projectors, primal update) move four
 // slices per load, so a count that is not a multiple of 4 is padded with zero slices,
-// which every kernel leaves zero.  TGV, 71 angles, us an iteration with the projectors for any
-// count and no padding / with the vector ones: 64^2 x 3 29 / 14, 5 29 / 22, 9 32 / 26; 256^2 x 5 147 / 92, 9
-// 160 / 121, 17 236 / 161; 1024^2 x 5 1333 / 1062.  One and two slices stay as they are.
-int padded_slices(int S) { return S <= 2 ? S : (S + 3) & ~3; }
+// which every kernel leaves zero.  Not so in small images, whose iteration is bound by the latency of
+// its kernels, longer with four slices per thread than with one or two.  us an iteration (3-D TGV, Frobenius, one
+// channel, 5 of the 15 slices; 12, 60 angles) with the one-ray projectors and no padding / with the present ones
+// and padding / without: 10^2 x 9 8.4 / 9.9 / 7.7, 16.0 / 12.2 / 11.5; 23^2 x 15 16.1 / 17.2 / 16.5, 19.3 / 17.2 /
+// 16.6; 52^2 x 13 15.6 / 13.1 / 11.7, 23.5 / 17.4 / 16.6; 64^2 x 13 16.9 / 14.4 / 13.1, 25.4 / 19.6 / 19.5;
+// 128^2 x 9 27.1 / 22.8 / 21.4, 41.0 / 35.5 / 38.1; 256^2 x 5, 71 angles 147 / 92 / -.  3 slices are padded at any
+// size: four take the two-launch form.  One and two stay as they are.
+int padded_slices(int N, int S) {
+  const bool small = (long long)N * N * S < 3 << 14;
+  return S <= 2 || (small && S != 3) ? S : (S + 3) & ~3;
+}
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
@@ -849,9 +856,10 @@ int gt_problem_create(const gt_desc *desc, gt_problem **out) {
   const long long Sr = (long long)D.Nz * D.C;
   if ((long long)D.N * D.N > (1LL << 30) || Sr > (1LL << 20) || (long long)D.nd * D.nang > (1LL << 30))
     return set_err(GT_ERR_ARG, "problem too large for 32-bit pixel / bin indices");
-  int rc = create_problem(D, (int)Sr, padded_slices((int)Sr), out);
+  const int S = padded_slices(D.N, (int)Sr);
+  int rc = create_problem(D, (int)Sr, S, out);
   // no room for the padding (0.23 KB per pixel and more at S = 5): as without it, by slower kernels
-  if (rc == GT_ERR_OOM && padded_slices((int)Sr) != Sr) rc = create_problem(D, (int)Sr, (int)Sr, out);
+  if (rc == GT_ERR_OOM && S != Sr) rc = create_problem(D, (int)Sr, (int)Sr, out);
   return rc;
 }
 
@@ -1864,7 +1872,7 @@ static int create_subs(const gt_subs_desc *D, bool pad, gt_subs **out) {
   }
   // device block
   const size_t NN = (size_t)D->N * D->N;
-  const int ld0 = pad ? padded_slices(s->S0) : s->S0, ld1 = pad ? padded_slices(s->S1) : s->S1;
+  const int ld0 = pad ? padded_slices(D->N, s->S0) : s->S0, ld1 = pad ? padded_slices(D->N, s->S1) : s->S1;
   const size_t nb0 = (size_t)D->nang0 * nd0 * ld0, nb1 = (size_t)D->nang1 * nd0 * ld1,
                nblo = (size_t)D->nang1 * D->nd1 * s->S1lo;
   size_t off = 0;

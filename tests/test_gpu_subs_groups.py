@@ -8,7 +8,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-N, MU = 16, 0.2
+N, MU = 24, 0.2
 
 
 def _subs(C0, C1, Nz, nang0, nang1, coupling="UNCORR"):
