@@ -236,26 +236,28 @@ __global__ void __launch_bounds__(256) k_wgrad_reduce(const float *__restrict__ 
 
 // db[co] (+)= sum over batch and voxels of dY: a cluster of 8 blocks per channel, each an
 // eighth of the voxels, added in a fixed order through distributed shared memory.  HBM bound; one
-// block per channel (16 blocks on 152 SMs) took 229 us for 16 x 262144 values.
+// block per channel (16 blocks on 152 SMs) took 229 us for 16 x 262144 values.  Up to 2048 values of
+// a channel one block: the cluster's barriers cost more (64 x 1024 values 5.1 us, 3.8 with one block).
 constexpr int BG_CL = 8;
+constexpr long long BG_ONE = 2048;
 
-__global__ void __cluster_dims__(BG_CL, 1, 1) __launch_bounds__(256)
+template <int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256)
     k_bias_grad(const float *__restrict__ dy, int Cdy, int dy_off, long long vol, int B, int vec,
                 float *__restrict__ db, int accumulate) {
   __shared__ float sh[8];
   __shared__ float total;
-  cg::cluster_group cl = cg::this_cluster();
-  const int co = blockIdx.x / BG_CL, rank = (int)cl.block_rank();
+  const int co = blockIdx.x / CL, rank = blockIdx.x % CL;
   float a = 0.f;
   for (int b = 0; b < B; ++b) {
     const float *__restrict__ p = dy + ((size_t)b * Cdy + dy_off + co) * vol;
     if (vec) {  // vol a multiple of 4, dy on a 16-byte boundary
-      for (long long v = rank * 256 + threadIdx.x; v < vol / 4; v += BG_CL * 256) {
+      for (long long v = rank * 256 + threadIdx.x; v < vol / 4; v += CL * 256) {
         const float4 q = __ldg(reinterpret_cast<const float4 *>(p) + v);
         a += (q.x + q.y) + (q.z + q.w);
       }
     } else {
-      for (long long v = rank * 256 + threadIdx.x; v < vol; v += BG_CL * 256) a += p[v];
+      for (long long v = rank * 256 + threadIdx.x; v < vol; v += CL * 256) a += p[v];
     }
   }
 #pragma unroll
@@ -267,12 +269,15 @@ __global__ void __cluster_dims__(BG_CL, 1, 1) __launch_bounds__(256)
 #pragma unroll
     for (int k = 0; k < 8; ++k) r += sh[k];
     total = r;
+    if (CL == 1) db[co] = accumulate ? db[co] + r : r;
   }
+  if constexpr (CL == 1) return;
+  cg::cluster_group cl = cg::this_cluster();
   cl.sync();
   if (rank == 0 && threadIdx.x == 0) {
     float r = 0.f;
 #pragma unroll
-    for (int k = 0; k < BG_CL; ++k) r += *cl.map_shared_rank(&total, k);
+    for (int k = 0; k < CL; ++k) r += *cl.map_shared_rank(&total, k);
     db[co] = accumulate ? db[co] + r : r;
   }
   cl.sync();  // the other blocks' shared memory is read until here
@@ -348,7 +353,10 @@ int gt_nn_bias_grad(const float *dy, int Co, int Cdy, int dy_off, int B, long lo
                     void *stream) {
   if (!dy || !db || Co < 1 || dy_off < 0 || dy_off + Co > Cdy) return gt::set_error(GT_ERR_ARG, "gt_nn_bias_grad: bad argument");
   const int vec = vol % 4 == 0 && reinterpret_cast<size_t>(dy) % 16 == 0;
-  k_bias_grad<<<(unsigned)Co * BG_CL, 256, 0, (cudaStream_t)stream>>>(dy, Cdy, dy_off, vol, B, vec, db, accumulate);
+  if (B * vol <= BG_ONE)
+    k_bias_grad<1><<<Co, 256, 0, (cudaStream_t)stream>>>(dy, Cdy, dy_off, vol, B, vec, db, accumulate);
+  else
+    k_bias_grad<BG_CL><<<(unsigned)Co * BG_CL, 256, 0, (cudaStream_t)stream>>>(dy, Cdy, dy_off, vol, B, vec, db, accumulate);
   NN_CK(cudaGetLastError(), "gt_nn_bias_grad");
   return GT_OK;
 }

@@ -74,3 +74,34 @@ def test_plane_of_more_than_2_31_voxels(W):
                                        None))
     got = out.cpu()
     assert torch.equal(got[1], want) and not got[0].any() and not got[2].any()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("W", [64, 40])
+def test_1x1x1_convolution_large_tile(dtype, W):
+    """8 channels x 4 voxels per thread; a partial channel tile, two input channels beyond a staged chunk."""
+    from graptor_gb300 import _lib as L
+    B, D, H, ci, co = 2, 16, 112, 18, 21
+    g = torch.Generator().manual_seed(4)
+    x = torch.randn((B, ci, D, H, W), generator=g).to(dtype)
+    w = (torch.randn((co, ci, 1, 1, 1), generator=g) * 0.2).to(torch.bfloat16)
+    bias = torch.randn(co, generator=g)
+    y = torch.zeros((B, co, D, H, W), device="cuda")
+    xd, wd, bd = x.cuda(), w.cuda(), bias.cuda()
+    L.check(L.lib().gt_nn_conv3d(_p(xd), int(dtype == torch.bfloat16), ci, ci, 0, _p(wd), _p(bd), _p(y), 0, co, co, 0, B, D,
+                                 H, W, 1, 0, 0, None))
+    want = torch.nn.functional.conv3d(x.double(), w.double(), bias.double())
+    assert float((y.double().cpu() - want).abs().max()) <= 19 * 2.0 ** -24 * 18 * 5  # 19 terms below 5
+
+
+@pytest.mark.parametrize("B,vol", [(1, 1), (3, 5), (2, 1024), (1, 2048), (1, 2049), (2, 1028), (3, 683)])
+def test_bias_gradient_on_both_sides_of_one_block(B, vol):
+    from graptor_gb300 import _lib as L
+    co = 5
+    dy = torch.randn((B, co + 1, vol), generator=torch.Generator().manual_seed(vol))
+    dyd, db = dy.cuda(), torch.full((co,), 2.0, device="cuda")
+    for acc in (0, 1):
+        L.check(L.lib().gt_nn_bias_grad(_p(dyd), co, co + 1, 1, B, vol, _p(db), acc, None))
+        want = (1 + acc) * dy[:, 1:].double().sum((0, 2))
+        scale = float(dy.double().abs().sum((0, 2)).max()) + 1
+        assert float((db.double().cpu() - want).abs().max()) <= 40 * 2.0 ** -24 * scale  # some 9 + 5 + 8 additions deep
