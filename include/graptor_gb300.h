@@ -268,7 +268,7 @@ GT_API int gt_batch_set_active(gt_batch *b, int k, int active);
  * work units of every active member (dual update, forward projection + data
  * prox, back projection, primal update), every member with one fixed launch
  * shape.  Mode 0 is the faster one wherever measured (64 problems of up to 128^2 x 8
- * x 4: 0.81 ms an iteration against 1.33 ms); mode 1 has four graph nodes per
+ * x 4: 0.81 ms an iteration against 1.35 ms); mode 1 has four graph nodes per
  * iteration whatever the number of members, and its shapes need no tuning.  It needs every member to share the dimension, the
  * regularisation and the coupling (Frobenius or uncorrelated, <= 8 channels);
  * it returns GT_ERR_ARG otherwise.  Iterates are identical in both modes. */
